@@ -52,6 +52,7 @@
 #include <thread>
 #include <vector>
 
+#include "ilu_sched.h"
 #include "xt_device.h"
 
 namespace xt {
@@ -60,23 +61,11 @@ __device__ int g_ilu_error;  // 0 = clear; 1 = ring wait gave up; 2 = producer w
 
 namespace {
 
-constexpr int kMaxG = 3;
 constexpr int kNB = 16;          // mbarriers per direction: levels in flight < kNB
 constexpr int kTabLevels = 64;  // level table entries staged in shared memory
 constexpr int kHdrBytes = 2 * kNB * 8 + 16 + kTabLevels * 32;
 constexpr long long kSpinLimit = 1ll << 20;
 constexpr int kStageThreads = 512;  // compute warps + the producer and waiter warps, at most
-
-struct TriHost {
-    int ngroups = 0, nlevels = 0, g = 1, maxw = 0;
-    std::vector<int> level_ptr, group_row0, ext_ptr, ext_col;
-    std::vector<double> ext_v, int_v, dinv;
-    std::vector<int> order;  // level order -> group id
-    std::vector<int> pos;    // group id -> level-order position
-    std::vector<int> slot;   // group id -> window slot
-    int nslots = 0;
-    std::vector<double> minv;  // level order, g*g: inverse of the group's diagonal block
-};
 
 // Level-schedule one triangle.  upper == false: rows' L parts
 // (jlu(i) .. ju(i)-1); upper == true: U parts (ju(i) .. jlu(i+1)-1).
@@ -200,11 +189,6 @@ TriHost schedule(int n, const double* alu, const int* jlu, const int* ju, int g,
 
 }  // namespace
 
-// Both schedules, kept on the host to build staged sweeps on first use.
-struct IluSched {
-    TriHost L, U;
-};
-
 namespace {
 
 // Per-level blob layout (sections 16-byte aligned, offsets in bytes):
@@ -237,66 +221,6 @@ struct StageTri {
     DBuf<unsigned char> blob;
     DBuf<int> table;  // per level {off16, pos16, grp0, iss, len16, rhs16, ng, ne, nb or passes}
 };
-
-int max_dyn_smem()
-{
-    static const int v = [] {
-        int dev = 0, r = 0;
-        cudaGetDevice(&dev);
-        if (cudaDeviceGetAttribute(&r, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
-            r = 48 * 1024;
-        return r;
-    }();
-    return v;
-}
-
-bool trace_on() { return std::getenv("XTFEM_TRACE") != nullptr; }
-
-// Runs a() on a second host thread (on the caller's device) while b() runs
-// on this one; returns the first failure, its message set on this thread
-// (an exception in a() becomes XT_ERR_HOST; one in b() is rethrown after
-// the join).
-template <class A, class B>
-int side_by_side(A&& a, B&& b)
-{
-    int dev = 0;
-    XT_CUDA(cudaGetDevice(&dev));
-    int ra = XT_OK;
-    std::string ea;
-    std::thread t([&] {
-        try {
-            if (cudaSetDevice(dev) != cudaSuccess) {
-                ra = XT_ERR_CUDA;
-                ea = "could not select the device on a helper thread";
-                return;
-            }
-            ra = a();
-            if (ra != XT_OK) ea = last_error();
-        } catch (const std::exception& e) {
-            ra = XT_ERR_HOST;
-            ea = e.what();
-        }
-    });
-    int rb = XT_OK;
-    try {
-        rb = b();
-    } catch (...) {
-        t.join();
-        throw;
-    }
-    t.join();
-    if (ra != XT_OK) {
-        set_error(ea);
-        return ra;
-    }
-    return rb;
-}
-
-int env_int(const char* name, int dflt)
-{
-    const char* e = std::getenv(name);
-    return e ? std::atoi(e) : dflt;
-}
 
 // Ring size cap; XTFEM_ILU_RING_KB shrinks it (tests use a tight ring to
 // make levels wait for the region of the level just before them).
@@ -2421,6 +2345,12 @@ int launch_tri(const DevIlu& F, const double* dAinv, const T* v, T* z, T* work, 
     // thread block; 1: node blocks; 0: rows through the ring.  A format
     // that cannot be laid out for the factor falls back to the next.
     int fmt = env_int("XTFEM_ILU_FMT", 4);
+    // FP64, and FP32 with one unknown per node: row records (dev_ilu_rows.cu)
+    if (fmt == 4 && (sizeof(T) == 8 || F.L.g == 1) && !env_int("XTFEM_ILU_SIMPLE", 0)) {
+        RowSweep* rows = nullptr;
+        XT_TRY(get_rows<T>(F, Q, s, rows));
+        if (rows) return run_rows<T>(*rows, Q, dAinv, v, z, s, skip);
+    }
     if constexpr (sizeof(T) == 4) {
         if (F.L.g == 3 && fmt == 4) {
             const int H = F.shares > 0 ? F.shares : env_int("XTFEM_ILU_SHARES", 2);
@@ -2699,6 +2629,7 @@ int build_ilu(DevIlu& d, int n, const double* alu, const int* jlu, const int* ju
     XT_TRY(upload_tri(d.U, sc->U, s));
     d.sched = sc;
     d.stages.clear();
+    d.rows.clear();
     d.blocks = 1;
     d.bounds.clear();
     d.part_sched.clear();
@@ -2756,6 +2687,27 @@ template int ilu_apply<double>(const DevIlu&, int, const double*, const double*,
                                double*, cudaStream_t, const int*);
 template int ilu_apply<float>(const DevIlu&, int, const double*, const float*, float*, float*,
                               cudaStream_t, const int*);
+
+int ilu_error_word(int** p)
+{
+    // the symbol's address, looked up once per device
+    static std::atomic<int*> addr[64];
+    int dev = 0;
+    XT_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) {
+        set_error("ilu_error_word: device index out of range");
+        return XT_ERR_ARG;
+    }
+    int* a = addr[dev].load(std::memory_order_acquire);
+    if (!a) {
+        void* v = nullptr;
+        XT_CUDA(cudaGetSymbolAddress(&v, g_ilu_error));
+        a = static_cast<int*>(v);
+        addr[dev].store(a, std::memory_order_release);
+    }
+    *p = a;
+    return XT_OK;
+}
 
 int ilu_check(cudaStream_t s)
 {

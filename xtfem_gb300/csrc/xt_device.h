@@ -198,6 +198,7 @@ struct DevTri {
 
 struct IluSched;  // host copy of both level schedules (dev_ilu.cu)
 struct IluStage;  // staged-sweep data for one temporal width and precision
+struct RowSweep;  // row-record sweep (dev_ilu_rows.cu)
 
 struct DevIlu {
     int n = 0;
@@ -205,6 +206,8 @@ struct DevIlu {
     std::shared_ptr<IluSched> sched;
     // built on first use for a (q, precision) pair; key 2*q + (FP32 ? 1 : 0)
     mutable std::map<int, std::shared_ptr<IluStage>> stages;
+    // row-record sweeps, built on first use for a (q, precision); null: unfit
+    mutable std::map<int, std::shared_ptr<RowSweep>> rows;
     // lanes per row of the FP32 register sweep (its rows per warp: 10 node
     // rows at 1, 5 at 2, 2 at 4); 0 = XTFEM_ILU_SHARES or 2.  Set by the
     // batch tuner.
@@ -234,6 +237,15 @@ std::vector<int> ilu_block_bounds(int n, int g, int blocks);
 template <class T>
 int ilu_apply(const DevIlu& F, int q, const double* dAinv, const T* v, T* z, T* work,
               cudaStream_t s, const int* skip = nullptr);
+
+// The row-record sweep of F for FP64 (groups of 1 or 3 rows) or FP32 (one-row
+// groups), built on first use; out is null when its rows or window do not
+// fit.  run_rows: ilu_apply through it.
+template <class T>
+int get_rows(const DevIlu& F, int q, cudaStream_t s, RowSweep*& out);
+template <class T>
+int run_rows(const RowSweep& R, int q, const double* dAinv, const T* v, T* z, cudaStream_t s,
+             const int* skip);
 
 // Reads and clears the device-side error word of the staged sweeps (a
 // bounded wait that gave up); XT_OK when clear.
