@@ -1232,7 +1232,7 @@ int xt_damage(int ne, int nn, int ndofn, int nnse, int nnte, int ngpe, int ncmp,
     XT_TRY(dNz.upload(Nz, ngp * nnse, s));
     XT_TRY(dNt.upload(Nt, nnt ? nnt : 1, s));
     XT_TRY(dNt32.alloc(nnt ? nnt : 1));
-    XT_TRY(ntmax.alloc(8));
+    XT_TRY(ntmax.alloc(damage_bounds_floats(nip)));
     XT_TRY(to_f32(dNt.p, dNt32.p, nnt, s));
     XT_TRY(dsol.upload(sol, nsol, s));
     XT_TRY(dym.upload(ym, ngp, s));

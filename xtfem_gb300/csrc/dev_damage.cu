@@ -20,12 +20,13 @@
 // elastic iff 1.5 sum_n tsig_n^2 + 3 sum_s tsig_s^2 <= sig_f^2.
 //
 // GB300's FP64 rate is a small fraction of its FP32 rate, so every step is
-// first screened in FP32 with a rigorous rounding bound.  Steps the screen
+// first screened in FP32 with a rigorous rounding bound: a whole chunk of the
+// table at once, then runs of steps, then single steps.  Steps the screen
 // proves elastic change nothing but the "last elastic" markers (sig_eff,
 // eps_old, sig_d are overwritten by every elastic step, so only the last one
 // before a plastic step, or before the slab ends, has to be evaluated).
-// Steps the screen cannot decide, and plastic steps, are evaluated exactly
-// in FP64 with the reference's operation order.
+// A point's first step the screen cannot decide, and all that follow, go to a
+// team of lanes of the warp that takes the point's FP64 steps (Team).
 #include <cstdlib>
 #include <mutex>
 
@@ -108,69 +109,6 @@ struct State {
     double p, d, ws, dpo, sigd;
 };
 
-// Plastic corrector of src/kokkos_kernel.h:175-341 in FP64, reference order.
-__device__ void corrector(const Mat& m, const double eps[6], State& st)
-{
-    const double d = st.d;
-    double de[6], ds[6], qs[6], dq[6];
-    for (int i = 0; i < 6; ++i) de[i] = eps[i] - st.epo[i];
-    dmat_mul(m, de, ds);
-    for (int i = 0; i < 6; ++i) ds[i] = ds[i] / (1.0 - m.cb * d);
-    const double c4 = m.Kb * (m.ca - m.cb) * d / ((1.0 - m.cb * d) * (1.0 - m.ca * d));
-    double trd = 0.0;
-    for (int i = 0; i < 3; ++i) trd += de[i];
-    for (int i = 0; i < 3; ++i) ds[i] += c4 * trd;
-    for (int i = 0; i < 6; ++i) qs[i] = st.sbk[i] - st.sef[i] - ds[i];
-    const double gam = CY * (1.0 - d) + 3.0 * m.G * (1.0 - m.cb) / (1.0 - m.cb * d);
-    double trq = 0.0;
-    for (int i = 0; i < 3; ++i) trq += qs[i];
-    trq = trq / 3.0;
-    dq[0] = qs[0] - trq; dq[1] = qs[1] - trq; dq[2] = qs[2] - trq;
-    dq[3] = qs[3]; dq[4] = qs[4]; dq[5] = qs[5];
-    const double qeq = vm_equiv(dq);
-    const double trs = -trq;
-    const double dp = (qeq - SIGF) / gam;
-    st.p += dp;
-    const double c5 = 1.0 + gam * dp / SIGF;
-    double dsg[6], sg[6];
-    for (int i = 0; i < 6; ++i) dsg[i] = -dq[i] / c5;
-    sg[0] = dsg[0] + trs; sg[1] = dsg[1] + trs; sg[2] = dsg[2] + trs;
-    sg[3] = dsg[3]; sg[4] = dsg[4]; sg[5] = dsg[5];
-    for (int i = 0; i < 6; ++i) {
-        const double dpl = 3.0 * dsg[i] * dp / (2.0 * SIGF);
-        st.epl[i] += dpl;
-        st.sbk[i] += 2.0 * CY * (1.0 - d) * dpl / 3.0;
-    }
-    for (int i = 0; i < 6; ++i) st.sef[i] = sg[i] + st.sbk[i];
-    double sdev[6];
-    deviator(st.sef, sdev);
-    const double seq = vm_equiv(sdev);
-    const double snew = fabs(seq - SIGF);
-    const double sold = fabs(st.sigd - SIGF);
-    st.ws += (snew * dp + sold * st.dpo) / 2.0;
-    if (st.ws >= WD) {
-        double sp[3] = {0.0, 0.0, 0.0}, sn[3] = {0.0, 0.0, 0.0};
-        for (int i = 0; i < 3; ++i) {
-            if (st.sef[i] < 0.0) sn[i] = st.sef[i];
-            else sp[i] = st.sef[i];
-        }
-        const double x = (1.0 - d) / (1.0 - HH * d);
-        const double yp = (1.0 + m.nu) / (2.0 * m.E) *
-                          (sp[0] * sp[0] + sp[1] * sp[1] + sp[2] * sp[2] +
-                           HH * x * x * (sn[0] * sn[0] + sn[1] * sn[1] + sn[2] * sn[2]));
-        double tr2 = 0.0;
-        for (int i = 0; i < 3; ++i) tr2 += st.sef[i];
-        const double yn = (tr2 >= 0.0) ? m.nu / (2.0 * m.E) * tr2 * tr2
-                                       : m.nu / (2.0 * m.E) * HH * x * x * tr2 * tr2;
-        st.d += pow((yp - yn) / SD, SEXP) * dp;
-    } else {
-        st.d = 0.0;
-    }
-    for (int i = 0; i < 6; ++i) st.epo[i] = eps[i];
-    st.sigd = seq;
-    st.dpo = dp;
-}
-
 // Affine screen coefficients for the current internal state: G (6x6, FP32,
 // G[k][i]), C0 (6, FP32) and the absolute rounding bound of the screened
 // teq^2.
@@ -184,7 +122,12 @@ __device__ void screen_setup(const Mat& m, const State& st, const double E[6][6]
     const double mn = m.coef * (1.0 - 2.0 * m.nu), ms = mn / 2.0;
     double dv[6];
     double S[6];
-    deviator(st.epl, dv);
+    // a third by multiplication: the bound covers its rounding
+    auto dev3 = [](const double* v, double* o) {
+        const double t = (v[0] + v[1] + v[2]) * (1.0 / 3.0);
+        for (int i = 0; i < 6; ++i) o[i] = i < 3 ? v[i] - t : v[i];
+    };
+    dev3(st.epl, dv);
     for (int i = 0; i < 6; ++i) {
         const double c0 = (c3 - 1.0) * (i < 3 ? mn : ms) * dv[i] - st.sbk[i];
         C0[i] = (float)c0;
@@ -192,7 +135,7 @@ __device__ void screen_setup(const Mat& m, const State& st, const double E[6][6]
     }
     for (int k = 0; k < 6; ++k) {
         double ed[6];
-        deviator(E[k], ed);
+        dev3(E[k], ed);
         for (int i = 0; i < 6; ++i) {
             const double gk = c1 * (i < 3 ? mn : ms) * ed[i];
             G[k][i] = (float)gk;
@@ -258,30 +201,413 @@ __device__ __noinline__ void slow_materialize(Slow* s, const double* __restrict_
     s->st.sigd = teq;
 }
 
-// exact FP64 step jj.  Returns 1 when the step was plastic (internal
-// variables changed; the screen is marked stale with an infinite error
-// bound, so the following steps take this exact path too), else 0; an
-// elastic step on a stale screen rebuilds it.  A plastic phase therefore
-// rebuilds the screen once, at its end, not after every plastic step.
-__device__ __noinline__ int slow_step(Slow* s, const double* __restrict__ Nt, int jj, int last_el,
-                                      const float* __restrict__ ntmax, Screen* sc)
-{
-    double eps[6], tse[6];
-    strain_at(s, Nt, jj, eps);
-    const double teq = predictor(s->m, s->st.d, eps, s->st.epl, s->st.sbk, tse);
-    if (teq <= SIGF) {
-        for (int i = 0; i < 6; ++i) { s->st.sef[i] = tse[i]; s->st.epo[i] = eps[i]; }
-        s->st.sigd = teq;
-        if (isinf(sc->err2)) {
-            screen_setup(s->m, s->st, s->E, ntmax, sc->G, sc->C0, sc->err2, sc->e);
-            return 2;
-        }
-        return 0;
+// ---------------------------------------------------------------------------
+// Exact steps of one point by a team of L lanes of a warp.
+//
+// This part takes an FP64 instruction of one warp in 64 cycles whatever its
+// live lanes, so a point's chain of plastic steps costs its FP64 instruction
+// count: one thread doing the six components in turn took about 940 of them a
+// step (29 us).  Here lane i < 6 of a team holds component i of every tensor,
+// lane 6 the trace of every tensor as a component of its own (the predictor
+// and the corrector act on the trace as on a component, with coefficients of
+// its own, so no trace is ever summed), and the scalars are held by all: about
+// 85 instructions a plastic step without damage growth, 130 with it.  The
+// factors of the damage (four quotients) are formed by four lanes in one
+// division, and again only when the damage has changed.  A team's L lanes
+// screen L steps at once between plastic phases.
+//
+// The formulas are those of src/kokkos_kernel.h:96-341 with the sums regrouped
+// (c5 = 1 + gam dp / SIGF is qeq / SIGF; the deviator of D tee is
+// a (tee - tr / 3)); everything in FP64.
+//
+// Measured (GB300, against one thread a point): a slab of 25,600 steps on
+// 192,000 points, 170 of them plastic, 122 -> 19.6 ms (3.05 us a plastic step
+// of the point with the most, 4,900 of its 6,300 cycles FP64 issue); 1,536
+// points, 2,560 steps, host arrays, 31.0 -> 5.1 ms; no plastic point (192,000
+// points, 25,600 steps) 2.1 -> 0.45 ms, from the chunk bound and fused sums.
+//
+// L = 32 (one point a warp) when few of the warp's points need exact steps,
+// else L = 8 (four points a warp, each FP64 instruction serving four).  The
+// teams of a warp run in step: every branch below is taken by the whole warp
+// (a vote), and a team that does not take part keeps its values.
+template <int L>
+struct Team {
+    // lane constants: elastic coefficients, weight in the equivalent stress,
+    // share of the trace (normal 1/3, shear 0, trace 1)
+    double a, off, w, third;
+    double cb, ca, cacb, kb3, g3;     // factors of the moduli (load)
+    double cden;                      // the coefficient of d in the lane's quotient of factors()
+    double ky, kn;                    // (1 + nu) / 2E and nu / 2E
+    double E[6];                      // strain basis of the lane's component
+    double epo, epl, sef, sbk;        // the lane's components
+    double p, d, ws, dpo, sigd;       // the point's scalars
+    double c1, c3m1, c2i, Ai, Bi, rgam, cyd, hx2;  // factors of d
+    float g[6][6], c0[6], err2;       // FP32 screen of the whole point
+    double sumg;                      // sum_k ntmax_k |g_k| of the lane's component
+    unsigned mask;
+    int lane;
+
+    __device__ __forceinline__ double get(double v, int src) const { return __shfl_sync(mask, v, src, L); }
+    // a condition of any of the warp's teams (L = 32: of the one team)
+    static __device__ __forceinline__ bool any(bool c) { return L == 32 ? c : __any_sync(0xffffffffu, c) != 0; }
+    // sum over lanes 0..7 of the team
+    __device__ __forceinline__ double sum8(double v) const
+    {
+        v += __shfl_xor_sync(mask, v, 4, L);
+        v += __shfl_xor_sync(mask, v, 2, L);
+        v += __shfl_xor_sync(mask, v, 1, L);
+        return L == 8 ? v : get(v, 0);
     }
-    if (last_el >= 0) slow_materialize(s, Nt, last_el);
-    corrector(s->m, eps, s->st);
-    sc->err2 = __int_as_float(0x7f800000);  // +inf: screen stale
-    return 1;
+
+    __device__ void load(const DamageArgs& A, int gp)
+    {
+        const int i = lane;
+        const double Ey = A.ym[gp], nu = A.nu[gp];
+        ca = (1.0 + nu) / (3.0 * (1.0 - nu));
+        cb = 2.0 * (4.0 - 5.0 * nu) / (15.0 * (1.0 - nu));
+        cacb = ca - cb;
+        g3 = 3.0 * (Ey / (2.0 * (1.0 + nu))) * (1.0 - cb);
+        cden = i == 0 ? cb : (i == 1 ? ca : HH);
+        ky = (1.0 + nu) / (2.0 * Ey);
+        kn = nu / (2.0 * Ey);
+        const double coef = Ey / ((1.0 + nu) * (1.0 - 2.0 * nu)), mn = coef * (1.0 - 2.0 * nu);
+        const bool norm = i < 3, shear = i >= 3 && i < 6, tr = i == 6;
+        a = shear ? 0.5 * mn : (norm || tr ? mn : 0.0);
+        off = norm ? coef * nu : (tr ? 3.0 * coef * nu : 0.0);
+        w = norm ? 1.5 : (shear ? 3.0 : 0.0);
+        third = norm ? 1.0 / 3.0 : (tr ? 1.0 : 0.0);
+        kb3 = Ey / (3.0 * (1.0 - 2.0 * nu)) * (norm ? 1.0 : (tr ? 3.0 : 0.0));
+        // component i of the strain rows: N_a u_x (+ N_b u_y for a shear)
+        const double* Na = (i == 0 ? A.Nx : (i == 1 || i == 3 ? A.Ny : A.Nz)) + (size_t)gp * A.nnse;
+        const double* Nb = (i == 4 ? A.Ny : A.Nx) + (size_t)gp * A.nnse;
+        const int ux = i == 1 || i == 4 ? 1 : (i == 2 ? 2 : 0), uy = i == 3 ? 1 : 2;
+        for (int k = 0; k < 6; ++k) E[k] = 0.0;
+        if (i < 6)
+            for (int n = 0; n < A.nnse; ++n) {
+                const double* u = A.sol + (size_t)(A.nodes[(size_t)gp * A.nnse + n] - 1) * 3;
+                const double na = Na[n], nb = shear ? Nb[n] : 0.0;
+                for (int k = 0; k < 6; ++k) {
+                    const double* uk = u + (size_t)k * A.nn * 3;
+                    E[k] = fma(na, uk[ux], fma(nb, uk[uy], E[k]));
+                }
+            }
+        const size_t b6 = (size_t)gp * A.ncmp + (i < 6 ? i : 0);
+        epo = i < 6 ? A.eps_old[b6] : 0.0;
+        epl = i < 6 ? A.eps_pl[b6] : 0.0;
+        sef = i < 6 ? A.sig_eff[b6] : 0.0;
+        sbk = i < 6 ? A.sig_back[b6] : 0.0;
+        auto trace = [&](double& v) {
+            const double t = get(v, 0) + get(v, 1) + get(v, 2);
+            if (tr) v = t;
+        };
+        for (int k = 0; k < 6; ++k) trace(E[k]);
+        trace(epo);
+        trace(epl);
+        trace(sef);
+        trace(sbk);
+        p = A.p[gp];
+        d = A.D[gp];
+        ws = A.ws[gp];
+        dpo = A.del_po[gp];
+        sigd = A.sig_d[gp];
+    }
+
+    // the factors of d: 1 / (1 - cb d), 1 / (1 - ca d), (1 - d) / (1 - H d) and
+    // 1 / gam = (1 - cb d) / (CY (1 - d)(1 - cb d) + 3 G (1 - cb)), one division
+    // in lanes 0..3
+    __device__ __forceinline__ void factors()
+    {
+        const double omd = 1.0 - d, ncb = fma(-cb, d, 1.0), own = fma(-cden, d, 1.0);
+        const double gd = fma(CY * omd, ncb, g3);
+        const double quo = (lane == 2 ? omd : (lane == 3 ? ncb : 1.0)) / (lane == 3 ? gd : own);
+        const double r1 = get(quo, 0), ra = get(quo, 1), x = get(quo, 2);
+        rgam = get(quo, 3);
+        c1 = r1;
+        c3m1 = fma(cb * omd, r1, -1.0);
+        const double c2 = cacb * d * r1 * ra;
+        c2i = c2 * third;
+        Ai = a * r1;
+        Bi = fma(off, r1, kb3 * c2);
+        cyd = (2.0 * CY / 3.0) * omd;
+        hx2 = HH * x * x;
+    }
+
+    // screen coefficients of the strain basis (they change with d), then of
+    // the internal variables; the bounds are those of screen_setup
+    __device__ void screen_basis(const float* __restrict__ ntmax)
+    {
+        sumg = 0.0;
+        for (int k = 0; k < 6; ++k) {
+            const double gk = c1 * a * fma(-third, get(E[k], 6), E[k]);
+            sumg = fma((double)__ldg(ntmax + k), fabs(gk), sumg);
+            const float f = (float)gk;
+#pragma unroll
+            for (int i = 0; i < 6; ++i) g[k][i] = __shfl_sync(mask, f, i, L);
+        }
+    }
+    __device__ __forceinline__ void screen_state()
+    {
+        const double c = fma(c3m1 * a, fma(-third, get(epl, 6), epl), -sbk);
+        const float f = (float)c;
+#pragma unroll
+        for (int i = 0; i < 6; ++i) c0[i] = __shfl_sync(mask, f, i, L);
+        const double S = fabs(c) + sumg;
+        const double tot = sum8(w * S * S);
+        const double u = 32.0 * 5.9604644775390625e-8;
+        err2 = (float)(tot * (2.0 * u + u * u + 16.0 * 5.9604644775390625e-8)) * 1.0001f + 1e-30f;
+    }
+    // teq^2 of step j in FP32
+    __device__ __forceinline__ float screen(const float2* __restrict__ nt2, int j) const
+    {
+        const float2 t0 = __ldg(nt2 + 3 * (size_t)j), t1 = __ldg(nt2 + 3 * (size_t)j + 1),
+                     t2 = __ldg(nt2 + 3 * (size_t)j + 2);
+        const float wv[6] = {t0.x, t0.y, t1.x, t1.y, t2.x, t2.y};
+        float q = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 6; ++i) {
+            float acc = c0[i];
+#pragma unroll
+            for (int k = 0; k < 6; ++k) acc = fmaf(wv[k], g[k][i], acc);
+            q = fmaf(i < 3 ? 1.5f : 3.0f, acc * acc, q);
+        }
+        return q;
+    }
+
+    __device__ __forceinline__ double strain(const double nt[6]) const
+    {
+        double e = nt[0] * E[0];
+#pragma unroll
+        for (int k = 1; k < 6; ++k) e = fma(nt[k], E[k], e);
+        return e;
+    }
+    // elastic predictor: the trial elastic strain, its trace and teq^2
+    __device__ __forceinline__ double predict(double eps, double& tee, double& ttr) const
+    {
+        tee = fma(c2i, get(eps, 6), fma(c3m1, epl, c1 * eps));
+        ttr = get(tee, 6);
+        const double ts = fma(a, fma(-third, ttr, tee), -sbk);
+        return sum8(w * ts * ts);
+    }
+    // outputs of an elastic step
+    __device__ __forceinline__ void elastic(double eps, double tee, double ttr, double q, bool take)
+    {
+        const double s = fma(off, ttr, a * tee), t = sqrt(q);
+        if (L == 32 || take) {
+            sef = s;
+            epo = eps;
+            sigd = t;
+        }
+    }
+    // plastic corrector; returns whether d changed
+    __device__ __forceinline__ bool correct(double eps, bool part)
+    {
+        const bool take = L == 32 || part;
+        const double de = eps - epo;
+        const double qs = sbk - sef - fma(Ai, de, Bi * get(de, 6));
+        const double qtr = get(qs, 6);
+        const double dq = fma(-third, qtr, qs);
+        const double q2 = sum8(w * dq * dq);
+        // qeq = sqrt(q2), and its reciprocal: one Newton step on q2 rsqrt(q2)
+        const double rq = rsqrt(q2);
+        double qeq = q2 * rq;
+        qeq = fma(fma(-qeq, qeq, q2), 0.5 * rq, qeq);
+        const double dp = (qeq - SIGF) * rgam;
+        const double dsg = -dq * (SIGF * rq);
+        const double k1 = dp * (1.5 / SIGF);
+        const double nepl = fma(dsg, k1, epl);
+        const double nsbk = fma(dsg, k1 * cyd, sbk);
+        const double nsef = fma(-third, qtr, dsg) + nsbk;
+        // the equivalent stress, and the damage rate's square where it may be
+        // needed: both sums in one butterfly (lanes 0..3 the one, 4..7 the
+        // other) and both roots in one
+        const double tr2 = get(nsef, 6);
+        const double sd = fma(-third, tr2, nsef);
+        const double v = w * sd * sd;
+        double seq, rate = 0.0;
+        if (any(take && ws >= WD)) {
+            const double y = lane < 3 ? (nsef < 0.0 ? hx2 : 1.0) * nsef * nsef : 0.0;
+            const bool up = (lane & 4) != 0;
+            double t = (up ? y : v) + __shfl_xor_sync(mask, up ? v : y, 4, L);
+            t += __shfl_xor_sync(mask, t, 2, L);
+            t += __shfl_xor_sync(mask, t, 1, L);
+            const double yn = kn * (tr2 >= 0.0 ? 1.0 : hx2) * tr2 * tr2;
+            const double root = sqrt(up ? fma(ky, t, -yn) * (1.0 / SD) : t);
+            seq = get(root, 0);
+            rate = get(root, 4);
+        } else {
+            seq = sqrt(sum8(v));
+        }
+        const double nws = ws + fma(fabs(seq - SIGF), dp, fabs(sigd - SIGF) * dpo) * 0.5;
+        const bool grow = take && nws >= WD;
+        if (any(grow && ws < WD)) {  // the step that crosses the threshold
+            const double sp = sum8(lane < 3 ? (nsef < 0.0 ? hx2 : 1.0) * nsef * nsef : 0.0);
+            const double yn = kn * (tr2 >= 0.0 ? 1.0 : hx2) * tr2 * tr2;
+            const double r = sqrt(fma(ky, sp, -yn) * (1.0 / SD));
+            if (ws < WD) rate = r;
+        }
+        // SEXP = 1/2
+        const double nd = grow ? fma(rate, dp, d) : 0.0;
+        const bool changed = take && nd != d;
+        if (take) {
+            p += dp;
+            epl = nepl;
+            sbk = nsbk;
+            sef = nsef;
+            ws = nws;
+            d = nd;
+            epo = eps;
+            sigd = seq;
+            dpo = dp;
+        }
+        return changed;
+    }
+};
+
+// A step's six shape values, the same for the whole team.
+__device__ __forceinline__ void shape_row(const double* __restrict__ Nt, int j, double nt[6])
+{
+    // a caller's table is aligned to 8 bytes only
+#pragma unroll
+    for (int k = 0; k < 6; ++k) nt[k] = __ldg(Nt + (size_t)j * 6 + k);
+}
+
+// The slab's remaining steps of the warp's points in `todo` (one bit a lane:
+// the lane's point gp, from its step from, its last proven step last) by
+// teams of L lanes, 32 / L points at a time.
+template <int L>
+__device__ __noinline__ void exact_points(const DamageArgs& A, const float* __restrict__ ntmax,
+                                          unsigned todo, int gp_lane, int from_lane, int last_lane)
+{
+    constexpr int TEAMS = 32 / L;
+    constexpr int kPasses = L == 32 ? 4 : 8;  // screening passes between two exact steps of other teams
+    const unsigned full = 0xffffffffu;
+    const float thr = (float)(SIGF * SIGF) * 0.99999976f;
+    const int wl = threadIdx.x & 31, team = wl / L;
+    const float2* nt2 = reinterpret_cast<const float2*>(A.Nt32);
+    while (todo) {
+        // the team's point: the team-th bit of todo (none: the team idles on
+        // the first one's data and stores nothing)
+        unsigned m = todo;
+        int src = __ffs(todo) - 1;
+        bool on = false;
+        for (int t = 0; t < TEAMS; ++t) {
+            const int b = m ? __ffs(m) - 1 : -1;
+            if (t == team && b >= 0) {
+                src = b;
+                on = true;
+            }
+            if (b >= 0) m &= m - 1;
+        }
+        todo = m;
+        const int gp = __shfl_sync(full, gp_lane, src);
+        int jj = __shfl_sync(full, from_lane, src), last = __shfl_sync(full, last_lane, src);
+        if (!on) jj = A.nip;
+        Team<L> T;
+        T.mask = L == 32 ? full : (0xffu << (wl & ~7));
+        T.lane = wl % L;
+        T.load(A, gp);
+        T.factors();
+        T.screen_basis(ntmax);
+        T.screen_state();
+        bool stale = false, fresh_basis = true;
+        unsigned n_exact = 0, n_plastic = 0;
+        // the first unproven step is exact; nt holds step jj's shape values
+        // while the team is at an exact step
+        bool exact = on;
+        double nt[6];
+        shape_row(A.Nt, on ? jj : 0, nt);
+        while (Team<L>::any(jj < A.nip)) {
+            // screening: L steps a pass, until a step is not proven
+            for (int pass = 0; pass < kPasses; ++pass) {
+                const bool scan = jj < A.nip && !exact && !stale;
+                if (!Team<L>::any(scan)) break;
+                bool fail = false;
+                if (scan && jj + T.lane < A.nip) fail = !(T.screen(nt2, jj + T.lane) + T.err2 < thr);
+                const unsigned b = (__ballot_sync(full, fail) & T.mask) >> (L == 32 ? 0 : (wl & ~7));
+                if (scan) {
+                    const int f = b ? __ffs(b) - 1 : min(L, A.nip - jj);
+                    if (f > 0) last = jj + f - 1;
+                    jj += f;
+                    exact = b != 0;
+                    if (exact) shape_row(A.Nt, jj, nt);
+                }
+            }
+            const bool act = jj < A.nip && (exact || stale);
+            if (!Team<L>::any(act)) continue;
+            double nx[6];  // the next step's shape values, loaded meanwhile
+            shape_row(A.Nt, min(jj + 1, A.nip - 1), nx);
+            const double eps = T.strain(nt);
+            double tee, ttr;
+            const double q = T.predict(eps, tee, ttr);
+            const bool plastic = act && !(q <= SIGF * SIGF);
+            if (act) ++n_exact;
+            // a plastic step after proven ones: their last one's outputs first
+            const bool pend = plastic && last >= 0;
+            if (Team<L>::any(pend)) {
+                double lt[6], le_tee, le_ttr;
+                shape_row(A.Nt, last >= 0 ? last : 0, lt);
+                const double le = T.strain(lt);
+                const double lq = T.predict(le, le_tee, le_ttr);
+                T.elastic(le, le_tee, le_ttr, lq, pend);
+            }
+            if (Team<L>::any(act && !plastic)) T.elastic(eps, tee, ttr, q, act && !plastic);
+            bool dch = false;
+            if (Team<L>::any(plastic)) {
+                dch = T.correct(eps, plastic);
+                if (plastic) ++n_plastic;
+                if (Team<L>::any(dch)) T.factors();
+                if (dch) fresh_basis = false;
+            }
+            // the screen is rebuilt once a plastic phase has ended
+            const bool rebuild = act && !plastic && stale;
+            if (Team<L>::any(rebuild)) {
+                if (Team<L>::any(rebuild && !fresh_basis)) {
+                    T.screen_basis(ntmax);
+                    if (rebuild) fresh_basis = true;
+                }
+                T.screen_state();
+            }
+            if (act) {
+                stale = plastic;
+                exact = false;
+                last = -1;
+                ++jj;
+#pragma unroll
+                for (int k = 0; k < 6; ++k) nt[k] = nx[k];
+            }
+        }
+        // outputs of the last proven step
+        if (Team<L>::any(last >= 0)) {
+            double lt[6], tee, ttr;
+            shape_row(A.Nt, last >= 0 ? last : 0, lt);
+            const double le = T.strain(lt);
+            const double lq = T.predict(le, tee, ttr);
+            T.elastic(le, tee, ttr, lq, last >= 0);
+        }
+        if (on) {
+            const int i = T.lane;
+            const size_t b6 = (size_t)gp * A.ncmp;
+            if (i < 6) {
+                A.eps_old[b6 + i] = T.epo;
+                A.eps_pl[b6 + i] = T.epl;
+                A.sig_eff[b6 + i] = T.sef;
+                A.sig_back[b6 + i] = T.sbk;
+            }
+            if (i == 0) {
+                const bool gone = A.gpsta && A.gpsta[gp] == 0;  // src/kokkos_damage.f90:102-107
+                A.p[gp] = T.p;
+                A.D[gp] = gone ? 0.0 : T.d;
+                A.ws[gp] = gone ? 0.0 : T.ws;
+                A.del_po[gp] = T.dpo;
+                A.sig_d[gp] = T.sigd;
+                if (A.counters) {
+                    atomicAdd(&A.counters[0], (unsigned long long)n_plastic);
+                    atomicAdd(&A.counters[1], (unsigned long long)A.nip - n_exact);
+                    atomicAdd(&A.counters[2], (unsigned long long)n_exact);
+                }
+            }
+        }
+    }
 }
 
 // The slab's update of point gidx (a copy of the last point, storing
@@ -313,12 +639,12 @@ __device__ __forceinline__ void damage_point(const DamageArgs& a, const float* _
         for (int k = 0; k < 6; ++k) {
             const double* u = a.sol + (size_t)k * a.nn * a.ndofn + (size_t)nd * a.ndofn;
             const double u0 = u[0], u1 = u[1], u2 = u[2];
-            s.E[k][0] += nx * u0;
-            s.E[k][1] += ny * u1;
-            s.E[k][2] += nz * u2;
-            s.E[k][3] += ny * u0 + nx * u1;
-            s.E[k][4] += nz * u1 + ny * u2;
-            s.E[k][5] += nz * u0 + nx * u2;
+            s.E[k][0] = fma(nx, u0, s.E[k][0]);
+            s.E[k][1] = fma(ny, u1, s.E[k][1]);
+            s.E[k][2] = fma(nz, u2, s.E[k][2]);
+            s.E[k][3] = fma(ny, u0, fma(nx, u1, s.E[k][3]));
+            s.E[k][4] = fma(nz, u1, fma(ny, u2, s.E[k][4]));
+            s.E[k][5] = fma(nz, u0, fma(nx, u2, s.E[k][5]));
         }
     }
     State& st = s.st;
@@ -351,7 +677,7 @@ __device__ __forceinline__ void damage_point(const DamageArgs& a, const float* _
     // proven elastic when q + err2 < sig_f^2 (margin covers the float add)
     const float thr = (float)(SIGF * SIGF) * 0.99999976f;
     int last_el = -1;  // last step known elastic whose outputs are pending
-    unsigned n_exact = 0, n_plastic = 0;
+    int first = -1;    // first step the screen does not prove elastic
     // The FP32 shape table is shared by every point: the block streams it
     // through shared memory in chunks, so each step's six values are a
     // broadcast shared-memory read instead of an L2 round trip.
@@ -360,7 +686,28 @@ __device__ __forceinline__ void damage_point(const DamageArgs& a, const float* _
     const float2* nt2 = reinterpret_cast<const float2*>(a.Nt32);
     for (int j0 = 0; j0 < a.nip; j0 += kNtChunk) {
     const int jn = min(kNtChunk, a.nip - j0);
-    __syncthreads();
+    // One bound for the whole chunk first: |tsig_i| <= |C0_i| + e_i + sum_k
+    // mx_k |g_ki| with mx_k the chunk's largest |Nt_k|, inflated as the run
+    // bound below.  Most points (stress well under yield) need nothing else,
+    // and a block of such points does not load the chunk's table.
+    bool open = first < 0;
+    if (run_bound && open && err2 < thr) {
+        const float* mx = ntmax + 8 * (1 + j0 / kNtChunk);
+        float qb = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 6; ++i) {
+            float dev = 0.0f;
+#pragma unroll
+            for (int k = 0; k < 6; ++k) dev = fmaf(__ldg(mx + k), fabsf(G[k][i]), dev);
+            const float b = fabsf(C0[i]) + ecomp[i] + dev * 1.000001f;
+            qb = fmaf(i < 3 ? 1.5f : 3.0f, b * b, qb);
+        }
+        if (qb * 1.0000039f < thr) {
+            last_el = j0 + jn - 1;
+            open = false;
+        }
+    }
+    if (!__syncthreads_or(open)) continue;
     for (int i = threadIdx.x; i < 3 * jn; i += blockDim.x) sNt[i] = __ldg(nt2 + 3 * (size_t)j0 + i);
     __syncthreads();
     // Run bounds: delta_k >= |Nt_k(t) - Nt_k(t0)| of the FP64 table over each
@@ -379,10 +726,9 @@ __device__ __forceinline__ void damage_point(const DamageArgs& a, const float* _
         }
     }
     __syncthreads();
-    for (int jr = 0; jr < jn; jr += kRun) {
+    for (int jr = 0; jr < jn && open && first < 0; jr += kRun) {
     const int jre = min(jn, jr + kRun);
-    // One bound for the whole run (fresh screens only: a stale one has an
-    // infinite err2): with acc_i(t0) the screened component at the run's
+    // One bound for the whole run: with acc_i(t0) the screened component at the run's
     // first step, every step of the run has |tsig_i| <= |acc_i(t0)| + e_i +
     // sum_k delta_k |g_ki| =: B_i (g the FP64 coefficient, |g| <= |G|(1 +
     // 1.01u); the FP32 sum of the six non-negative products is inflated by
@@ -428,30 +774,22 @@ __device__ __forceinline__ void damage_point(const DamageArgs& a, const float* _
             last_el = jj;
             continue;
         }
-        ++n_exact;
-        sc.err2 = err2;
-        const int r = slow_step(&s, a.Nt, jj, last_el, ntmax, &sc);
-        if (r == 1) {
-            ++n_plastic;
-            err2 = sc.err2;  // stale: every step is exact until one is elastic
-        } else if (r == 2) {  // screen rebuilt after a plastic phase
-#pragma unroll
-            for (int k = 0; k < 6; ++k)
-#pragma unroll
-                for (int i = 0; i < 6; ++i) G[k][i] = sc.G[k][i];
-#pragma unroll
-            for (int i = 0; i < 6; ++i) {
-                C0[i] = sc.C0[i];
-                ecomp[i] = sc.e[i];
-            }
-            err2 = sc.err2;
-        }
-        last_el = -1;
+        first = jj;
+        break;
     }
     }
     }
+    // Points with an unproven step go to the whole warp, which takes the rest
+    // of their slab; nothing of their state has changed yet.  Two points or
+    // fewer one after another (their plastic chains at full speed, 32 steps a
+    // screening pass), more four at a time.
+    const unsigned todo = __ballot_sync(0xffffffffu, live && first >= 0);
+    if (todo) {
+        if (__popc(todo) <= 2) exact_points<32>(a, ntmax, todo, gp, first, last_el);
+        else exact_points<8>(a, ntmax, todo, gp, first, last_el);
+    }
+    if (!live || first >= 0) return;
     if (last_el >= 0) slow_materialize(&s, a.Nt, last_el);
-    if (!live) return;
 
     if (a.gpsta && a.gpsta[gp] == 0) {  // src/kokkos_damage.f90:102-107
         st.d = 0.0;
@@ -468,33 +806,35 @@ __device__ __forceinline__ void damage_point(const DamageArgs& a, const float* _
     a.ws[gp] = st.ws;
     a.del_po[gp] = st.dpo;
     a.sig_d[gp] = st.sigd;
-    if (a.counters) {
-        atomicAdd(&a.counters[0], (unsigned long long)n_plastic);
-        atomicAdd(&a.counters[1], (unsigned long long)a.nip - n_exact);
-        atomicAdd(&a.counters[2], (unsigned long long)n_exact);
-    }
+    if (a.counters) atomicAdd(&a.counters[1], (unsigned long long)a.nip);
 }
 
-// Points are dealt to blocks round-robin (pass it, thread t of block b
-// takes point (it blockDim + t) gridDim + b): plastic points cluster in
-// space, i.e. in consecutive point numbers, and their FP64 steps would
-// otherwise pile up in a few blocks on a few SMs while the rest of the GPU
-// idles.  One pass per thread is one thread per point; a small grid with
-// several passes keeps the update on a few SMs.
+// Points are dealt to blocks round-robin (pass it, slot s of block b takes
+// point (it slots + s) gridDim + b): plastic points cluster in space, i.e. in
+// consecutive point numbers, and their FP64 steps would otherwise pile up in
+// a few blocks on a few SMs while the rest of the GPU idles.  One pass per
+// slot is one slot per point; a small grid with several passes keeps the
+// update on a few SMs.  A warp has ppw slots (its first ppw lanes; the others
+// follow along on a copy of the last point): fewer than 32 where the points
+// do not fill the GPU, so that fewer plastic chains share a warp.
 __global__ void __launch_bounds__(256)
-k_damage(DamageArgs a, const float* __restrict__ ntmax, int run_bound, int passes)
+k_damage(DamageArgs a, const float* __restrict__ ntmax, int run_bound, int passes, int ppw)
 {
+    const int lane = threadIdx.x & 31, slots = (int)(blockDim.x >> 5) * ppw;
+    const int slot = (int)(threadIdx.x >> 5) * ppw + lane;
     for (int it = 0; it < passes; ++it)
         damage_point(a, ntmax, run_bound,
-                     ((long long)it * blockDim.x + threadIdx.x) * gridDim.x + blockIdx.x);
+                     lane < ppw ? ((long long)it * slots + slot) * gridDim.x + blockIdx.x : (long long)a.ngp);
 }
 
-// max_t |Nt_k(t)| per k over the slab (single block)
-__global__ void k_ntmax(const float* __restrict__ nt32, int nip, float* __restrict__ out)
+// max_t |Nt_k(t)| per k of each chunk of kNtChunk steps (one block a chunk)
+// into out + 8 (1 + chunk), then of the whole slab into out
+__global__ void __launch_bounds__(256) k_ntmax(const float* __restrict__ nt32, int nip, float* __restrict__ out)
 {
-    __shared__ float sh[6][32];
+    __shared__ float sh[6][8];
     float m[6] = {0, 0, 0, 0, 0, 0};
-    for (int j = threadIdx.x; j < nip; j += blockDim.x)
+    const int j1 = min(nip, ((int)blockIdx.x + 1) * kNtChunk);
+    for (int j = blockIdx.x * kNtChunk + threadIdx.x; j < j1; j += blockDim.x)
         for (int k = 0; k < 6; ++k) m[k] = fmaxf(m[k], fabsf(nt32[(size_t)j * 6 + k]));
     for (int k = 0; k < 6; ++k) {
         float v = m[k];
@@ -504,9 +844,17 @@ __global__ void k_ntmax(const float* __restrict__ nt32, int nip, float* __restri
     __syncthreads();
     if (threadIdx.x < 6) {
         float v = 0.0f;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) v = fmaxf(v, sh[threadIdx.x][w]);
-        out[threadIdx.x] = v * 1.000001f;
+        for (int w = 0; w < 8; ++w) v = fmaxf(v, sh[threadIdx.x][w]);
+        out[8 * (1 + blockIdx.x) + threadIdx.x] = v * 1.000001f;
     }
+}
+
+__global__ void k_ntmax_all(int chunks, float* __restrict__ out)
+{
+    if (threadIdx.x >= 6) return;
+    float v = 0.0f;
+    for (int c = 0; c < chunks; ++c) v = fmaxf(v, out[8 * (1 + c) + threadIdx.x]);
+    out[threadIdx.x] = v;
 }
 
 __global__ void k_nt_table(int nip, double t0, double t1, double t2, double w, double* nt64,
@@ -583,11 +931,13 @@ __global__ void k_any_ge(const double* __restrict__ D, int n, double Dc, int* fl
 
 // Scratch of the allocation-free damage entry point (xt_damage_device):
 // the FP32 copy of the temporal shape table (6 values per step, up to
-// kDamageStaticMaxNip steps), the six shape-value bounds and the three step
-// counters.  1.5 MB in all, part of the library image; one set per process
+// kDamageStaticMaxNip steps), the shape-value bounds of the slab and of its
+// chunks and the three step counters.  1.5 MB in all, part of the library image; one set per process
 // and device, so concurrent calls share it.
 constexpr size_t kStaticNt = (size_t)kDamageStaticMaxNip * 6;
-constexpr size_t kStaticBytes = kStaticNt * sizeof(float) + 64 + 3 * sizeof(unsigned long long);
+constexpr size_t kStaticMax = 8 * (1 + (kDamageStaticMaxNip + kNtChunk - 1) / kNtChunk) * sizeof(float);
+constexpr size_t kStaticBytes = kStaticNt * sizeof(float) + kStaticMax + 3 * sizeof(unsigned long long);
+static_assert(kStaticMax % 8 == 0 && kNtChunk == kDamageChunk, "scratch layout");
 static __device__ __align__(256) unsigned char g_damage_scratch[kStaticBytes];
 
 }  // namespace
@@ -631,7 +981,7 @@ int damage_static_scratch(int device, float** nt32, float** ntmax, unsigned long
     unsigned char* b = static_cast<unsigned char*>(base);
     *nt32 = reinterpret_cast<float*>(b);
     *ntmax = reinterpret_cast<float*>(b + kStaticNt * sizeof(float));
-    *counters = reinterpret_cast<unsigned long long*>(b + kStaticNt * sizeof(float) + 64);
+    *counters = reinterpret_cast<unsigned long long*>(b + kStaticNt * sizeof(float) + kStaticMax);
     return XT_OK;
 }
 
@@ -658,11 +1008,14 @@ int damage_update(const DamageArgs& a, cudaStream_t s)
         return XT_ERR_ARG;
     }
     if (a.ngp <= 0 || a.nip <= 0) return XT_OK;
+    // (the chunks' bounds lie behind the slab's: damage_bounds_floats)
     if (!a.ntmax) {
         set_error("damage_update: missing scratch for the shape-value bounds");
         return XT_ERR_ARG;
     }
-    k_ntmax<<<1, 1024, 0, s>>>(a.Nt32, a.nip, a.ntmax);
+    const int chunks = (a.nip + kNtChunk - 1) / kNtChunk;
+    k_ntmax<<<chunks, 256, 0, s>>>(a.Nt32, a.nip, a.ntmax);
+    k_ntmax_all<<<1, 32, 0, s>>>(chunks, a.ntmax);
     // XTFEM_DAMAGE_RUN=0: screen every step (no per-run bound)
     const char* e = std::getenv("XTFEM_DAMAGE_RUN");
     const int run_bound = (!e || std::atoi(e) != 0) ? 1 : 0;
@@ -677,11 +1030,17 @@ int damage_update(const DamageArgs& a, cudaStream_t s)
     // points in turn (0: one thread per point)
     const char* eb = std::getenv("XTFEM_DAMAGE_BLOCKS");
     const long long want = eb ? std::atoll(eb) : 0;
-    const long long full = ((long long)a.ngp + nt - 1) / nt;
+    // slots per warp: as many as leave about twelve warps an SM.  A 1,536-point
+    // update (2,560 steps) takes 7.0 ms with 32 slots a warp, its plastic
+    // points three and more to a warp, and 5.1 ms with one.
+    int ppw = 32;
+    while (ppw > 1 && (long long)a.ngp <= (long long)(ppw / 2) * 152 * 12) ppw /= 2;
+    const int slots = nt / 32 * ppw;
+    const long long full = ((long long)a.ngp + slots - 1) / slots;
     const int grid = (int)((want > 0 && want < full) ? want : full);
-    const int passes = (int)(((long long)a.ngp + (long long)grid * nt - 1) / ((long long)grid * nt));
-    k_damage<<<grid, nt, 0, s>>>(a, a.ntmax, run_bound, passes);
-    note_launches(2);
+    const int passes = (int)(((long long)a.ngp + (long long)grid * slots - 1) / ((long long)grid * slots));
+    k_damage<<<grid, nt, 0, s>>>(a, a.ntmax, run_bound, passes, ppw);
+    note_launches(3);
     XT_CUDA(cudaGetLastError());
     return XT_OK;
 }

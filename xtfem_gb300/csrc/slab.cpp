@@ -324,6 +324,7 @@ int damage_slab(xt_slab_s& s, double* stats)
         XT_TRY((to_blocks<double, double>(s.disp.p, s.dblk.p, s.p, s.q, st)));
         XT_TRY(s.Nt64.alloc((size_t)s.nip * 6));
         XT_TRY(s.Nt32.alloc((size_t)s.nip * 6));
+        XT_TRY(s.ntmax.alloc(damage_bounds_floats(s.nip)));
         XT_TRY(nt_table_device(s.nip, s.tc[0], s.tc[1], s.tc[2], s.w, s.Nt64.p, s.Nt32.p, st));
         XT_CUDA(cudaMemsetAsync(s.counters.p, 0, 3 * sizeof(unsigned long long), st));
         DamageArgs a{};
@@ -391,6 +392,7 @@ int damage_launch(xt_slab_s& s)
     XT_CUDA(cudaStreamWaitEvent(ds, s.ev_sol, 0));
     XT_TRY(s.Nt64.alloc((size_t)s.nip * 6));
     XT_TRY(s.Nt32.alloc((size_t)s.nip * 6));
+    XT_TRY(s.ntmax.alloc(damage_bounds_floats(s.nip)));
     XT_TRY(nt_table_device(s.nip, s.tc[0], s.tc[1], s.tc[2], s.w, s.Nt64.p, s.Nt32.p, ds));
     XT_CUDA(cudaMemsetAsync(s.counters.p, 0, 3 * sizeof(unsigned long long), ds));
     DamageArgs a{};
@@ -689,7 +691,6 @@ int xt_slab_create(xth_problem h, const xt_slab_config* cfg, xt_slab* out)
         XT_TRY(s->nef.alloc(1));
         XT_TRY(s->flag.alloc(1));
         XT_TRY(s->counters.alloc(3));
-        XT_TRY(s->ntmax.alloc(8));
         XT_CUDA(cudaStreamSynchronize(st));
         s->w = 2.0 * M_PI * cfg->freq;
         s->dt = cfg->dt0 * cfg->n1;

@@ -480,8 +480,14 @@ struct DamageArgs {
     double *p, *D, *ws, *del_po, *sig_d;            // ngp
     const int* gpsta;            // optional: zero D, ws where gpsta == 0
     unsigned long long* counters;  // optional [3]: plastic, screened, exact steps
-    float* ntmax;                // device scratch, 6 floats (per-slab |Nt_k| bounds)
+    float* ntmax;                // device scratch of damage_bounds_floats(nip) floats (|Nt_k| bounds)
 };
+// Steps a chunk of the update's shape table; the floats its bounds take.
+constexpr int kDamageChunk = 1024;
+inline size_t damage_bounds_floats(int nip)
+{
+    return 8 * (1 + ((size_t)(nip > 0 ? nip : 1) + kDamageChunk - 1) / kDamageChunk);
+}
 int damage_update(const DamageArgs& a, cudaStream_t s);
 
 // Static device scratch of the allocation-free damage entry point: FP32
