@@ -420,11 +420,13 @@ __global__ void __launch_bounds__((kRowWarps + 1) * 32, 1) k_tri_rows(RowArgs<T>
         __syncwarp();
         asm volatile("bar.sync 0;" ::: "memory");  // levels 0 and 1 are there
         for (int l = 0; l < a.nl; ++l) {
-            // level l's entry was read in the interval before: its place is free
+            // level l's entry was read in the interval before, so its place is
+            // free; level 0's is read in interval 0 itself, its place follows
+            // one interval later
             if (lane == 0 && ok) {
-                if (l + NR < a.nl) {
-                    copy(l + NR);
-                    issued = l + NR + 1;
+                for (int m = l == 1 ? NR : l + NR; l > 0 && m <= l + NR && m < a.nl; ++m) {
+                    copy(m);
+                    issued = m + 1;
                 }
                 if (l + 2 < a.nl) ok = wait(l + 2);
             }
