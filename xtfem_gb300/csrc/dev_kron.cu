@@ -14,7 +14,7 @@
 // Roofline: the kernel streams nnz(K)+nnz(M) column indices and values once
 // plus the row pointers, and touches X (gathered, L2-resident) and Y once.
 // In FP32 it is HBM-bound; in FP64 the GB300's FP64 pipe (about 1.2 TFLOP/s)
-// binds first because every nonzero carries q FMAs.
+// binds first because every nonzero carries q FMAs (k_kron_nb64).
 #include <algorithm>
 #include <cstdint>
 #include <cstdlib>
@@ -146,21 +146,17 @@ k_kron_spmm(int p, const int* __restrict__ kptr, const int* __restrict__ kcol,
                 ak[b] += __shfl_xor_sync(0xffffffffu, ak[b], off, LANES);
                 am[b] += __shfl_xor_sync(0xffffffffu, am[b], off, LANES);
             }
-        // epilogue: lane a < Q forms output block a of this row
-        if (act) {
+        // epilogue: lane a < Q forms output block a of this row (every lane
+        // holds all the sums; a branch per a would issue the mixing Q times)
+        if (act && lane < Q) {
+            T acc = T(0);
 #pragma unroll
-            for (int a = 0; a < Q; ++a) {
-                if (lane == a) {
-                    T acc = T(0);
-#pragma unroll
-                    for (int b = 0; b < Q; ++b) {
-                        acc = fma(sA[b * Q + a], ak[b], acc);
-                        acc = fma(sB[b * Q + a], am[b], acc);
-                    }
-                    T* yp = y + (size_t)r * Q + a;
-                    *yp = (beta == T(0)) ? alpha * acc : fma(beta, *yp, alpha * acc);
-                }
+            for (int b = 0; b < Q; ++b) {
+                acc = fma(sA[b * Q + lane], ak[b], acc);
+                acc = fma(sB[b * Q + lane], am[b], acc);
             }
+            T* yp = y + (size_t)r * Q + lane;
+            *yp = (beta == T(0)) ? alpha * acc : fma(beta, *yp, alpha * acc);
         }
     }
 }
@@ -172,14 +168,16 @@ bool nb_enabled()
     return !e || std::atoi(e) != 0;
 }
 
-// b[at[i]] = double-float of a[i]
-__global__ void k_scatter_df(const double* __restrict__ a, const int* __restrict__ at,
-                             float2* __restrict__ b, size_t n)
+// The node-block copies of CSR value i, at at[i]: FP64 and double-float.
+__global__ void k_scatter_blocks(const double* __restrict__ a, const int* __restrict__ at,
+                                 double* __restrict__ b64, float2* __restrict__ bdf, size_t n)
 {
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (size_t)gridDim.x * blockDim.x) {
-        const float h = __double2float_rn(a[i]);
-        b[at[i]] = make_float2(h, __double2float_rn(a[i] - (double)h));
+        const double v = a[i];
+        const float h = __double2float_rn(v);
+        b64[at[i]] = v;
+        bdf[at[i]] = make_float2(h, __double2float_rn(v - (double)h));
     }
 }
 
@@ -273,19 +271,14 @@ k_kron_df(int p, const int* __restrict__ kptr, const int* __restrict__ kcol,
                 df_add_df(kh[b], kl[b], a1, a2);
                 df_add_df(mh[b], ml[b], b1, b2);
             }
-        if (act) {
+        if (act && lane < Q) {
+            float h = 0.0f, l = 0.0f;
 #pragma unroll
-            for (int a = 0; a < Q; ++a) {
-                if (lane == a) {
-                    float h = 0.0f, l = 0.0f;
-#pragma unroll
-                    for (int b = 0; b < Q; ++b) {
-                        df_mul_acc(h, l, sA[b * Q + a].x, sA[b * Q + a].y, kh[b], kl[b]);
-                        df_mul_acc(h, l, sB[b * Q + a].x, sB[b * Q + a].y, mh[b], ml[b]);
-                    }
-                    y[(size_t)r * Q + a] = df_norm(h, l);
-                }
+            for (int b = 0; b < Q; ++b) {
+                df_mul_acc(h, l, sA[b * Q + lane].x, sA[b * Q + lane].y, kh[b], kl[b]);
+                df_mul_acc(h, l, sB[b * Q + lane].x, sB[b * Q + lane].y, mh[b], ml[b]);
             }
+            y[(size_t)r * Q + lane] = df_norm(h, l);
         }
     }
 }
@@ -399,6 +392,87 @@ __global__ void __launch_bounds__(256) kb_kron_nb(const FlexStepItem* __restrict
     if (e.ctl[1] != 0) return;
     kron_nb_body<Q>(e.nodes, e.bptr, e.bcol, e.kv, e.mv, e.A, e.B, e.zfix, e.wfix, blockIdx.x,
                     gridDim.x);
+}
+
+// FP64 node-block apply, Y = alpha (K X A^T + M X B^T) + beta Y: a thread owns
+// (node row a, DOF c, temporal entry b) and accumulates (KX)[3a+c][b] and
+// (MX)[3a+c][b] over the node row's blocks, four FP64 multiply-adds a block;
+// the Q threads of (a, c) exchange their sums through shared memory for the
+// q x q mixing.  Threads are dealt to (a, c, b) without a gap, so that the
+// multiply-adds are the whole of the FP64 work: this part's FP64 pipe (a warp
+// instruction every 19 cycles of an SM) is what bounds the operator, 1.72 M
+// warp instructions and 105 us on the 20 x 20 x 60 rod (q = 6).  The CSR
+// kernel spends half as much again on row tails and the lanes' tree sums.
+// Measured there: 119 us; figures against the CSR kernel at kron_spmm.
+template <int Q>
+__global__ void __launch_bounds__(256)
+k_kron_nb64(int nodes, const int* __restrict__ bptr, const int* __restrict__ bcol,
+            const int* __restrict__ mask, const double* __restrict__ kv,
+            const double* __restrict__ mv, const double* __restrict__ dA,
+            const double* __restrict__ dB, double alpha, double beta,
+            const double* __restrict__ x, double* __restrict__ y)
+{
+    constexpr int TPN = 3 * Q, NPB = 256 / TPN;
+    __shared__ double sA[Q * Q], sB[Q * Q], sK[256], sM[256];
+    const int t = threadIdx.x;
+    for (int i = t; i < Q * Q; i += 256) {
+        sA[i] = dA[i];
+        sB[i] = dB[i];
+    }
+    const int nl = t / TPN, rem = t - nl * TPN, c = rem / Q, b = rem - c * Q;
+    const int a = blockIdx.x * NPB + nl;
+    const bool act = nl < NPB && a < nodes;
+    double ak = 0.0, am = 0.0;
+    if (act) {
+        const int b1 = bptr[a + 1];
+#pragma unroll 3
+        for (int k = bptr[a]; k < b1; ++k) {
+            const double* xb = x + (size_t)bcol[k] * TPN + b;
+            const double* kr = kv + (size_t)k * 9 + c * 3;
+            const double x0 = xb[0], x1 = xb[Q], x2 = xb[2 * Q];
+            const double xc = c == 0 ? x0 : (c == 1 ? x1 : x2);
+            const double k0 = kr[0], k1 = kr[1], k2 = kr[2], m = mv[k];
+            const int mk = mask[k];
+            if (mk == 0xfff) {
+                ak = fma(k0, x0, ak);
+                ak = fma(k1, x1, ak);
+                ak = fma(k2, x2, ak);
+                am = fma(m, xc, am);
+            } else {  // only the entries that K and M have: 0 times an infinite x is no zero
+                const int r = mk >> (3 * c);
+                if (r & 1) ak = fma(k0, x0, ak);
+                if (r & 2) ak = fma(k1, x1, ak);
+                if (r & 4) ak = fma(k2, x2, ak);
+                if (mk >> 9) am = fma(m, xc, am);
+            }
+        }
+    }
+    sK[t] = ak;
+    sM[t] = am;
+    __syncthreads();
+    if (act) {
+        const int base = t - b;
+        double acc = 0.0;
+#pragma unroll
+        for (int j = 0; j < Q; ++j) {
+            acc = fma(sA[j * Q + b], sK[base + j], acc);
+            acc = fma(sB[j * Q + b], sM[base + j], acc);
+        }
+        double* yp = y + (size_t)(3 * a + c) * Q + b;
+        *yp = beta == 0.0 ? alpha * acc : fma(beta, *yp, alpha * acc);
+    }
+}
+
+template <int Q>
+int launch_nb64(const DevNodeBlocks& nb, const double* dA, const double* dB, double alpha,
+                double beta, const double* x, double* y, cudaStream_t s)
+{
+    constexpr int NPB = 256 / (3 * Q);
+    k_kron_nb64<Q><<<(nb.nodes + NPB - 1) / NPB, 256, 0, s>>>(
+        nb.nodes, nb.ptr.p, nb.col.p, nb.mask.p, nb.k64.p, nb.m64.p, dA, dB, alpha, beta, x, y);
+    note_launches(1);
+    XT_CUDA(cudaGetLastError());
+    return XT_OK;
 }
 
 template <int Q>
@@ -573,75 +647,86 @@ int csr_build_node_blocks(DevCsr& K, int n, const int* ki, const int* kj, const 
     if (n <= 0 || n % 3 != 0 || K.n != n) return XT_OK;
     const int nodes = n / 3;
     std::vector<int> ptr(nodes + 1, 0), col;
-    std::vector<float2> kdf, mdf;
+    std::vector<double> m64;
+    col.reserve((size_t)K.nnz / 9 + nodes);
+    m64.reserve((size_t)K.nnz / 9 + nodes);
     std::vector<int> pos(nodes, -1);  // block index of neighbour node b in the current row
     std::vector<int> from_csr((size_t)K.nnz, -1);
-    auto split = [](double v) {
-        const float h = (float)v;
-        return make_float2(h, (float)(v - (double)h));
-    };
+    std::vector<int> order, mask;  // mask: the block entries that K (bits 0..8) and M (9..11) have
+    mask.reserve((size_t)K.nnz / 9 + nodes);
     for (int a = 0; a < nodes; ++a) {
         const int first = (int)col.size();
+        order.clear();
         for (int c = 0; c < 3; ++c)
             for (int k = ki[3 * a + c] - 1; k < ki[3 * a + c + 1] - 1; ++k) {
                 const int b = (kj[k] - 1) / 3;
                 if (pos[b] < 0) {
-                    pos[b] = (int)col.size();
-                    col.push_back(b);
-                    kdf.resize(kdf.size() + 9, make_float2(0.f, 0.f));
-                    mdf.push_back(make_float2(0.f, 0.f));
+                    pos[b] = 0;
+                    order.push_back(b);
                 }
             }
         // neighbour nodes in ascending order (the CSR columns are sorted)
-        std::vector<int> order(col.begin() + first, col.end());
         std::sort(order.begin(), order.end());
         for (size_t t = 0; t < order.size(); ++t) pos[order[t]] = first + (int)t;
-        std::copy(order.begin(), order.end(), col.begin() + first);
+        col.insert(col.end(), order.begin(), order.end());
+        mask.resize(col.size(), 0);
+        bool fits = true;
         for (int c = 0; c < 3; ++c)
             for (int k = ki[3 * a + c] - 1; k < ki[3 * a + c + 1] - 1; ++k) {
                 const int j = kj[k] - 1, b = j / 3;
-                const size_t at = (size_t)pos[b] * 9 + c * 3 + (j - 3 * b);
-                kdf[at] = split(kv[k]);
+                const int e = c * 3 + (j - 3 * b);
+                const size_t at = (size_t)pos[b] * 9 + e;
+                // one entry a place: a column listed twice stays CSR
+                if (at >= (size_t)INT32_MAX || (mask[pos[b]] >> e & 1)) fits = false;
+                mask[pos[b]] |= 1 << e;
                 from_csr[k] = (int)at;
             }
         // M: m_ab on the three diagonal entries of each block, nothing else
-        std::vector<double> mval(order.size(), 0.0);
-        std::vector<int> mcount(order.size(), 0);
-        bool fits = true;
+        m64.resize(col.size(), 0.0);
         for (int c = 0; c < 3 && fits; ++c)
             for (int k = mi[3 * a + c] - 1; k < mi[3 * a + c + 1] - 1; ++k) {
                 const int j = mj[k] - 1, b = j / 3;
                 if (j - 3 * b != c || pos[b] < 0) { fits = false; break; }
-                const int t = pos[b] - first;
-                if (mcount[t] > 0 && mval[t] != mv[k]) { fits = false; break; }
-                mval[t] = mv[k];
-                ++mcount[t];
+                int& mk = mask[pos[b]];
+                if ((mk >> (9 + c) & 1) || (mk >> 9 && m64[pos[b]] != mv[k])) { fits = false; break; }
+                m64[pos[b]] = mv[k];
+                mk |= 1 << (9 + c);
             }
-        for (size_t t = 0; t < order.size() && fits; ++t) {
-            if (mcount[t] != 0 && mcount[t] != 3) fits = false;
-            mdf[first + t] = split(mval[t]);
-        }
+        for (size_t t = first; t < col.size() && fits; ++t)
+            if (mask[t] >> 9 != 0 && mask[t] >> 9 != 7) fits = false;
         for (int b : order) pos[b] = -1;
         if (!fits) return XT_OK;  // no exact node-block form: the CSR kernel stays
         ptr[a + 1] = (int)col.size();
     }
     nb.nodes = nodes;
     nb.nblocks = (int)col.size();
+    const size_t n9 = (size_t)nb.nblocks * 9;
     XT_TRY(nb.ptr.upload(ptr.data(), ptr.size(), s));
     XT_TRY(nb.col.upload(col.data(), col.size(), s));
-    XT_TRY(nb.kdf.upload(kdf.data(), kdf.size(), s));
-    XT_TRY(nb.mdf.upload(mdf.data(), mdf.size(), s));
+    XT_TRY(nb.m64.upload(m64.data(), m64.size(), s));
+    XT_TRY(nb.mask.upload(mask.data(), mask.size(), s));
     XT_TRY(nb.from_csr.upload(from_csr.data(), from_csr.size(), s));
-    XT_CUDA(cudaStreamSynchronize(s));  // host staging vectors go out of scope
+    XT_TRY(nb.kdf.alloc(n9));
+    XT_TRY(nb.k64.alloc(n9));
+    XT_TRY(nb.mdf.alloc((size_t)nb.nblocks));
+    // K's values from its CSR copy on the device, zero where that has no entry
+    XT_CUDA(cudaMemsetAsync(nb.kdf.p, 0, n9 * sizeof(float2), s));
+    XT_CUDA(cudaMemsetAsync(nb.k64.p, 0, n9 * sizeof(double), s));
+    if (nb.nblocks) {
+        k_to_df<<<256, 256, 0, s>>>(nb.m64.p, nb.mdf.p, (size_t)nb.nblocks);
+        note_launches(1);
+    }
     nb.ok = true;
+    XT_TRY(node_blocks_refresh(K, s));
+    XT_CUDA(cudaStreamSynchronize(s));  // host staging vectors go out of scope
     return XT_OK;
 }
 
 int node_blocks_refresh(DevCsr& K, cudaStream_t s)
 {
     if (!K.nb.ok || K.nnz == 0) return XT_OK;
-    k_scatter_df<<<std::max(1, std::min(4096, (K.nnz + 255) / 256)), 256, 0, s>>>(
-        K.v64.p, K.nb.from_csr.p, K.nb.kdf.p, (size_t)K.nnz);
+    k_scatter_blocks<<<std::max(1, std::min(4096, (K.nnz + 255) / 256)), 256, 0, s>>>(
+        K.v64.p, K.nb.from_csr.p, K.nb.k64.p, K.nb.kdf.p, (size_t)K.nnz);
     note_launches(1);
     XT_CUDA(cudaGetLastError());
     return XT_OK;
@@ -668,6 +753,25 @@ int kron_spmm(const DevCsr& K, const DevCsr& M, int q, const double* dA,
         return XT_ERR_ARG;
     }
     if (K.n == 0) return XT_OK;
+    if constexpr (sizeof(T) == 8) {
+        // FP64 in node blocks where these hold little but K's own entries (a
+        // place without an entry costs its issue all the same: with blocks
+        // less than 5/8 full the CSR kernel does less work).  20 x 20 x 60
+        // rod, q = 6: 179 us in CSR form, 119 us in blocks (255 us in CSR form
+        // with a mixing branch per output); 10 x 10 x 30 rod 38 and 25 us.
+        if (K.nb.ok && 5LL * 9 * K.nb.nblocks <= 8LL * K.nnz && nb_enabled()) {
+            switch (q) {
+            case 1: return launch_nb64<1>(K.nb, dA, dB, alpha, beta, x, y, s);
+            case 2: return launch_nb64<2>(K.nb, dA, dB, alpha, beta, x, y, s);
+            case 3: return launch_nb64<3>(K.nb, dA, dB, alpha, beta, x, y, s);
+            case 4: return launch_nb64<4>(K.nb, dA, dB, alpha, beta, x, y, s);
+            case 5: return launch_nb64<5>(K.nb, dA, dB, alpha, beta, x, y, s);
+            case 6: return launch_nb64<6>(K.nb, dA, dB, alpha, beta, x, y, s);
+            case 7: return launch_nb64<7>(K.nb, dA, dB, alpha, beta, x, y, s);
+            default: return launch_nb64<8>(K.nb, dA, dB, alpha, beta, x, y, s);
+            }
+        }
+    }
     switch (q) {
     case 1: return launch_q<T, 1>(K, M, dA, dB, alpha, beta, x, y, s);
     case 2: return launch_q<T, 2>(K, M, dA, dB, alpha, beta, x, y, s);

@@ -105,6 +105,8 @@ struct DevNodeBlocks {
     DBuf<int> ptr, col;    // nodes + 1 block pointers, neighbour node per block
     DBuf<float2> kdf;      // 9 per block, row-major, double-float
     DBuf<float2> mdf;      // 1 per block, double-float
+    DBuf<double> k64, m64; // the same in FP64
+    DBuf<int> mask;        // entries of the block that K (bits 0..8) and M (9..11) have
     DBuf<int> from_csr;    // K's nnz entries: position of each in kdf
 };
 
