@@ -7,16 +7,15 @@
 // element triplets into CSR (tricsr, src/spmtx.f90:359-407).  Here the
 // pattern is fixed once per mesh, so reassembly is two kernels:
 //
-//   k_element_k   one thread block per element: the geometry of the 2x2x2
-//                 Gauss points (shape-function derivatives, Jacobian
+//   k_element_k   one thread per pair of an element's nodes: the geometry of
+//                 the 2x2x2 Gauss points (shape-function derivatives, Jacobian
 //                 determinant; the reference's sign table, abscissa and
-//                 closed-form 3x3 inverse) in shared memory, then one thread
-//                 per entry (i a, j b) of the 24 x 24 element matrix,
-//                 summing over the Gauss points the isotropic B^T D B entry
+//                 closed-form 3x3 inverse) in shared memory, then the pair's
+//                 3 x 3 block of the element matrix, the isotropic B^T D B
 //                   detJ (lambda N_i,a N_j,b + mu N_i,b N_j,a
 //                         + mu delta_ab grad N_i . grad N_j)
-//                 with lambda = E nu / ((1 + nu)(1 - 2 nu)) and
-//                 mu = E / (2 (1 + nu)) of that Gauss point;
+//                 summed over the points with lambda = E nu / ((1 + nu)(1 - 2 nu))
+//                 and mu = E / (2 (1 + nu)) of each (K_ji is its transpose);
 //   k_gather_k    one thread per CSR entry: the sum of its element
 //                 contributions in ascending element order (a fixed order,
 //                 so the result is the same bits run to run), 1 on the
@@ -44,85 +43,126 @@ __constant__ signed char c_sign[8][3] = {{-1, -1, +1}, {-1, -1, -1}, {-1, +1, -1
                                          {-1, +1, +1}, {+1, -1, +1}, {+1, -1, -1},
                                          {+1, +1, -1}, {+1, +1, +1}};
 
-__global__ void __launch_bounds__(576)
+// Node pairs i <= j of an element, and the packed element matrix: 36 blocks
+// K_ij of 3 x 3 entries (K_ji is the transpose).
+constexpr int kPairs = 36, kPacked = 9 * kPairs;
+constexpr int kElems = 8;  // elements of a thread block
+
+__host__ __device__ constexpr int pair_of(int i, int j)  // i <= j
+{
+    return i * 8 - i * (i - 1) / 2 + (j - i);
+}
+
+// One thread per (element, node pair), eight elements a block; the geometry
+// of the 64 Gauss points first, one thread each.  FP64-bound: a pair sums
+// S1 = sum_l lambda detJ grad N_i grad N_j^T and S2 likewise with mu (21
+// multiply-adds a point) and forms K_ij = S1 + S2^T + tr(S2) I from them, half
+// of the 24 x 24 matrix; a thread per entry of the whole matrix spent about
+// nine operations a point on each of its 576 entries.  20 x 20 x 60 rod
+// (24,000 elements), the whole reassembly and one apply with host vectors:
+// 4,580 -> 913 us (the reassembly alone 4,144 -> 641 us, the copies of the
+// moduli and the gather among it).
+__global__ void __launch_bounds__(kElems * kPairs)
 k_element_k(int ne, const int* __restrict__ conn, const double* __restrict__ xyz,
             const int* __restrict__ gel, const double* __restrict__ ym,
             const double* __restrict__ nu, double* __restrict__ ke)
 {
-    __shared__ double dN[8][8][3];  // [gauss point][node][x, y, z]
-    __shared__ double det[8], lam[8], mu[8];
-    const int e = blockIdx.x;
-    if (e >= ne) return;
+    __shared__ double ref[8][8][3];             // reference derivatives [point][node][axis]
+    __shared__ double dN[kElems][8][8][3];      // [element][point][node][x, y, z]
+    __shared__ double ld[kElems][8], md[kElems][8];  // lambda detJ, mu detJ
     const int t = threadIdx.x;
-    if (t < 8) {
-        const int l = t;
+    if (t < 192) {
+        const int l = t / 24, i = (t - l * 24) / 3, m = t % 3;
         const double g[2] = {-kGaussAbs, kGaussAbs};
-        const double xi = g[(l >> 2) & 1], eta = g[(l >> 1) & 1], zeta = g[l & 1];
-        double xe[8][3], dn[8][3];
-        for (int i = 0; i < 8; ++i) {
-            const int nd = conn[(size_t)e * 8 + i];
-            for (int m = 0; m < 3; ++m) xe[i][m] = xyz[(size_t)nd * 3 + m];
-            const double sx = c_sign[i][0], sy = c_sign[i][1], sz = c_sign[i][2];
-            dn[i][0] = 0.125 * sx * (1.0 + sy * eta) * (1.0 + sz * zeta);
-            dn[i][1] = 0.125 * sy * (1.0 + sx * xi) * (1.0 + sz * zeta);
-            dn[i][2] = 0.125 * sz * (1.0 + sx * xi) * (1.0 + sy * eta);
-        }
-        double J[3][3];
-        for (int a = 0; a < 3; ++a)
-            for (int m = 0; m < 3; ++m) {
-                double s = 0.0;
-                for (int i = 0; i < 8; ++i) s += dn[i][a] * xe[i][m];
-                J[a][m] = s;
-            }
-        const double d = J[0][0] * J[1][1] * J[2][2] + J[0][1] * J[1][2] * J[2][0] +
-                         J[0][2] * J[1][0] * J[2][1] - J[0][0] * J[1][2] * J[2][1] -
-                         J[0][1] * J[1][0] * J[2][2] - J[0][2] * J[1][1] * J[2][0];
-        double inv[3][3];
-        inv[0][0] = (J[1][1] * J[2][2] - J[1][2] * J[2][1]) / d;
-        inv[0][1] = (J[0][2] * J[2][1] - J[0][1] * J[2][2]) / d;
-        inv[0][2] = (J[0][1] * J[1][2] - J[0][2] * J[1][1]) / d;
-        inv[1][0] = (J[1][2] * J[2][0] - J[1][0] * J[2][2]) / d;
-        inv[1][1] = (J[0][0] * J[2][2] - J[0][2] * J[2][0]) / d;
-        inv[1][2] = (J[0][2] * J[1][0] - J[0][0] * J[1][2]) / d;
-        inv[2][0] = (J[1][0] * J[2][1] - J[1][1] * J[2][0]) / d;
-        inv[2][1] = (J[0][1] * J[2][0] - J[0][0] * J[2][1]) / d;
-        inv[2][2] = (J[0][0] * J[1][1] - J[0][1] * J[1][0]) / d;
-        for (int i = 0; i < 8; ++i)
-            for (int m = 0; m < 3; ++m) {
-                double s = 0.0;
-                for (int a = 0; a < 3; ++a) s += inv[m][a] * dn[i][a];
-                dN[l][i][m] = s;
-            }
-        det[l] = d;
-        const size_t gi = (size_t)(gel ? gel[e] : e) * 8 + l;  // the moduli's element
-        const double E = ym[gi], v = nu[gi];
-        const double c = E / ((1.0 + v) * (1.0 - 2.0 * v));
-        lam[l] = c * v;
-        mu[l] = c * (0.5 - v);
+        const double p[3] = {1.0 + c_sign[i][0] * g[(l >> 2) & 1], 1.0 + c_sign[i][1] * g[(l >> 1) & 1],
+                             1.0 + c_sign[i][2] * g[l & 1]};
+        const int u = m == 0 ? 1 : 0, v = m == 2 ? 1 : 2;
+        ref[l][i][m] = 0.125 * c_sign[i][m] * p[u] * p[v];
     }
     __syncthreads();
-    // entry (r, c) of the row-major 24 x 24 element matrix, DOF 3 node + comp
-    const int r = t / 24, cc = t - r * 24;
-    const int i = r / 3, a = r - 3 * i, j = cc / 3, b = cc - 3 * j;
-    double s = 0.0;
-    for (int l = 0; l < 8; ++l) {
-        double v = lam[l] * dN[l][i][a] * dN[l][j][b] + mu[l] * dN[l][i][b] * dN[l][j][a];
-        if (a == b)
-            v += mu[l] * (dN[l][i][0] * dN[l][j][0] + dN[l][i][1] * dN[l][j][1] +
-                          dN[l][i][2] * dN[l][j][2]);
-        s += v * det[l];
+    if (t < 8 * kElems) {
+        const int el = t >> 3, l = t & 7, e = blockIdx.x * kElems + el;
+        if (e < ne) {
+            double J[3][3] = {};
+            for (int i = 0; i < 8; ++i) {
+                const int nd = conn[(size_t)e * 8 + i];
+                double xe[3];
+                for (int m = 0; m < 3; ++m) xe[m] = xyz[(size_t)nd * 3 + m];
+                for (int a = 0; a < 3; ++a)
+                    for (int m = 0; m < 3; ++m) J[a][m] = fma(ref[l][i][a], xe[m], J[a][m]);
+            }
+            double inv[3][3];
+            inv[0][0] = J[1][1] * J[2][2] - J[1][2] * J[2][1];
+            inv[0][1] = J[0][2] * J[2][1] - J[0][1] * J[2][2];
+            inv[0][2] = J[0][1] * J[1][2] - J[0][2] * J[1][1];
+            inv[1][0] = J[1][2] * J[2][0] - J[1][0] * J[2][2];
+            inv[1][1] = J[0][0] * J[2][2] - J[0][2] * J[2][0];
+            inv[1][2] = J[0][2] * J[1][0] - J[0][0] * J[1][2];
+            inv[2][0] = J[1][0] * J[2][1] - J[1][1] * J[2][0];
+            inv[2][1] = J[0][1] * J[2][0] - J[0][0] * J[2][1];
+            inv[2][2] = J[0][0] * J[1][1] - J[0][1] * J[1][0];
+            const double d = J[0][0] * inv[0][0] + J[0][1] * inv[1][0] + J[0][2] * inv[2][0];
+            const double rd = 1.0 / d;
+            for (int a = 0; a < 3; ++a)
+                for (int m = 0; m < 3; ++m) inv[a][m] *= rd;
+            for (int i = 0; i < 8; ++i)
+                for (int m = 0; m < 3; ++m)
+                    dN[el][l][i][m] = fma(inv[m][2], ref[l][i][2],
+                                          fma(inv[m][1], ref[l][i][1], inv[m][0] * ref[l][i][0]));
+            const size_t gi = (size_t)(gel ? gel[e] : e) * 8 + l;  // the moduli's element
+            const double E = ym[gi], v = nu[gi];
+            const double c = E / ((1.0 + v) * (1.0 - 2.0 * v)) * d;
+            ld[el][l] = c * v;
+            md[el][l] = c * (0.5 - v);
+        }
     }
-    ke[(size_t)e * 576 + t] = s;
+    __syncthreads();
+    const int el = t / kPairs, pr = t - el * kPairs, e = blockIdx.x * kElems + el;
+    if (e >= ne) return;
+    int i = 0;
+    while (pr >= pair_of(i, 7) + 1) ++i;
+    const int j = i + pr - pair_of(i, i);
+    double s1[3][3] = {}, s2[3][3] = {};
+    for (int l = 0; l < 8; ++l) {
+        const double* gi = dN[el][l][i];
+        const double* gj = dN[el][l][j];
+        const double lam = ld[el][l], mu = md[el][l];
+        for (int a = 0; a < 3; ++a) {
+            const double p1 = lam * gi[a], p2 = mu * gi[a];
+            for (int b = 0; b < 3; ++b) {
+                s1[a][b] = fma(p1, gj[b], s1[a][b]);
+                s2[a][b] = fma(p2, gj[b], s2[a][b]);
+            }
+        }
+    }
+    const double tr = s2[0][0] + s2[1][1] + s2[2][2];
+    double* o = ke + (size_t)e * kPacked + pr * 9;
+    for (int a = 0; a < 3; ++a)
+        for (int b = 0; b < 3; ++b) o[a * 3 + b] = s1[a][b] + s2[b][a] + (a == b ? tr : 0.0);
 }
 
+// K's entries from the element matrices, in every form the operators read:
+// FP64 and FP32 CSR values and, where K has them, its node blocks (FP64 and
+// double-float) at at[k].
 __global__ void k_gather_k(int nnz, const int* __restrict__ cptr, const int* __restrict__ cidx,
                            const double* __restrict__ ke, const unsigned char* __restrict__ bcdiag,
-                           double* __restrict__ kv)
+                           double* __restrict__ kv, float* __restrict__ kv32,
+                           const int* __restrict__ at, double* __restrict__ b64,
+                           float2* __restrict__ bdf)
 {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nnz; k += gridDim.x * blockDim.x) {
         double s = 0.0;
-        for (int t = cptr[k]; t < cptr[k + 1]; ++t) s += ke[cidx[t]];
-        kv[k] = bcdiag[k] ? 1.0 : s;
+        const int t1 = cptr[k + 1];
+        for (int t = cptr[k]; t < t1; ++t) s += ke[cidx[t]];
+        if (bcdiag[k]) s = 1.0;
+        const float h = __double2float_rn(s);
+        kv[k] = s;
+        kv32[k] = h;
+        if (at) {
+            const int p = at[k];
+            b64[p] = s;
+            bdf[p] = make_float2(h, __double2float_rn(s - (double)h));
+        }
     }
 }
 
@@ -308,7 +348,12 @@ int system_set_mesh(System& S, int nn, int ne, const double* xyz, const int* con
     for (int k = 0; k < nnz; ++k) cnt[k + 1] += cnt[k];
     std::vector<int> idx(cnt[nnz]), fill(cnt.begin(), cnt.end() - 1);
     for (size_t t = 0; t < where.size(); ++t)
-        if (where[t] >= 0) idx[fill[where[t]]++] = (int)t;
+        if (where[t] >= 0) {
+            const int e = (int)(t / 576), r = (int)(t % 576) / 24, c = (int)(t % 24);
+            const int i = r / 3, a = r % 3, j = c / 3, b = c % 3;
+            idx[fill[where[t]]++] = e * kPacked + (i <= j ? pair_of(i, j) * 9 + 3 * a + b
+                                                         : pair_of(j, i) * 9 + 3 * b + a);
+        }
     // the new K (1-based host copy for the upload and the node-block form)
     std::vector<int> ia(n + 1), ja(nnz);
     for (int r = 0; r <= n; ++r) ia[r] = rp[r] + 1;
@@ -337,7 +382,7 @@ int system_set_mesh(System& S, int nn, int ne, const double* xyz, const int* con
     } else {
         A.gel.release();
     }
-    XT_TRY(A.ke.alloc((size_t)ne * 576));
+    XT_TRY(A.ke.alloc((size_t)ne * kPacked));
     XT_TRY(A.ym.alloc((size_t)ne * 8));
     XT_TRY(A.nu.alloc((size_t)ne * 8));
     XT_CUDA(cudaStreamSynchronize(s));  // host staging vectors go out of scope
@@ -368,16 +413,17 @@ int system_assemble_k_device(System& S, const double* ym, const double* nu, bool
         return XT_ERR_STATE;
     }
     cudaStream_t s = S.stream;
-    k_element_k<<<A.ne, 576, 0, s>>>(A.ne, A.conn.p, A.xyz.p, by_gel ? A.gel.p : nullptr, ym, nu,
-                                     A.ke.p);
-    const int nnz = S.K.nnz;
+    k_element_k<<<(A.ne + kElems - 1) / kElems, kElems * kPairs, 0, s>>>(
+        A.ne, A.conn.p, A.xyz.p, by_gel ? A.gel.p : nullptr, ym, nu, A.ke.p);
+    DevCsr& K = S.K;
+    const int nnz = K.nnz;
     const int blocks = std::max(1, std::min(4096, (nnz + 255) / 256));
-    k_gather_k<<<blocks, 256, 0, s>>>(nnz, A.cptr.p, A.cidx.p, A.ke.p, A.bcdiag.p, S.K.v64.p);
+    const bool nb = K.nb.ok;
+    k_gather_k<<<blocks, 256, 0, s>>>(nnz, A.cptr.p, A.cidx.p, A.ke.p, A.bcdiag.p, K.v64.p, K.v32.p,
+                                     nb ? K.nb.from_csr.p : nullptr, K.nb.k64.p, K.nb.kdf.p);
     note_launches(2);
     XT_CUDA(cudaGetLastError());
-    XT_TRY(to_f32(S.K.v64.p, S.K.v32.p, (size_t)nnz, s));
-    S.K.vdf.release();  // remade from the new values on first use
-    XT_TRY(node_blocks_refresh(S.K, s));
+    K.vdf.release();  // remade from the new values on first use
     return XT_OK;
 }
 

@@ -119,7 +119,7 @@ struct DevAssembly {
     DBuf<int> conn;              // ne x 8, 0-based nodes
     DBuf<int> cptr, cidx;        // per K entry: its element-matrix entries
     DBuf<unsigned char> bcdiag;  // per K entry: diagonal of a constrained DOF
-    DBuf<double> ke;             // ne x 576 element matrices
+    DBuf<double> ke;             // element matrices, packed (dev_assembly.cu)
     DBuf<double> ym, nu;         // ne x 8 Gauss-point moduli
     DBuf<int> gel;               // optional: element e's index in full-mesh moduli arrays
 };
