@@ -52,6 +52,7 @@
 #include <thread>
 #include <vector>
 
+#include "ilu_ring.cuh"
 #include "ilu_sched.h"
 #include "xt_device.h"
 
@@ -638,7 +639,8 @@ struct IluStage {
     bool reg_ok = false;
     // the same per row block of a block-Jacobi factor: one thread block per
     // (block, temporal block), each block's sweep arguments in a device table
-    int parts = 0, ncw = 0, win_elems = 0;
+    int parts = 0, ncw = 0;
+    size_t smem = 0;
     long long lanesL = 0, lanesU = 0;
     std::vector<std::shared_ptr<RegTri>> regLp, regUp;
     DBuf<unsigned char> argsL, argsU;  // RegArgs per block
@@ -1403,53 +1405,76 @@ __global__ void __launch_bounds__(kStageThreads, 1) k_tri_col(StageArgs<float> a
 }  // namespace
 
 // ---------------------------------------------------------------------------
-// Register-prefetched row sweep (FP32, g = 3; the default for FP32).
+// Row sweep with a level's data in registers ahead ("register sweep"; FP32,
+// g = 3; the default for FP32).
 //
 // One thread block per temporal block (Q blocks per sweep, each on its own
-// SM), each the whole level chain, as the column format; but the factor
-// data never passes through shared memory.  Shared memory holds only the
-// solution window (3 rows x 1 value per slot); every record of a level is
-// loaded from global memory (L2) straight into registers two levels ahead
-// of its use, so a level's critical path is: window reads at byte offsets
-// already in registers, one multiply-add per factor entry, the share and
-// diagonal-block shuffles, the window store and one block barrier.  A level
-// has no branch: every warp has a fixed-size slot at every level.
+// SM), each the whole level chain, as the column format, in rows: a level
+// has no branch, every warp has a fixed-size slot at every level.
 //
 // Layout.  Lane = (group of the warp's chunk, row r of the group, share h
 // of the row's entries, H shares): lanes g*3H + r*H + h; a lane owns a
-// share of the row's off-diagonal entries, one per step, SMAX steps (a
-// multiple of 4; entries past the lane's own read an all-zero window slot
+// share of the row's off-diagonal entries, one per step, SMAX steps (an
+// even number; entries past the lane's own read an all-zero window slot
 // with value 0).  The groups of a level are sorted by their longest row
 // and dealt to chunks of 32/(3H) groups; a level with more chunks than the
 // ncw warps is split into consecutive sub-levels (its groups are
 // independent).  Chunk w of (sub-)level l sits in the fixed slot l*ncw + w;
 // warps without a chunk at a level get an empty slot.  A slot holds, per
 // lane (loads of 16 bytes, consecutive lanes adjacent):
-//   float4 {minv[r][0..2] (row r of the inverted 3 x 3 diagonal block),
-//           window offset of the row (-1: lane stores nothing)}   512 B
-//   int    destination (forward: the backward sweep's right-hand-side
-//          slot of the row; backward: row * Q of z)               128 B
-//   uint4  byte offsets in the window of steps 4k..4k+3          SMAX/4 x 512 B
-//   float4 factor values of steps 4k..4k+3                       SMAX/4 x 512 B
-// The right-hand sides are per-temporal-block arrays in the same lane-slot
+//   per row of the warp (32 / H of them; the row's lanes read one address):
+//     float4 {minv[r][0..2] (row r of the inverted 3 x 3 diagonal block),
+//             window offset of the row (-1: nothing is stored)}
+//     int    destination (forward: the backward sweep's right-hand-side
+//            place of the row; backward: row * Q of z)
+//   per lane, for every four steps and a last pair (loads of up to 16 bytes,
+//   consecutive lanes adjacent): the byte offsets in the window and the
+//   factor values of the steps,
+// each part padded to 128 bytes.
+// The right-hand sides are per-temporal-block arrays in the same row
 // order (the forward sweep's from a pre-pass that also applies the q x q
 // mixing with A^-1; the backward sweep's written by the forward sweep), so
-// every load of a level has an address known in advance.  The loads are
-// inline-PTX non-coherent loads (volatile, so they are issued where they
-// stand, two levels before their use), and the level barrier is a
-// volatile bar.sync that they do not cross.  A row's entries are summed in
-// a step order chosen on the host so that a warp's window reads of one
-// step fall into distinct shared-memory banks where possible.
+// every copy of a level has an address known in advance.  A row's entries
+// are summed in a step order chosen on the host so that a warp's window reads
+// of one step fall into distinct shared-memory banks where possible.
+//
+// Flow.  One more warp of the block copies levels ahead into a ring in shared
+// memory (ilu_ring.cuh); the others read the next level's entry into registers
+// behind the window reads of the current one, so a level's critical path is:
+// window reads at offsets already in registers, the multiply-adds, the share
+// and diagonal-block shuffles, the window store and the level barrier.
+// What bounds it: the chain (about 350 cycles a level with one warp, 400 with
+// three) and, in wide levels, the SM's shared-memory port (18 wavefronts of
+// slot data and about 15 of window reads a warp).  Read from global memory
+// straight into registers four levels ahead, a level also paid the L1's share
+// of those loads, with a record per lane instead of per row and an L2 prefetch
+// instruction that touched each line of the slot: 786 cycles a level on the
+// 20 x 20 x 60 rod, 620 now.  Figures at launch_reg.
 constexpr int kRegMaxWarps = 16;
-constexpr unsigned kRegLaneTab = 640;
+// Bytes of a slot's row records, of its offsets and of the whole slot.
+__host__ __device__ constexpr unsigned reg_pad(unsigned b) { return (b + 127u) / 128u * 128u; }
+__host__ __device__ constexpr unsigned reg_rows_bytes(int H) { return reg_pad(20u * 32u / (unsigned)H); }
+__host__ __device__ constexpr unsigned reg_offs_bytes(int smax, bool w16) { return (unsigned)smax * 32u * (w16 ? 2u : 4u); }
+__host__ __device__ constexpr unsigned reg_slot_bytes(int H, int smax, bool w16)
+{
+    return reg_rows_bytes(H) + reg_offs_bytes(smax, w16) + (unsigned)smax * 128u;
+}
+// Place of step st of a lane among the offsets or values (in entries): fours
+// of a lane together, a last pair likewise.
+__host__ __device__ constexpr unsigned reg_step_at(int smax, int st, int lane)
+{
+    return st < smax / 4 * 4 ? ((unsigned)(st >> 2) * 32u + (unsigned)lane) * 4u + (unsigned)(st & 3)
+                             : (unsigned)(smax / 4) * 128u + (unsigned)lane * 2u + (unsigned)(st & 1);
+}
 
 struct RegTri {
     int nl = 0, ncw = 0, H = 0, smax = 0, slot_bytes = 0;
     int win_elems = 0, zero_off = 0;
     bool w16 = false;  // 16-bit window byte offsets (window <= 64 KB)
-    long long lanes = 0;  // nl * ncw * 32
+    int nr = 0;  // levels of a part of the ring
+    long long lanes = 0;  // nl * ncw * 32 / H: places of right-hand sides
     DBuf<unsigned char> slots;
-    std::vector<int> row_slot;             // host: lane slot of each row's h = 0 lane
+    std::vector<int> row_slot;             // host: right-hand-side place of each row
     std::vector<std::vector<int>> chunks;  // host (build only): level-order groups per chunk
     std::vector<int> chunk_slot, chunk_steps;
 };
@@ -1498,7 +1523,7 @@ bool reg_plan(const TriHost& h, int H, RegTri& t, int force_ncw = 0)
                 const int i = grp[gw], G = h.order[i];
                 for (int r = 0; r < g; ++r) {
                     steps = std::max(steps, (rowlen(i, r) + H - 1) / H);
-                    t.row_slot[(size_t)G * g + r] = (int)(slot * 32 + gw * GS + r * H);
+                    t.row_slot[(size_t)G * g + r] = (int)(slot * (32 / H) + gw * g + r);
                 }
             }
             if (slot * 32 + 31 >= INT32_MAX) return false;
@@ -1509,12 +1534,28 @@ bool reg_plan(const TriHost& h, int H, RegTri& t, int force_ncw = 0)
         }
     }
     t.nl = nl;
-    t.smax = (smax + 3) / 4 * 4;
-    t.lanes = (long long)nl * t.ncw * 32;
+    t.smax = (smax + 1) / 2 * 2;
+    t.lanes = (long long)nl * t.ncw * (32 / H);
     t.zero_off = h.nslots * g;
     t.win_elems = (h.nslots + 1) * g;
-    return t.smax <= 32 && (long long)t.win_elems * 4 <= (long long)max_dyn_smem();
+    return t.smax <= 32;
 }
+
+// Ring bytes of one level, and the dynamic shared memory of a sweep.
+unsigned reg_level_bytes(const RegTri& t, int smax, bool w16)
+{
+    return (unsigned)t.ncw * (reg_slot_bytes(t.H, smax, w16) + 128u / (unsigned)t.H);
+}
+size_t reg_smem(const RegTri& t)
+{
+    return reg_pad((unsigned)t.win_elems * 4u) +
+           (size_t)kRingParts * t.nr * reg_level_bytes(t, t.smax, t.w16);
+}
+int reg_ring(const RegTri& t, int smax, bool w16, long long room)
+{
+    return ring_levels(reg_level_bytes(t, smax, w16), room - (long long)reg_pad((unsigned)t.win_elems * 4u));
+}
+constexpr long long kRegStatic = 2048;  // static shared memory of a sweep, at most
 
 // Slots of a planned triangle.  dst: forward, the other triangle's
 // row_slot; backward (dst empty): row * Q.
@@ -1523,18 +1564,19 @@ int reg_fill(const TriHost& h, RegTri& t, int smax, int Q, const std::vector<int
 {
     const int g = 3, H = t.H, GS = 3 * H, GPW = 32 / GS;
     t.smax = smax;
-    const unsigned ob = t.w16 ? 256u : 512u;  // bytes of one offset quad per warp
-    t.slot_bytes = (int)(kRegLaneTab + (unsigned)(smax / 4) * (ob + 512u));
+    const unsigned rb = reg_rows_bytes(H), ob = reg_offs_bytes(smax, t.w16);
+    const int rw = 32 / H;  // row records of a slot
+    t.slot_bytes = (int)reg_slot_bytes(H, smax, t.w16);
     const size_t nslot = (size_t)t.nl * t.ncw;
     std::vector<unsigned char> blob(nslot * t.slot_bytes, 0);
     // every lane of every slot starts empty: no store, all steps on the zero slot
     for (size_t sl = 0; sl < nslot; ++sl) {
         unsigned char* b = blob.data() + sl * t.slot_bytes;
         const int none = -1;
-        for (int lane = 0; lane < 32; ++lane) std::memcpy(b + lane * 16 + 12, &none, 4);
-        for (int e = 0; e < (smax / 4) * 128; ++e) {
-            if (t.w16) reinterpret_cast<unsigned short*>(b + kRegLaneTab)[e] = (unsigned short)(t.zero_off * 4);
-            else reinterpret_cast<unsigned*>(b + kRegLaneTab)[e] = (unsigned)t.zero_off * 4u;
+        for (int r = 0; r < rw; ++r) std::memcpy(b + r * 16 + 12, &none, 4);
+        for (int e = 0; e < smax * 32; ++e) {
+            if (t.w16) reinterpret_cast<unsigned short*>(b + rb)[e] = (unsigned short)(t.zero_off * 4);
+            else reinterpret_cast<unsigned*>(b + rb)[e] = (unsigned)t.zero_off * 4u;
         }
     }
     std::vector<int> seen(t.win_elems, 0);
@@ -1547,24 +1589,24 @@ int reg_fill(const TriHost& h, RegTri& t, int smax, int Q, const std::vector<int
         const int slot = t.chunk_slot[c];
         unsigned char* b = blob.data() + (size_t)slot * t.slot_bytes;
         float* gm = reinterpret_cast<float*>(b);
-        int* go = reinterpret_cast<int*>(b + 512);
-        unsigned* off = reinterpret_cast<unsigned*>(b + kRegLaneTab);
-        unsigned short* off16 = reinterpret_cast<unsigned short*>(b + kRegLaneTab);
-        float* val = reinterpret_cast<float*>(b + kRegLaneTab + (smax / 4) * ob);
+        int* go = reinterpret_cast<int*>(b + 16 * rw);
+        unsigned* off = reinterpret_cast<unsigned*>(b + rb);
+        unsigned short* off16 = reinterpret_cast<unsigned short*>(b + rb);
+        float* val = reinterpret_cast<float*>(b + rb + ob);
         const auto& grp = t.chunks[c];
         for (int lane = 0; lane < 32; ++lane) {
             ent[lane].clear();
             const int gw = lane / GS, r = (lane % GS) / H, hh = lane % H;
             if (gw >= GPW || gw >= (int)grp.size()) continue;
             const int i = grp[gw], G = h.order[i];
-            for (int k = 0; k < 3; ++k) gm[lane * 4 + k] = (float)h.minv[(size_t)i * 9 + r * 3 + k];
             if (hh == 0) {
-                const int wo = h.slot[G] * g + r;
-                std::memcpy(&gm[lane * 4 + 3], &wo, 4);
+                const int rec = gw * g + r, wo = h.slot[G] * g + r;
+                for (int k = 0; k < 3; ++k) gm[rec * 4 + k] = (float)h.minv[(size_t)i * 9 + r * 3 + k];
+                std::memcpy(&gm[rec * 4 + 3], &wo, 4);
                 const long long d = dst ? (long long)(*dst)[(size_t)G * g + r]
                                         : ((long long)row0 + (long long)G * g + r) * Q;
                 valid = valid && wo >= 0 && wo < t.zero_off && d >= 0 && d < INT32_MAX;
-                go[lane] = (int)d;
+                go[rec] = (int)d;
             }
             const int kb = h.ext_ptr[(size_t)i * g + r], ke = h.ext_ptr[(size_t)i * g + r + 1];
             for (int k = kb + hh; k < ke; k += H) {
@@ -1602,10 +1644,10 @@ int reg_fill(const TriHost& h, RegTri& t, int smax, int Q, const std::vector<int
                     seen[o] = epoch;
                     load[o & 31]++;
                 }
-                const size_t oi = ((size_t)(st >> 2) * 32 + lane) * 4 + (st & 3);
+                const size_t oi = reg_step_at(smax, st, lane);
                 if (t.w16) off16[oi] = (unsigned short)(o * 4);
                 else off[oi] = (unsigned)o * 4u;
-                val[((size_t)(st >> 2) * 32 + lane) * 4 + (st & 3)] = v;
+                val[oi] = v;
             }
         }
         for (int lane = 0; lane < 32; ++lane) valid = valid && ent[lane].empty();
@@ -1621,9 +1663,9 @@ int reg_fill(const TriHost& h, RegTri& t, int smax, int Q, const std::vector<int
 // Register capacities (steps per lane) compiled for each share count.
 int reg_smax(int H, int need)
 {
-    static const int caps2[] = {8, 12, 16}, caps1[] = {12, 20}, caps4[] = {8};
+    static const int caps2[] = {8, 10, 12, 16}, caps1[] = {12, 20}, caps4[] = {8};
     const int* c = H == 2 ? caps2 : (H == 1 ? caps1 : caps4);
-    const int n = H == 2 ? 3 : (H == 1 ? 2 : 1);
+    const int n = H == 2 ? 4 : (H == 1 ? 2 : 1);
     for (int i = 0; i < n; ++i)
         if (need <= c[i]) return c[i];
     return 0;
@@ -1646,7 +1688,15 @@ int build_reg(const IluSched& S, int Q, int H, IluStage& st, cudaStream_t s)
     // (XTFEM_ILU_W16=0: 32-bit)
     const bool w16 = (long long)std::max(L->win_elems, U->win_elems) * 4 <= 65536 &&
                      env_int("XTFEM_ILU_W16", 1) != 0;
-    L->w16 = U->w16 = w16;
+    // fewer warps (more sub-levels) where the ring does not fit
+    const long long room = (long long)max_dyn_smem() - kRegStatic;
+    auto fit = [&](const TriHost& h, RegTri& t) {
+        while ((t.nr = reg_ring(t, smax, w16, room)) == 0 && t.ncw > 1)
+            if (!reg_plan(h, H, t, t.ncw - 1)) return false;
+        t.w16 = w16;
+        return t.nr > 0;
+    };
+    if (!fit(S.U, *U) || !fit(S.L, *L)) return XT_OK;
     XT_TRY(side_by_side([&] { return reg_fill(S.U, *U, smax, Q, nullptr, s); },
                         [&] { return reg_fill(S.L, *L, smax, Q, &U->row_slot, s); }));
     if (!L->slots.p || !U->slots.p) return XT_OK;
@@ -1670,302 +1720,185 @@ int build_reg(const IluSched& S, int Q, int H, IluStage& st, cudaStream_t s)
     return XT_OK;
 }
 
-__device__ __forceinline__ float4 nc_v4f(const void* p)
-{
-    float4 r;
-    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
-                 : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w)
-                 : "l"(p));
-    return r;
-}
-__device__ __forceinline__ uint4 nc_v4u(const void* p)
-{
-    uint4 r;
-    asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
-                 : "l"(p));
-    return r;
-}
-__device__ __forceinline__ float nc_f(const void* p)
-{
-    float r;
-    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(r) : "l"(p));
-    return r;
-}
-__device__ __forceinline__ int nc_i(const void* p)
-{
-    int r;
-    asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(r) : "l"(p));
-    return r;
-}
 __device__ __forceinline__ float lds_f(unsigned addr)
 {
     float r;
     asm volatile("ld.shared.f32 %0, [%1];" : "=f"(r) : "r"(addr));
     return r;
 }
-__device__ __forceinline__ void prefetch_l2(const void* p)
+__device__ __forceinline__ unsigned lds_u(unsigned addr)
 {
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
-}
-__device__ __forceinline__ void level_barrier()
-{
-    asm volatile("bar.sync 0;" ::: "memory");
-}
-
-// Offsets of four steps: four 32-bit window byte offsets, or (W16) four
-// 16-bit ones packed in two words.
-template <bool W16> struct RegOff;
-template <> struct RegOff<false> {
-    uint4 o;
-    __device__ __forceinline__ unsigned at(int i) const
-    {
-        return i == 0 ? o.x : (i == 1 ? o.y : (i == 2 ? o.z : o.w));
-    }
-};
-template <> struct RegOff<true> {
-    uint2 o;
-    __device__ __forceinline__ unsigned at(int i) const
-    {
-        const unsigned w = i < 2 ? o.x : o.y;
-        return (i & 1) ? (w >> 16) : (w & 0xffffu);
-    }
-};
-
-template <int SMAX, bool W16>
-struct RegSet {
-    RegOff<W16> off[SMAX / 4];
-    float4 val[SMAX / 4];
-    float4 gm;
-    int go;
-    float b;
-};
-
-// The slot at p (already offset to this warp's slot of the level) and the
-// right-hand side at bsrc.
-__device__ __forceinline__ uint2 nc_v2u(const void* p)
-{
-    uint2 r;
-    asm volatile("ld.global.nc.v2.u32 {%0, %1}, [%2];" : "=r"(r.x), "=r"(r.y) : "l"(p));
+    unsigned r;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(r) : "r"(addr));
     return r;
 }
-
+__device__ __forceinline__ uint2 lds_v2(unsigned addr)
+{
+    uint2 r;
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(r.x), "=r"(r.y) : "r"(addr));
+    return r;
+}
+__device__ __forceinline__ uint4 lds_v4(unsigned addr)
+{
+    uint4 r;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
+                 : "r"(addr));
+    return r;
+}
+// One level's data of a lane: window byte offsets (32-bit words, or W16 two
+// 16-bit ones to a word) and factor values of the steps, the row's record,
+// destination and right-hand side.
 template <int SMAX, bool W16>
-__device__ __forceinline__ void reg_load(RegSet<SMAX, W16>& S, const unsigned char* p,
-                                         const float* bsrc, int lane)
-{
-    constexpr int ob = W16 ? 256 : 512;
-    S.gm = nc_v4f(p + lane * 16);
-    S.go = nc_i(p + 512 + lane * 4);
-    S.b = nc_f(bsrc);
-#pragma unroll
-    for (int k = 0; k < SMAX / 4; ++k) {
-        if constexpr (W16) S.off[k].o = nc_v2u(p + kRegLaneTab + k * 256 + lane * 8);
-        else S.off[k].o = nc_v4u(p + kRegLaneTab + k * 512 + lane * 16);
-        S.val[k] = nc_v4f(p + kRegLaneTab + (SMAX / 4) * ob + k * 512 + lane * 16);
+struct RegSet {
+    unsigned off[W16 ? SMAX / 2 : SMAX];
+    float val[SMAX];
+    float gm[3];
+    int wo, go;
+    float b;
+    __device__ __forceinline__ unsigned at(int st) const
+    {
+        if constexpr (W16) return (st & 1) ? (off[st / 2] >> 16) : (off[st / 2] & 0xffffu);
+        else return off[st];
     }
-}
+};
 
+// The slot at p and the row's right-hand side at pb (shared memory).
 template <int H, int SMAX, bool W16>
-__device__ __forceinline__ void reg_level(const RegSet<SMAX, W16>& S, unsigned wbase, float* win,
-                                          float* out, int lane0)
+__device__ __forceinline__ void reg_load(RegSet<SMAX, W16>& S, unsigned p, unsigned pb, int lane)
 {
-    // four accumulators: dependent chains of SMAX / 4 multiply-adds
-    float acc0 = 0.0f, acc1 = 0.0f, acc2 = 0.0f, acc3 = 0.0f;
+    constexpr unsigned RB = reg_rows_bytes(H), OB = reg_offs_bytes(SMAX, W16);
+    constexpr int F = SMAX / 4;
+    const unsigned po = p + RB, pv = p + RB + OB;
 #pragma unroll
-    for (int k = 0; k < SMAX / 4; ++k) {
-        const float x0 = lds_f(wbase + S.off[k].at(0)), x1 = lds_f(wbase + S.off[k].at(1));
-        const float x2 = lds_f(wbase + S.off[k].at(2)), x3 = lds_f(wbase + S.off[k].at(3));
-        acc0 = fmaf(S.val[k].x, x0, acc0);
-        acc1 = fmaf(S.val[k].y, x1, acc1);
-        acc2 = fmaf(S.val[k].z, x2, acc2);
-        acc3 = fmaf(S.val[k].w, x3, acc3);
+    for (int k = 0; k < F; ++k) {
+        if constexpr (W16) {
+            const uint2 o = lds_v2(po + k * 256 + lane * 8);
+            S.off[2 * k] = o.x;
+            S.off[2 * k + 1] = o.y;
+        } else {
+            const uint4 o = lds_v4(po + k * 512 + lane * 16);
+            S.off[4 * k] = o.x;
+            S.off[4 * k + 1] = o.y;
+            S.off[4 * k + 2] = o.z;
+            S.off[4 * k + 3] = o.w;
+        }
+        const uint4 v = lds_v4(pv + k * 512 + lane * 16);
+        S.val[4 * k] = __uint_as_float(v.x);
+        S.val[4 * k + 1] = __uint_as_float(v.y);
+        S.val[4 * k + 2] = __uint_as_float(v.z);
+        S.val[4 * k + 3] = __uint_as_float(v.w);
     }
-    float acc = (acc0 + acc1) + (acc2 + acc3);
-#pragma unroll
-    for (int m = 1; m < H; m <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
-    const float d = S.b - acc;
-    const float d0 = __shfl_sync(0xffffffffu, d, lane0);
-    const float d1 = __shfl_sync(0xffffffffu, d, lane0 + H);
-    const float d2 = __shfl_sync(0xffffffffu, d, lane0 + 2 * H);
-    const float sol = fmaf(S.gm.z, d2, fmaf(S.gm.y, d1, S.gm.x * d0));
-    const int wo = __float_as_int(S.gm.w);
-    if (wo >= 0) {
-        win[wo] = sol;
-        out[S.go] = sol;
+    if constexpr (SMAX % 4 != 0) {
+        if constexpr (W16) {
+            S.off[2 * F] = lds_u(po + F * 256 + lane * 4);
+        } else {
+            const uint2 o = lds_v2(po + F * 512 + lane * 8);
+            S.off[4 * F] = o.x;
+            S.off[4 * F + 1] = o.y;
+        }
+        const uint2 v = lds_v2(pv + F * 512 + lane * 8);
+        S.val[4 * F] = __uint_as_float(v.x);
+        S.val[4 * F + 1] = __uint_as_float(v.y);
     }
+    const uint4 g = lds_v4(p + (lane / H) * 16);
+    S.gm[0] = __uint_as_float(g.x);
+    S.gm[1] = __uint_as_float(g.y);
+    S.gm[2] = __uint_as_float(g.z);
+    S.wo = (int)g.w;
+    S.go = (int)lds_u(p + 16 * (32 / H) + (lane / H) * 4);
+    S.b = lds_f(pb);
 }
 
-// One temporal block tb of one sweep (one thread block).  DEP register
-// sets (2, 3 or 4): a set's loads have DEP - 1 levels of work to land in.
-template <int H, int SMAX, bool UPPER, bool W16, int DEP>
+// One temporal block tb of one sweep (one thread block of ncw + 1 warps).
+template <int H, int SMAX, bool UPPER, bool W16>
 __device__ __forceinline__ void tri_reg_body(const RegArgs& a, int tb)
 {
-    extern __shared__ __align__(16) float rwin[];
+    extern __shared__ __align__(128) unsigned char reg_mem[];
+    __shared__ unsigned long long bars[kRingParts];
     if (a.skip && a.skip[0] != 0) return;  // uniform: before any barrier
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    constexpr int GS = 3 * H;
-    const int lane0 = (lane / GS) * GS;
-    const unsigned wbase = (unsigned)__cvta_generic_to_shared(rwin);
-    float* out = UPPER ? a.out + tb : a.out + (size_t)tb * a.ostride;
+    constexpr int GS = 3 * H, RW = 32 / H;
+    constexpr unsigned SB = reg_slot_bytes(H, SMAX, W16);
+    float* rwin = reinterpret_cast<float*>(reg_mem);
+    const unsigned wbase = smem_addr(reg_mem);
+    const SweepRing ring(wbase + reg_pad((unsigned)a.win * 4u), smem_addr(bars), a.nr, a.nl, a.ncw, SB, RW * 4u);
     if (threadIdx.x < 3) rwin[a.zero_off + threadIdx.x] = 0.0f;
-    // this warp's slot and right-hand side advance by one level's worth
-    const size_t sstep = (size_t)a.ncw * a.slot_bytes;
-    const unsigned char* sp = a.slots + (size_t)warp * a.slot_bytes;
-    const float* bp = a.rhs + (size_t)tb * a.rstride + (size_t)warp * 32 + lane;
-    // L2 prefetch of the slot and right-hand side a.pf levels ahead of the
-    // register loads: the slots of a sweep are read once per apply, from
-    // DRAM, and the register loads alone do not cover DRAM latency.  Lane i
-    // touches the slot's 128-byte line i, lane 31 the right-hand-side line.
-    auto prefetch = [&](int L) {
-        if (a.pf > 0 && L < a.nl) {
-            const size_t o = (size_t)lane * 128;
-            if (o < (size_t)a.slot_bytes)
-                prefetch_l2(a.slots + ((size_t)L * a.ncw + warp) * a.slot_bytes + o);
-            else if (lane == 31)
-                prefetch_l2(a.rhs + (size_t)tb * a.rstride + ((size_t)L * a.ncw + warp) * 32);
-        }
-    };
-    for (int L = DEP; L < DEP + a.pf; ++L) prefetch(L);
-    // In the level loop the prefetch is a running pointer: the line this
-    // thread touches at level DEP + pf, advanced by one level's worth (no
-    // address arithmetic per level).  pfl: the loop's last level index l
-    // whose level l + DEP + pf exists.
-    const bool pf_slot = a.pf > 0 && lane * 128 < a.slot_bytes;
-    const bool pf_rhs = a.pf > 0 && !pf_slot && lane == 31;
-    const unsigned char* pp =
-        pf_slot ? a.slots + ((size_t)(DEP + a.pf) * a.ncw + warp) * a.slot_bytes + (size_t)lane * 128
-                : reinterpret_cast<const unsigned char*>(
-                      a.rhs + (size_t)tb * a.rstride + ((size_t)(DEP + a.pf) * a.ncw + warp) * 32);
-    const size_t pstep = pf_slot ? sstep : (size_t)a.ncw * 32 * sizeof(float);
-    const bool pf_on = pf_slot || pf_rhs;
-    const int pfl = a.nl - DEP - a.pf;
-    // one level: compute it with set S, reload S with the level DEP ahead,
-    // prefetch, advance, barrier
-    auto level = [&](RegSet<SMAX, W16>& S, int lk) {
-        reg_level<H, SMAX, W16>(S, wbase, rwin, out, lane0);
-        if (lk + DEP < a.nl) reg_load<SMAX, W16>(S, sp, bp, lane);
-        if (pf_on && lk < pfl) prefetch_l2(pp);
-        pp += pstep;
-        sp += sstep;
-        bp += a.ncw * 32;
-        level_barrier();
-    };
-    if constexpr (DEP == 4) {
-        // four register sets, four levels per trip
-        RegSet<SMAX, W16> s0, s1, s2, s3;
-        reg_load<SMAX, W16>(s0, sp, bp, lane);
-        if (a.nl > 1) reg_load<SMAX, W16>(s1, sp + sstep, bp + a.ncw * 32, lane);
-        if (a.nl > 2) reg_load<SMAX, W16>(s2, sp + 2 * sstep, bp + 2 * a.ncw * 32, lane);
-        if (a.nl > 3) reg_load<SMAX, W16>(s3, sp + 3 * sstep, bp + 3 * a.ncw * 32, lane);
-        sp += 4 * sstep;
-        bp += 4 * a.ncw * 32;
-        level_barrier();  // the zero slot is set
-        for (int l = 0; l < a.nl; l += 4) {
-            level(s0, l);
-            if (l + 1 < a.nl) level(s1, l + 1);
-            if (l + 2 < a.nl) level(s2, l + 2);
-            if (l + 3 < a.nl) level(s3, l + 3);
-        }
+    if (threadIdx.x == 0) ring.init();
+    __syncthreads();
+    if (warp == a.ncw) {
+        if (!ring.copies(a.slots, reinterpret_cast<const unsigned char*>(a.rhs + (size_t)tb * a.rstride), lane))
+            g_ilu_error = 1;
         return;
     }
-    if constexpr (DEP == 3) {
-        // three register sets, three levels per trip
-        RegSet<SMAX, W16> s0, s1, s2;
-        reg_load<SMAX, W16>(s0, sp, bp, lane);
-        if (a.nl > 1) reg_load<SMAX, W16>(s1, sp + sstep, bp + a.ncw * 32, lane);
-        if (a.nl > 2) reg_load<SMAX, W16>(s2, sp + 2 * sstep, bp + 2 * a.ncw * 32, lane);
-        sp += 3 * sstep;
-        bp += 3 * a.ncw * 32;
-        level_barrier();  // the zero slot is set
-        for (int l = 0; l < a.nl; l += 3) {
-            reg_level<H, SMAX, W16>(s0, wbase, rwin, out, lane0);
-            if (l + 3 < a.nl) reg_load<SMAX, W16>(s0, sp, bp, lane);
-            if (pf_on && l < pfl) prefetch_l2(pp);
-            pp += pstep;
-            sp += sstep;
-            bp += a.ncw * 32;
-            level_barrier();
-            if (l + 1 < a.nl) {
-                reg_level<H, SMAX, W16>(s1, wbase, rwin, out, lane0);
-                if (l + 4 < a.nl) reg_load<SMAX, W16>(s1, sp, bp, lane);
-                if (pf_on && l + 1 < pfl) prefetch_l2(pp);
-                pp += pstep;
-                sp += sstep;
-                bp += a.ncw * 32;
-                level_barrier();
-            }
-            if (l + 2 < a.nl) {
-                reg_level<H, SMAX, W16>(s2, wbase, rwin, out, lane0);
-                if (l + 5 < a.nl) reg_load<SMAX, W16>(s2, sp, bp, lane);
-                if (pf_on && l + 2 < pfl) prefetch_l2(pp);
-                pp += pstep;
-                sp += sstep;
-                bp += a.ncw * 32;
-                level_barrier();
-            }
-        }
-        return;
-    }
-    // two register sets, a pair of levels per trip: the set a level used is
-    // reloaded, right after it, with the level two ahead
-    RegSet<SMAX, W16> s0, s1;
-    reg_load<SMAX, W16>(s0, sp, bp, lane);
-    if (a.nl > 1) reg_load<SMAX, W16>(s1, sp + sstep, bp + a.ncw * 32, lane);
-    sp += 2 * sstep;
-    bp += 2 * a.ncw * 32;
-    level_barrier();  // the zero slot is set
+    const int lane0 = (lane / GS) * GS;
+    float* out = UPPER ? a.out + tb : a.out + (size_t)tb * a.ostride;
+    RegSet<SMAX, W16> R[2];
+    RingReader rd(ring, (unsigned)warp * SB, (unsigned)(warp * RW + lane / H) * 4u);
+    auto fetch = [&](RegSet<SMAX, W16>& S) {
+        rd.enter(ring);
+        reg_load<H, SMAX, W16>(S, rd.s, rd.b, lane);
+        rd.next(ring);
+    };
+    float psol = 0.0f;
+    int pgo = -1;  // the last level's result, on its way to global memory
+    const bool owner = lane % H == 0;
+    // one level: its window reads; behind them the next level's entry into nx
+    // (beyond the last level: old data, read and not used) and the last
+    // level's results to global memory; its sums
+    auto level = [&](const RegSet<SMAX, W16>& S, RegSet<SMAX, W16>& nx) {
+        float x[SMAX];
+#pragma unroll
+        for (int st = 0; st < SMAX; ++st) x[st] = lds_f(wbase + S.at(st));
+        fetch(nx);
+        if (pgo >= 0) out[pgo] = psol;
+        // four accumulators: dependent chains of SMAX / 4 multiply-adds
+        float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+        for (int st = 0; st < SMAX; ++st) acc[st & 3] = fmaf(S.val[st], x[st], acc[st & 3]);
+        float sum = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+#pragma unroll
+        for (int m = 1; m < H; m <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, m);
+        const float d = S.b - sum;
+        const float d0 = __shfl_sync(0xffffffffu, d, lane0);
+        const float d1 = __shfl_sync(0xffffffffu, d, lane0 + H);
+        const float d2 = __shfl_sync(0xffffffffu, d, lane0 + 2 * H);
+        psol = fmaf(S.gm[2], d2, fmaf(S.gm[1], d1, S.gm[0] * d0));
+        const bool own = owner && S.wo >= 0;
+        if (own) rwin[S.wo] = psol;
+        pgo = own ? S.go : -1;
+        ring_level(ring.computing());
+        rd.used(ring);
+    };
+    fetch(R[0]);
     for (int l = 0; l < a.nl; l += 2) {
-        reg_level<H, SMAX, W16>(s0, wbase, rwin, out, lane0);
-        if (l + 2 < a.nl) reg_load<SMAX, W16>(s0, sp, bp, lane);
-        if (pf_on && l < pfl) prefetch_l2(pp);
-        pp += pstep;
-        sp += sstep;
-        bp += a.ncw * 32;
-        level_barrier();
-        if (l + 1 < a.nl) {
-            reg_level<H, SMAX, W16>(s1, wbase, rwin, out, lane0);
-            if (l + 3 < a.nl) reg_load<SMAX, W16>(s1, sp, bp, lane);
-            if (pf_on && l + 1 < pfl) prefetch_l2(pp);
-            pp += pstep;
-            sp += sstep;
-            bp += a.ncw * 32;
-            level_barrier();
-        }
+        level(R[0], R[1]);
+        if (l + 1 < a.nl) level(R[1], R[0]);
     }
+    if (pgo >= 0) out[pgo] = psol;
 }
 
-// Warps of a sweep with DEP register sets: at most 12 for four sets leave
-// each thread the registers (131) the sets need.
-__host__ __device__ constexpr int reg_max_warps(int dep)
+template <int H, int SMAX, bool UPPER, bool W16>
+__global__ void __launch_bounds__((kRegMaxWarps + 1) * 32, 1) k_tri_reg(RegArgs a)
 {
-    return dep <= 3 ? kRegMaxWarps : 12;
-}
-
-template <int H, int SMAX, bool UPPER, bool W16, int DEP>
-__global__ void __launch_bounds__(reg_max_warps(DEP) * 32, 1)
-    k_tri_reg(RegArgs a)
-{
-    tri_reg_body<H, SMAX, UPPER, W16, DEP>(a, blockIdx.x);
+    tri_reg_body<H, SMAX, UPPER, W16>(a, blockIdx.x);
 }
 
 // One thread block per (entry, temporal block): entry blockIdx.x / q of the
 // table, temporal block blockIdx.x % q.  The entries are the row blocks of
 // a block-Jacobi factor (the output and the skip flag are the launch's) or
-// the sweeps of a batch of systems (each entry's own); the prefetch
-// distance is the launch's.
+// the sweeps of a batch of systems (each entry's own).
 template <int H, int SMAX, bool UPPER, bool W16>
-__global__ void __launch_bounds__(kRegMaxWarps * 32, 1)
-    k_tri_reg_parts(const RegArgs* __restrict__ args, int q, int pf, const int* skip, float* out)
+__global__ void __launch_bounds__((kRegMaxWarps + 1) * 32, 1)
+    k_tri_reg_parts(const RegArgs* __restrict__ args, int q, const int* skip, float* out)
 {
     RegArgs a = args[blockIdx.x / q];
-    a.pf = pf;
     if (skip) a.skip = skip;
     if (out) a.out = out;
-    tri_reg_body<H, SMAX, UPPER, W16, 2>(a, blockIdx.x % q);
+    tri_reg_body<H, SMAX, UPPER, W16>(a, blockIdx.x % q);
 }
 
-// Forward-sweep right-hand sides in lane-slot order, one array per temporal
+// Forward-sweep right-hand sides in row order, one array per temporal
 // block: rhs[q][s] = sum_j Ainv(q, j) v(row(s), j) (0 for unused slots).
 template <int Q>
 __global__ void k_rhs_slots(const int* __restrict__ src, long long lanes,
@@ -2022,6 +1955,11 @@ int build_reg_parts(const DevIlu& F, int Q, int H, IluStage& st, cudaStream_t s)
     const int smax = reg_smax(H, need);
     if (smax == 0) return XT_OK;
     const bool w16 = (long long)win * 4 <= 65536 && env_int("XTFEM_ILU_W16", 1) != 0;
+    for (auto* v : {&Ls, &Us})
+        for (auto& t : *v) {
+            t->nr = reg_ring(*t, smax, w16, (long long)max_dyn_smem() - kRegStatic);
+            if (t->nr == 0) return XT_OK;
+        }
     std::vector<long long> offL(P + 1, 0), offU(P + 1, 0);
     for (int b = 0; b < P; ++b) {
         offL[b + 1] = offL[b] + Ls[b]->lanes;
@@ -2046,11 +1984,13 @@ int build_reg_parts(const DevIlu& F, int Q, int H, IluStage& st, cudaStream_t s)
     XT_TRY(st.rrhsU.alloc((size_t)Q * offU[P]));
     XT_CUDA(cudaMemsetAsync(st.rrhsU.p, 0, sizeof(float) * Q * offU[P], s));
     std::vector<RegArgs> aL(P), aU(P);
+    size_t smem = 0;
     for (int b = 0; b < P; ++b) {
         aL[b] = RegArgs{Ls[b]->slots.p, st.rrhsL.p + offL[b], nullptr, offL[P], offU[P],
-                        Ls[b]->nl, ncw, Ls[b]->slot_bytes, Ls[b]->zero_off, 0, nullptr};
+                        Ls[b]->nl, ncw, Ls[b]->win_elems, Ls[b]->nr, Ls[b]->zero_off, nullptr};
         aU[b] = RegArgs{Us[b]->slots.p, st.rrhsU.p + offU[b], nullptr, offU[P], 0,
-                        Us[b]->nl, ncw, Us[b]->slot_bytes, Us[b]->zero_off, 0, nullptr};
+                        Us[b]->nl, ncw, Us[b]->win_elems, Us[b]->nr, Us[b]->zero_off, nullptr};
+        smem = std::max(smem, std::max(reg_smem(*Ls[b]), reg_smem(*Us[b])));
     }
     XT_TRY(st.argsL.upload(reinterpret_cast<const unsigned char*>(aL.data()), sizeof(RegArgs) * P, s));
     XT_TRY(st.argsU.upload(reinterpret_cast<const unsigned char*>(aU.data()), sizeof(RegArgs) * P, s));
@@ -2067,7 +2007,7 @@ int build_reg_parts(const DevIlu& F, int Q, int H, IluStage& st, cudaStream_t s)
     }
     st.parts = P;
     st.ncw = ncw;
-    st.win_elems = win;
+    st.smem = smem;
     st.lanesL = offL[P];
     st.lanesU = offU[P];
     st.regLp = Ls;
@@ -2078,50 +2018,53 @@ int build_reg_parts(const DevIlu& F, int Q, int H, IluStage& st, cudaStream_t s)
     return XT_OK;
 }
 
-template <int Q, int H, int SMAX, bool W16, int DEP = 2>
+// Measured (GB300, both sweeps and the pre-pass, q = 6), before with the slots
+// read from global memory straight into registers: 20 x 20 x 60 rod 605 -> 471
+// us, 10 x 10 x 30 rod 161 -> 153 us, 4 x 4 x 12 rod 72.6 -> 62.6 us.
+template <int Q, int H, int SMAX, bool W16>
 int launch_reg(const IluStage& st, const double* dAinv, const float* v, float* z, cudaStream_t s,
                const int* skip)
 {
-    static std::atomic<bool> attr{false};
-    if (!attr.load(std::memory_order_acquire)) {
-        XT_CUDA(cudaFuncSetAttribute(k_tri_reg<H, SMAX, false, W16, DEP>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem()));
-        XT_CUDA(cudaFuncSetAttribute(k_tri_reg<H, SMAX, true, W16, DEP>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem()));
-        attr.store(true, std::memory_order_release);
-    }
-    const int pf = std::max(0, std::min(64, env_int("XTFEM_ILU_PF", 8)));
+    const int dyn = max_dyn_smem() - (int)kRegStatic;
     if (st.parts > 1) {
         static std::atomic<bool> pattr{false};
         if (!pattr.load(std::memory_order_acquire)) {
             XT_CUDA(cudaFuncSetAttribute(k_tri_reg_parts<H, SMAX, false, W16>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem()));
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
             XT_CUDA(cudaFuncSetAttribute(k_tri_reg_parts<H, SMAX, true, W16>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem()));
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
             pattr.store(true, std::memory_order_release);
         }
         const int nb = (int)std::max(1LL, std::min<long long>((st.lanesL + 255) / 256, 152LL * 8));
         k_rhs_slots<Q><<<nb, 256, 0, s>>>(st.srcL.p, st.lanesL, dAinv, v, st.rrhsL.p, skip);
         const RegArgs* aL = reinterpret_cast<const RegArgs*>(st.argsL.p);
         const RegArgs* aU = reinterpret_cast<const RegArgs*>(st.argsU.p);
-        const size_t smem = (size_t)st.win_elems * 4;
-        k_tri_reg_parts<H, SMAX, false, W16><<<Q * st.parts, st.ncw * 32, smem, s>>>(aL, Q, pf, skip,
-                                                                                  st.rrhsU.p);
-        k_tri_reg_parts<H, SMAX, true, W16><<<Q * st.parts, st.ncw * 32, smem, s>>>(aU, Q, pf, skip, z);
+        const int threads = (st.ncw + 1) * 32;
+        k_tri_reg_parts<H, SMAX, false, W16><<<Q * st.parts, threads, st.smem, s>>>(aL, Q, skip,
+                                                                                 st.rrhsU.p);
+        k_tri_reg_parts<H, SMAX, true, W16><<<Q * st.parts, threads, st.smem, s>>>(aU, Q, skip, z);
         note_launches(3);
         XT_CUDA(cudaGetLastError());
         return XT_OK;
+    }
+    static std::atomic<bool> attr{false};
+    if (!attr.load(std::memory_order_acquire)) {
+        XT_CUDA(cudaFuncSetAttribute(k_tri_reg<H, SMAX, false, W16>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
+        XT_CUDA(cudaFuncSetAttribute(k_tri_reg<H, SMAX, true, W16>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
+        attr.store(true, std::memory_order_release);
     }
     const RegTri& L = *st.regL;
     const RegTri& U = *st.regU;
     const int nblk = (int)std::max(1LL, std::min<long long>((L.lanes + 255) / 256, 152LL * 8));
     k_rhs_slots<Q><<<nblk, 256, 0, s>>>(st.srcL.p, L.lanes, dAinv, v, st.rrhsL.p, skip);
-    RegArgs aL{L.slots.p, st.rrhsL.p, st.rrhsU.p, L.lanes, U.lanes, L.nl, L.ncw, L.slot_bytes,
-               L.zero_off, pf, skip};
-    RegArgs aU{U.slots.p, st.rrhsU.p, z, U.lanes, 0, U.nl, U.ncw, U.slot_bytes, U.zero_off, pf,
-               skip};
-    k_tri_reg<H, SMAX, false, W16, DEP><<<Q, L.ncw * 32, (size_t)L.win_elems * 4, s>>>(aL);
-    k_tri_reg<H, SMAX, true, W16, DEP><<<Q, U.ncw * 32, (size_t)U.win_elems * 4, s>>>(aU);
+    const RegArgs aL{L.slots.p, st.rrhsL.p, st.rrhsU.p, L.lanes, U.lanes, L.nl, L.ncw, L.win_elems,
+                     L.nr, L.zero_off, skip};
+    const RegArgs aU{U.slots.p, st.rrhsU.p, z, U.lanes, 0, U.nl, U.ncw, U.win_elems, U.nr,
+                     U.zero_off, skip};
+    k_tri_reg<H, SMAX, false, W16><<<Q, (L.ncw + 1) * 32, reg_smem(L), s>>>(aL);
+    k_tri_reg<H, SMAX, true, W16><<<Q, (U.ncw + 1) * 32, reg_smem(U), s>>>(aU);
     note_launches(3);
     XT_CUDA(cudaGetLastError());
     return XT_OK;
@@ -2136,17 +2079,6 @@ int launch_reg_width(const IluStage& st, const double* dAinv, const float* v, fl
         set_error("register sweep: triangles with different offset widths");
         return XT_ERR_STATE;
     }
-    // four register sets (16-bit offsets, at most 12 steps per lane and 12
-    // warps), else three; XTFEM_ILU_DEPTH=2 or 3 caps them
-    if constexpr (SMAX <= 12) {
-        const int dep = env_int("XTFEM_ILU_DEPTH", 4);
-        const int w = std::max(st.regL->ncw, st.regU->ncw);
-        if (st.regL->w16 && st.parts <= 1) {
-            if (dep >= 4 && w <= reg_max_warps(4))
-                return launch_reg<Q, H, SMAX, true, 4>(st, dAinv, v, z, s, skip);
-            if (dep >= 3) return launch_reg<Q, H, SMAX, true, 3>(st, dAinv, v, z, s, skip);
-        }
-    }
     if (st.regL->w16) return launch_reg<Q, H, SMAX, true>(st, dAinv, v, z, s, skip);
     return launch_reg<Q, H, SMAX, false>(st, dAinv, v, z, s, skip);
 }
@@ -2157,6 +2089,7 @@ int launch_reg_any(const IluStage& st, const double* dAinv, const float* v, floa
 {
     const int H = st.regL->H, smax = st.regL->smax;
     if (H == 2 && smax == 8) return launch_reg_width<Q, 2, 8>(st, dAinv, v, z, s, skip);
+    if (H == 2 && smax == 10) return launch_reg_width<Q, 2, 10>(st, dAinv, v, z, s, skip);
     if (H == 2 && smax == 12) return launch_reg_width<Q, 2, 12>(st, dAinv, v, z, s, skip);
     if (H == 2 && smax == 16) return launch_reg_width<Q, 2, 16>(st, dAinv, v, z, s, skip);
     if (H == 1 && smax == 12) return launch_reg_width<Q, 1, 12>(st, dAinv, v, z, s, skip);
@@ -2496,7 +2429,7 @@ namespace {
 // launch_reg_any dispatches them).
 bool reg_pair_ok(int H, int smax)
 {
-    return (H == 2 && (smax == 8 || smax == 12 || smax == 16)) || (H == 1 && (smax == 12 || smax == 20)) ||
+    return (H == 2 && (smax == 8 || smax == 10 || smax == 12 || smax == 16)) || (H == 1 && (smax == 12 || smax == 20)) ||
            (H == 4 && smax == 8);
 }
 
@@ -2507,11 +2440,11 @@ int reg_group_hs(const RegGroup& g, int q, cudaStream_t s, bool prepare)
     auto kernel = g.upper ? (g.w16 ? k_tri_reg_parts<H, SMAX, true, true> : k_tri_reg_parts<H, SMAX, true, false>)
                           : (g.w16 ? k_tri_reg_parts<H, SMAX, false, true> : k_tri_reg_parts<H, SMAX, false, false>);
     if (prepare) {
-        XT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem()));
+        XT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     max_dyn_smem() - (int)kRegStatic));
         return XT_OK;
     }
-    const int pf = std::max(0, std::min(64, env_int("XTFEM_ILU_PF", 8)));
-    kernel<<<q * g.count, g.ncw * 32, g.smem, s>>>(a, q, pf, nullptr, nullptr);
+    kernel<<<q * g.count, (g.ncw + 1) * 32, g.smem, s>>>(a, q, nullptr, nullptr);
     note_launches(1);
     XT_CUDA(cudaGetLastError());
     return XT_OK;
@@ -2520,11 +2453,12 @@ int reg_group_hs(const RegGroup& g, int q, cudaStream_t s, bool prepare)
 int reg_group_any(const RegGroup& g, int q, cudaStream_t s, bool prepare)
 {
     if (g.count < 1 || g.ncw < 1 || g.ncw > kRegMaxWarps || (long long)q * g.count > INT32_MAX ||
-        g.smem > (size_t)max_dyn_smem() || !g.args.p) {
+        g.smem > (size_t)(max_dyn_smem() - kRegStatic) || !g.args.p) {
         set_error("register sweep group: bad shape");
         return XT_ERR_ARG;
     }
     if (g.H == 2 && g.smax == 8) return reg_group_hs<2, 8>(g, q, s, prepare);
+    if (g.H == 2 && g.smax == 10) return reg_group_hs<2, 10>(g, q, s, prepare);
     if (g.H == 2 && g.smax == 12) return reg_group_hs<2, 12>(g, q, s, prepare);
     if (g.H == 2 && g.smax == 16) return reg_group_hs<2, 16>(g, q, s, prepare);
     if (g.H == 1 && g.smax == 12) return reg_group_hs<1, 12>(g, q, s, prepare);
@@ -2548,19 +2482,18 @@ int ilu_reg_entry(const DevIlu& F, int q, float* z, const int* skip, cudaStream_
     const RegTri& L = *st->regL;
     const RegTri& U = *st->regU;
     if (L.w16 != U.w16 || L.H != U.H || L.smax != U.smax || !reg_pair_ok(L.H, L.smax)) return XT_OK;
-    const int pf = std::max(0, std::min(64, env_int("XTFEM_ILU_PF", 8)));
     e.src = st->srcL.p;
     e.lanes = L.lanes;
     e.rrhs = st->rrhsL.p;
     e.H = L.H;
     e.smax = L.smax;
     e.w16 = L.w16 ? 1 : 0;
-    e.L = RegArgs{L.slots.p, st->rrhsL.p, st->rrhsU.p, L.lanes, U.lanes, L.nl, L.ncw,
-                  L.slot_bytes, L.zero_off, pf, skip};
-    e.U = RegArgs{U.slots.p, st->rrhsU.p, z, U.lanes, 0, U.nl, U.ncw, U.slot_bytes, U.zero_off,
-                  pf, skip};
-    e.smemL = (size_t)L.win_elems * 4;
-    e.smemU = (size_t)U.win_elems * 4;
+    e.L = RegArgs{L.slots.p, st->rrhsL.p, st->rrhsU.p, L.lanes, U.lanes, L.nl, L.ncw, L.win_elems,
+                  L.nr, L.zero_off, skip};
+    e.U = RegArgs{U.slots.p, st->rrhsU.p, z, U.lanes, 0, U.nl, U.ncw, U.win_elems, U.nr, U.zero_off,
+                  skip};
+    e.smemL = reg_smem(L);
+    e.smemU = reg_smem(U);
     e.ok = true;
     return XT_OK;
 }

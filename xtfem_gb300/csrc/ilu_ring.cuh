@@ -1,0 +1,182 @@
+// ilu_ring.cuh -- the shared-memory ring of the triangular sweeps that keep a
+// level's data in registers ahead (dev_ilu.cu, dev_ilu_rows.cu).
+//
+// One warp of the thread block copies levels (the slots of all computing
+// warps, then their right-hand sides) into a ring of kRingParts parts of B
+// levels with cp.async.bulk, an mbarrier per part, waits for each part and
+// announces it on a named barrier; the computing warps read their entries
+// from it.  The copying warp takes no part in the levels: starting a copy
+// takes it about 200 cycles and an mbarrier wait 180 however long ago the copy
+// landed (joined to every level barrier it made a level of one warp 730 cycles
+// long).  Its waits are bounded: one that gives up raises the error word that
+// ilu_check reads, starts no further copy, lets the remaining levels run on
+// what is there and leaves once the copies have landed.
+//
+// Named barriers: 1 levels (the computing warps); 2, 3 a part has landed
+// (even, odd parts); 4, 5 a part has been read.  Both sides take part in every
+// part's barriers, so that no warp arrives twice in a phase.
+#pragma once
+
+namespace xt {
+
+constexpr int kRingParts = 4;
+constexpr int kRingSpin = 1 << 20;  // polls of a wait before it gives up
+
+__device__ __forceinline__ void ring_sync(int id, int threads)
+{
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void ring_arrive(int id, int threads)
+{
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+// The level barrier of the computing warps.
+__device__ __forceinline__ void ring_level(int threads)
+{
+    asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
+}
+
+struct SweepRing {
+    unsigned at;                   // shared-memory address of the ring
+    unsigned bars;                 // of the kRingParts mbarriers
+    unsigned lev_slots, lev_rhs;   // bytes of a level
+    int B, nl, nparts, ncw;
+    unsigned part_slots, part;     // bytes of a part's slots, of a part
+
+    __device__ __forceinline__ SweepRing(unsigned at_, unsigned bars_, int B_, int nl_, int ncw_,
+                                         unsigned slot_bytes, unsigned rhs_bytes)
+        : at(at_), bars(bars_), lev_slots((unsigned)ncw_ * slot_bytes),
+          lev_rhs((unsigned)ncw_ * rhs_bytes), B(B_), nl(nl_), nparts((nl_ + B_ - 1) / B_), ncw(ncw_)
+    {
+        part_slots = (unsigned)B * lev_slots;
+        part = part_slots + (unsigned)B * lev_rhs;
+    }
+    __device__ __forceinline__ int all() const { return (ncw + 1) * 32; }
+    __device__ __forceinline__ int computing() const { return ncw * 32; }
+
+    // one thread, before the block's first barrier
+    __device__ __forceinline__ void init() const
+    {
+        for (int k = 0; k < kRingParts; ++k)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bars + 8 * k) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __device__ __forceinline__ void copy(int m, const unsigned char* slots, const unsigned char* rhs) const
+    {
+        const unsigned bar = bars + 8u * (unsigned)(m % kRingParts);
+        const unsigned to = at + (unsigned)(m % kRingParts) * part;
+        const unsigned n = (unsigned)min(B, nl - m * B);
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
+                     "r"(n * (lev_slots + lev_rhs))
+                     : "memory");
+        asm volatile(
+            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(to),
+            "l"(slots + (size_t)m * part_slots), "r"(n * lev_slots), "r"(bar)
+            : "memory");
+        asm volatile(
+            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                to + part_slots),
+            "l"(rhs + (size_t)m * B * lev_rhs), "r"(n * lev_rhs), "r"(bar)
+            : "memory");
+    }
+    __device__ __forceinline__ bool wait(int m) const
+    {
+        const unsigned bar = bars + 8u * (unsigned)(m % kRingParts), parity = (unsigned)(m / kRingParts) & 1u;
+        for (int i = 0; i < kRingSpin; ++i) {
+            unsigned ok;
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t"
+                "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                "selp.u32 %0, 1, 0, p;\n\t}"
+                : "=r"(ok)
+                : "r"(bar), "r"(parity)
+                : "memory");
+            if (ok) return true;
+        }
+        return false;
+    }
+    // the copying warp's whole work; false when a wait gave up
+    __device__ __forceinline__ bool copies(const unsigned char* slots, const unsigned char* rhs, int lane) const
+    {
+        int issued = min(kRingParts, nparts);
+        bool ok = true;
+        if (lane == 0)
+            for (int m = 0; m < issued; ++m) copy(m, slots, rhs);
+        for (int m = 0; m < nparts; ++m) {
+            if (lane == 0 && ok) ok = wait(m);
+            __syncwarp();
+            ring_arrive(2 + (m & 1), all());
+            // the part before has been read: its place takes the next copy
+            if (m > 0) {
+                ring_sync(4 + ((m - 1) & 1), all());
+                if (lane == 0 && ok && m - 1 + kRingParts < nparts) {
+                    copy(m - 1 + kRingParts, slots, rhs);
+                    issued = m + kRingParts;
+                }
+            }
+        }
+        if (lane == 0 && !ok)  // leave with no copy in flight
+            for (int m = max(0, issued - kRingParts); m < issued; ++m) (void)wait(m);
+        return ok;
+    }
+};
+
+// A computing warp's way through the ring: where its next entry is.
+struct RingReader {
+    unsigned s, b;  // addresses of the next entry's slot and right-hand sides
+    unsigned s0, b0, ep = 0;
+    int ni = 0, left, ready = 2;       // the next entry: level in its part, parts not announced yet
+    int ci = 0, after, done = 4;       // the level at hand: in its part, parts behind it
+
+    __device__ __forceinline__ RingReader(const SweepRing& r, unsigned slot_off, unsigned rhs_off)
+        : s0(r.at + slot_off), b0(r.at + r.part_slots + rhs_off), left(r.nparts), after(r.nparts - 1)
+    {
+        s = s0;
+        b = b0;
+    }
+    // before the next entry is read (beyond the last one: old data)
+    __device__ __forceinline__ void enter(const SweepRing& r)
+    {
+        if (ni == 0 && left > 0) {
+            ring_sync(ready, r.all());
+            ready ^= 1;  // 2, 3, 2, ...
+            --left;
+        }
+    }
+    // after it
+    __device__ __forceinline__ void next(const SweepRing& r)
+    {
+        s += r.lev_slots;
+        b += r.lev_rhs;
+        if (++ni == r.B) {
+            ni = 0;
+            ep = ep == (kRingParts - 1) * r.part ? 0u : ep + r.part;
+            s = s0 + ep;
+            b = b0 + ep;
+        }
+    }
+    // after the barrier of a level: its entry is in registers and used
+    __device__ __forceinline__ void used(const SweepRing& r)
+    {
+        if (++ci == r.B) {
+            ci = 0;
+            if (after > 0) ring_arrive(done, r.all());
+            done ^= 1;  // 4, 5, 4, ...
+            --after;
+        }
+    }
+};
+
+// Levels of a part: starting a part's copies and waiting for it takes the
+// copying warp about 600 cycles, so two levels (of 300 cycles and more), four
+// where a level is one small warp's (the ring then stays under 40 KB, and a
+// batch's blocks share their SMs); one where two do not fit in `room` bytes,
+// 0 where one does not.
+inline int ring_levels(long long level_bytes, long long room)
+{
+    const long long n = room / (level_bytes * kRingParts);
+    const long long want = level_bytes <= 3072 ? 4 : 2;
+    return (int)(n < want ? (n < 0 ? 0 : n) : want);
+}
+
+}  // namespace xt

@@ -301,18 +301,17 @@ int flexd_scale_copy(const int* ctl, const double* st, int im, const float2* w, 
 int flexd_solve(const int* ctl, double* st, int im, cudaStream_t s);
 
 // Arguments of one register sweep (one triangle of one factor or row block;
-// dev_ilu.cu): the slots, the right-hand sides in lane-slot order ([q]
-// arrays of rstride), the output (forward: the backward sweep's right-hand
-// sides, ostride apart; backward: z, interleaved), levels, warps, slot
-// bytes, the window's zero slot, the L2 prefetch distance in levels (0 off)
-// and an optional skip flag (nothing to do when skip[0] != 0).
+// dev_ilu.cu): the slots, the right-hand sides in row order ([q] arrays of
+// rstride), the output (forward: the backward sweep's right-hand sides,
+// ostride apart; backward: z, interleaved), levels, computing warps, window
+// elements, levels of a part of the ring, the window's zero slot and an
+// optional skip flag (nothing to do when skip[0] != 0).
 struct RegArgs {
     const unsigned char* slots;
     const float* rhs;
     float* out;
     long long rstride, ostride;
-    int nl, ncw, slot_bytes, zero_off;
-    int pf;
+    int nl, ncw, win, nr, zero_off;
     const int* skip;
 };
 // A system's default FP32 ILU apply as a batch entry: the pre-pass's lane
@@ -326,7 +325,7 @@ struct IluRegEntry {
     float* rrhs = nullptr;     // forward right-hand sides, [q][lanes]
     int H = 0, smax = 0, w16 = 0;
     RegArgs L{}, U{};
-    size_t smemL = 0, smemU = 0;  // window bytes
+    size_t smemL = 0, smemU = 0;  // dynamic shared memory
 };
 int ilu_reg_entry(const DevIlu& F, int q, float* z, const int* skip, cudaStream_t s,
                   IluRegEntry& e);
