@@ -1,8 +1,8 @@
-"""The row-record triangular sweeps (FP64 factors; FP32 factors of one
-unknown per node) against the oracle's kronlusol: every number of lanes per
-row, one warp (each level split in sub-levels) and the default, one, three and
-six temporal blocks, on rods whose level widths fall below, on and above the
-groups of a warp.  Tolerances as in test_gpu_parity: 1e-10 in FP64 (the same
+"""The triangular sweeps of FP64 factors (row records) and of FP32 factors of
+one unknown per node (register sweep) against the oracle's kronlusol: every
+number of lanes per row, one warp (each level split in sub-levels) and the
+default, one, three and six temporal blocks, on rods whose level widths fall
+below, on and above the groups of a warp.  Tolerances as in test_gpu_parity: 1e-10 in FP64 (the same
 factor and inverted diagonal blocks in another summation order), 1e-4 in FP32
 (the factor itself is rounded)."""
 import numpy as np
@@ -29,7 +29,7 @@ def rod(request, xt):
 @pytest.mark.parametrize("group,fp32", [(1, False), (3, False), (1, True)])
 def test_row_sweep_matches_oracle(xt, orc, rod, monkeypatch, group, fp32, shares, warps, q):
     if shares:
-        monkeypatch.setenv("XTFEM_ILU_ROW_H", str(shares))
+        monkeypatch.setenv("XTFEM_ILU_SHARES" if fp32 else "XTFEM_ILU_ROW_H", str(shares))
     if warps:
         monkeypatch.setenv("XTFEM_ILU_WARPS", str(warps))
     A = rod["A"][:q, :q]

@@ -1406,18 +1406,18 @@ __global__ void __launch_bounds__(kStageThreads, 1) k_tri_col(StageArgs<float> a
 
 // ---------------------------------------------------------------------------
 // Row sweep with a level's data in registers ahead ("register sweep"; FP32,
-// g = 3; the default for FP32).
+// groups of g = 3 rows or of one; the default for FP32).
 //
 // One thread block per temporal block (Q blocks per sweep, each on its own
 // SM), each the whole level chain, as the column format, in rows: a level
 // has no branch, every warp has a fixed-size slot at every level.
 //
 // Layout.  Lane = (group of the warp's chunk, row r of the group, share h
-// of the row's entries, H shares): lanes g*3H + r*H + h; a lane owns a
+// of the row's entries, H shares): lanes k g H + r H + h; a lane owns a
 // share of the row's off-diagonal entries, one per step, SMAX steps (an
 // even number; entries past the lane's own read an all-zero window slot
 // with value 0).  The groups of a level are sorted by their longest row
-// and dealt to chunks of 32/(3H) groups; a level with more chunks than the
+// and dealt to chunks of 32/(g H) groups; a level with more chunks than the
 // ncw warps is split into consecutive sub-levels (its groups are
 // independent).  Chunk w of (sub-)level l sits in the fixed slot l*ncw + w;
 // warps without a chunk at a level get an empty slot.  A slot holds, per
@@ -1472,6 +1472,7 @@ struct RegTri {
     int win_elems = 0, zero_off = 0;
     bool w16 = false;  // 16-bit window byte offsets (window <= 64 KB)
     int nr = 0;  // levels of a part of the ring
+    int g = 3;   // rows of a group
     long long lanes = 0;  // nl * ncw * 32 / H: places of right-hand sides
     DBuf<unsigned char> slots;
     std::vector<int> row_slot;             // host: right-hand-side place of each row
@@ -1495,8 +1496,9 @@ int reg_warps(const TriHost& h, int GPW)
 // Chunks, sub-levels, slots and steps of one triangle (no device data yet).
 bool reg_plan(const TriHost& h, int H, RegTri& t, int force_ncw = 0)
 {
-    const int g = 3, GS = 3 * H, GPW = 32 / GS;
+    const int g = h.g, GPW = 32 / (g * H);
     t.H = H;
+    t.g = g;
     t.ncw = force_ncw > 0 ? force_ncw : reg_warps(h, GPW);
     t.row_slot.assign((size_t)h.ngroups * g, -1);
     t.chunks.clear();
@@ -1507,7 +1509,11 @@ bool reg_plan(const TriHost& h, int H, RegTri& t, int force_ncw = 0)
     auto rowlen = [&](int i, int r) {
         return h.ext_ptr[(size_t)i * g + r + 1] - h.ext_ptr[(size_t)i * g + r];
     };
-    auto longest = [&](int i) { return std::max(rowlen(i, 0), std::max(rowlen(i, 1), rowlen(i, 2))); };
+    auto longest = [&](int i) {
+        int m = 0;
+        for (int r = 0; r < g; ++r) m = std::max(m, rowlen(i, r));
+        return m;
+    };
     for (int l = 0; l < h.nlevels; ++l) {
         const int gb = h.level_ptr[l], ng = h.level_ptr[l + 1] - gb;
         ord.resize(ng);
@@ -1562,7 +1568,7 @@ constexpr long long kRegStatic = 2048;  // static shared memory of a sweep, at m
 int reg_fill(const TriHost& h, RegTri& t, int smax, int Q, const std::vector<int>* dst,
              cudaStream_t s, int row0 = 0)
 {
-    const int g = 3, H = t.H, GS = 3 * H, GPW = 32 / GS;
+    const int g = t.g, H = t.H, GS = g * H, GPW = 32 / GS;
     t.smax = smax;
     const unsigned rb = reg_rows_bytes(H), ob = reg_offs_bytes(smax, t.w16);
     const int rw = 32 / H;  // row records of a slot
@@ -1601,7 +1607,7 @@ int reg_fill(const TriHost& h, RegTri& t, int smax, int Q, const std::vector<int
             const int i = grp[gw], G = h.order[i];
             if (hh == 0) {
                 const int rec = gw * g + r, wo = h.slot[G] * g + r;
-                for (int k = 0; k < 3; ++k) gm[rec * 4 + k] = (float)h.minv[(size_t)i * 9 + r * 3 + k];
+                for (int k = 0; k < g; ++k) gm[rec * 4 + k] = (float)h.minv[((size_t)i * g + r) * g + k];
                 std::memcpy(&gm[rec * 4 + 3], &wo, 4);
                 const long long d = dst ? (long long)(*dst)[(size_t)G * g + r]
                                         : ((long long)row0 + (long long)G * g + r) * Q;
@@ -1674,7 +1680,7 @@ int reg_smax(int H, int need)
 int build_reg(const IluSched& S, int Q, int H, IluStage& st, cudaStream_t s)
 {
     st.reg_ok = false;
-    if (S.L.g != 3 || (H != 1 && H != 2 && H != 4)) return XT_OK;
+    if ((S.L.g != 3 && S.L.g != 1) || (H != 1 && H != 2 && H != 4)) return XT_OK;
     auto L = std::make_shared<RegTri>(), U = std::make_shared<RegTri>();
     // the triangles are planned side by side, then filled side by side (the
     // forward fill reads the backward triangle's row slots, set by its plan)
@@ -1688,6 +1694,7 @@ int build_reg(const IluSched& S, int Q, int H, IluStage& st, cudaStream_t s)
     // (XTFEM_ILU_W16=0: 32-bit)
     const bool w16 = (long long)std::max(L->win_elems, U->win_elems) * 4 <= 65536 &&
                      env_int("XTFEM_ILU_W16", 1) != 0;
+    if (S.L.g == 1 && !w16) return XT_OK;  // compiled for 16-bit offsets only
     // fewer warps (more sub-levels) where the ring does not fit
     const long long room = (long long)max_dyn_smem() - kRegStatic;
     auto fit = [&](const TriHost& h, RegTri& t) {
@@ -1811,19 +1818,19 @@ __device__ __forceinline__ void reg_load(RegSet<SMAX, W16>& S, unsigned p, unsig
 }
 
 // One temporal block tb of one sweep (one thread block of ncw + 1 warps).
-template <int H, int SMAX, bool UPPER, bool W16>
+template <int G, int H, int SMAX, bool UPPER, bool W16>
 __device__ __forceinline__ void tri_reg_body(const RegArgs& a, int tb)
 {
     extern __shared__ __align__(128) unsigned char reg_mem[];
     __shared__ unsigned long long bars[kRingParts];
     if (a.skip && a.skip[0] != 0) return;  // uniform: before any barrier
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    constexpr int GS = 3 * H, RW = 32 / H;
+    constexpr int GS = G * H, RW = 32 / H;
     constexpr unsigned SB = reg_slot_bytes(H, SMAX, W16);
     float* rwin = reinterpret_cast<float*>(reg_mem);
     const unsigned wbase = smem_addr(reg_mem);
     const SweepRing ring(wbase + reg_pad((unsigned)a.win * 4u), smem_addr(bars), a.nr, a.nl, a.ncw, SB, RW * 4u);
-    if (threadIdx.x < 3) rwin[a.zero_off + threadIdx.x] = 0.0f;
+    if (threadIdx.x < G) rwin[a.zero_off + threadIdx.x] = 0.0f;
     if (threadIdx.x == 0) ring.init();
     __syncthreads();
     if (warp == a.ncw) {
@@ -1860,10 +1867,14 @@ __device__ __forceinline__ void tri_reg_body(const RegArgs& a, int tb)
 #pragma unroll
         for (int m = 1; m < H; m <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, m);
         const float d = S.b - sum;
-        const float d0 = __shfl_sync(0xffffffffu, d, lane0);
-        const float d1 = __shfl_sync(0xffffffffu, d, lane0 + H);
-        const float d2 = __shfl_sync(0xffffffffu, d, lane0 + 2 * H);
-        psol = fmaf(S.gm[2], d2, fmaf(S.gm[1], d1, S.gm[0] * d0));
+        if constexpr (G == 1) {
+            psol = S.gm[0] * d;
+        } else {
+            const float d0 = __shfl_sync(0xffffffffu, d, lane0);
+            const float d1 = __shfl_sync(0xffffffffu, d, lane0 + H);
+            const float d2 = __shfl_sync(0xffffffffu, d, lane0 + 2 * H);
+            psol = fmaf(S.gm[2], d2, fmaf(S.gm[1], d1, S.gm[0] * d0));
+        }
         const bool own = owner && S.wo >= 0;
         if (own) rwin[S.wo] = psol;
         pgo = own ? S.go : -1;
@@ -1878,10 +1889,10 @@ __device__ __forceinline__ void tri_reg_body(const RegArgs& a, int tb)
     if (pgo >= 0) out[pgo] = psol;
 }
 
-template <int H, int SMAX, bool UPPER, bool W16>
+template <int G, int H, int SMAX, bool UPPER, bool W16>
 __global__ void __launch_bounds__((kRegMaxWarps + 1) * 32, 1) k_tri_reg(RegArgs a)
 {
-    tri_reg_body<H, SMAX, UPPER, W16>(a, blockIdx.x);
+    tri_reg_body<G, H, SMAX, UPPER, W16>(a, blockIdx.x);
 }
 
 // One thread block per (entry, temporal block): entry blockIdx.x / q of the
@@ -1895,7 +1906,7 @@ __global__ void __launch_bounds__((kRegMaxWarps + 1) * 32, 1)
     RegArgs a = args[blockIdx.x / q];
     if (skip) a.skip = skip;
     if (out) a.out = out;
-    tri_reg_body<H, SMAX, UPPER, W16>(a, blockIdx.x % q);
+    tri_reg_body<3, H, SMAX, UPPER, W16>(a, blockIdx.x % q);
 }
 
 // Forward-sweep right-hand sides in row order, one array per temporal
@@ -2018,40 +2029,48 @@ int build_reg_parts(const DevIlu& F, int Q, int H, IluStage& st, cudaStream_t s)
     return XT_OK;
 }
 
+// The sweeps of a block-Jacobi factor's row blocks.
+template <int Q, int H, int SMAX, bool W16>
+int launch_reg_blocks(const IluStage& st, const double* dAinv, const float* v, float* z, cudaStream_t s,
+                      const int* skip)
+{
+    static std::atomic<bool> attr{false};
+    if (!attr.load(std::memory_order_acquire)) {
+        const int dyn = max_dyn_smem() - (int)kRegStatic;
+        XT_CUDA(cudaFuncSetAttribute(k_tri_reg_parts<H, SMAX, false, W16>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
+        XT_CUDA(cudaFuncSetAttribute(k_tri_reg_parts<H, SMAX, true, W16>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
+        attr.store(true, std::memory_order_release);
+    }
+    const int nb = (int)std::max(1LL, std::min<long long>((st.lanesL + 255) / 256, 152LL * 8));
+    k_rhs_slots<Q><<<nb, 256, 0, s>>>(st.srcL.p, st.lanesL, dAinv, v, st.rrhsL.p, skip);
+    const RegArgs* aL = reinterpret_cast<const RegArgs*>(st.argsL.p);
+    const RegArgs* aU = reinterpret_cast<const RegArgs*>(st.argsU.p);
+    const int threads = (st.ncw + 1) * 32;
+    k_tri_reg_parts<H, SMAX, false, W16><<<Q * st.parts, threads, st.smem, s>>>(aL, Q, skip, st.rrhsU.p);
+    k_tri_reg_parts<H, SMAX, true, W16><<<Q * st.parts, threads, st.smem, s>>>(aU, Q, skip, z);
+    note_launches(3);
+    XT_CUDA(cudaGetLastError());
+    return XT_OK;
+}
+
 // Measured (GB300, both sweeps and the pre-pass, q = 6), before with the slots
 // read from global memory straight into registers: 20 x 20 x 60 rod 605 -> 471
 // us, 10 x 10 x 30 rod 161 -> 153 us, 4 x 4 x 12 rod 72.6 -> 62.6 us.
-template <int Q, int H, int SMAX, bool W16>
+template <int Q, int G, int H, int SMAX, bool W16>
 int launch_reg(const IluStage& st, const double* dAinv, const float* v, float* z, cudaStream_t s,
                const int* skip)
 {
-    const int dyn = max_dyn_smem() - (int)kRegStatic;
-    if (st.parts > 1) {
-        static std::atomic<bool> pattr{false};
-        if (!pattr.load(std::memory_order_acquire)) {
-            XT_CUDA(cudaFuncSetAttribute(k_tri_reg_parts<H, SMAX, false, W16>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
-            XT_CUDA(cudaFuncSetAttribute(k_tri_reg_parts<H, SMAX, true, W16>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
-            pattr.store(true, std::memory_order_release);
-        }
-        const int nb = (int)std::max(1LL, std::min<long long>((st.lanesL + 255) / 256, 152LL * 8));
-        k_rhs_slots<Q><<<nb, 256, 0, s>>>(st.srcL.p, st.lanesL, dAinv, v, st.rrhsL.p, skip);
-        const RegArgs* aL = reinterpret_cast<const RegArgs*>(st.argsL.p);
-        const RegArgs* aU = reinterpret_cast<const RegArgs*>(st.argsU.p);
-        const int threads = (st.ncw + 1) * 32;
-        k_tri_reg_parts<H, SMAX, false, W16><<<Q * st.parts, threads, st.smem, s>>>(aL, Q, skip,
-                                                                                 st.rrhsU.p);
-        k_tri_reg_parts<H, SMAX, true, W16><<<Q * st.parts, threads, st.smem, s>>>(aU, Q, skip, z);
-        note_launches(3);
-        XT_CUDA(cudaGetLastError());
-        return XT_OK;
+    if constexpr (G == 3) {
+        if (st.parts > 1) return launch_reg_blocks<Q, H, SMAX, W16>(st, dAinv, v, z, s, skip);
     }
     static std::atomic<bool> attr{false};
     if (!attr.load(std::memory_order_acquire)) {
-        XT_CUDA(cudaFuncSetAttribute(k_tri_reg<H, SMAX, false, W16>,
+        const int dyn = max_dyn_smem() - (int)kRegStatic;
+        XT_CUDA(cudaFuncSetAttribute(k_tri_reg<G, H, SMAX, false, W16>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
-        XT_CUDA(cudaFuncSetAttribute(k_tri_reg<H, SMAX, true, W16>,
+        XT_CUDA(cudaFuncSetAttribute(k_tri_reg<G, H, SMAX, true, W16>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
         attr.store(true, std::memory_order_release);
     }
@@ -2063,8 +2082,8 @@ int launch_reg(const IluStage& st, const double* dAinv, const float* v, float* z
                      L.nr, L.zero_off, skip};
     const RegArgs aU{U.slots.p, st.rrhsU.p, z, U.lanes, 0, U.nl, U.ncw, U.win_elems, U.nr,
                      U.zero_off, skip};
-    k_tri_reg<H, SMAX, false, W16><<<Q, (L.ncw + 1) * 32, reg_smem(L), s>>>(aL);
-    k_tri_reg<H, SMAX, true, W16><<<Q, (U.ncw + 1) * 32, reg_smem(U), s>>>(aU);
+    k_tri_reg<G, H, SMAX, false, W16><<<Q, (L.ncw + 1) * 32, reg_smem(L), s>>>(aL);
+    k_tri_reg<G, H, SMAX, true, W16><<<Q, (U.ncw + 1) * 32, reg_smem(U), s>>>(aU);
     note_launches(3);
     XT_CUDA(cudaGetLastError());
     return XT_OK;
@@ -2079,8 +2098,8 @@ int launch_reg_width(const IluStage& st, const double* dAinv, const float* v, fl
         set_error("register sweep: triangles with different offset widths");
         return XT_ERR_STATE;
     }
-    if (st.regL->w16) return launch_reg<Q, H, SMAX, true>(st, dAinv, v, z, s, skip);
-    return launch_reg<Q, H, SMAX, false>(st, dAinv, v, z, s, skip);
+    if (st.regL->w16) return launch_reg<Q, 3, H, SMAX, true>(st, dAinv, v, z, s, skip);
+    return launch_reg<Q, 3, H, SMAX, false>(st, dAinv, v, z, s, skip);
 }
 
 template <int Q>
@@ -2088,6 +2107,15 @@ int launch_reg_any(const IluStage& st, const double* dAinv, const float* v, floa
                    cudaStream_t s, const int* skip)
 {
     const int H = st.regL->H, smax = st.regL->smax;
+    if (st.regL->g == 1) {
+        if (H == 2 && smax == 8) return launch_reg<Q, 1, 2, 8, true>(st, dAinv, v, z, s, skip);
+        if (H == 2 && smax == 10) return launch_reg<Q, 1, 2, 10, true>(st, dAinv, v, z, s, skip);
+        if (H == 2 && smax == 12) return launch_reg<Q, 1, 2, 12, true>(st, dAinv, v, z, s, skip);
+        if (H == 2 && smax == 16) return launch_reg<Q, 1, 2, 16, true>(st, dAinv, v, z, s, skip);
+        if (H == 1 && smax == 12) return launch_reg<Q, 1, 1, 12, true>(st, dAinv, v, z, s, skip);
+        if (H == 1 && smax == 20) return launch_reg<Q, 1, 1, 20, true>(st, dAinv, v, z, s, skip);
+        if (H == 4 && smax == 8) return launch_reg<Q, 1, 4, 8, true>(st, dAinv, v, z, s, skip);
+    }
     if (H == 2 && smax == 8) return launch_reg_width<Q, 2, 8>(st, dAinv, v, z, s, skip);
     if (H == 2 && smax == 10) return launch_reg_width<Q, 2, 10>(st, dAinv, v, z, s, skip);
     if (H == 2 && smax == 12) return launch_reg_width<Q, 2, 12>(st, dAinv, v, z, s, skip);
@@ -2278,15 +2306,20 @@ int launch_tri(const DevIlu& F, const double* dAinv, const T* v, T* z, T* work, 
     // thread block; 1: node blocks; 0: rows through the ring.  A format
     // that cannot be laid out for the factor falls back to the next.
     int fmt = env_int("XTFEM_ILU_FMT", 4);
-    // FP64, and FP32 with one unknown per node: row records (dev_ilu_rows.cu)
-    if (fmt == 4 && (sizeof(T) == 8 || F.L.g == 1) && !env_int("XTFEM_ILU_SIMPLE", 0)) {
-        RowSweep* rows = nullptr;
-        XT_TRY(get_rows<T>(F, Q, s, rows));
-        if (rows) return run_rows<T>(*rows, Q, dAinv, v, z, s, skip);
+    if constexpr (sizeof(T) == 8) {  // FP64: row records (dev_ilu_rows.cu)
+        if (fmt == 4 && !env_int("XTFEM_ILU_SIMPLE", 0)) {
+            RowSweep* rows = nullptr;
+            XT_TRY(get_rows(F, Q, s, rows));
+            if (rows) return run_rows(*rows, Q, dAinv, v, z, s);
+        }
     }
     if constexpr (sizeof(T) == 4) {
-        if (F.L.g == 3 && fmt == 4) {
-            const int H = F.shares > 0 ? F.shares : env_int("XTFEM_ILU_SHARES", 2);
+        if ((F.L.g == 3 || F.L.g == 1) && fmt == 4) {
+            // two lanes a row; one where a level of one-row groups is wider
+            // than the 16 rows of a warp at two (20 x 20 x 60 mesh, 35 rows a
+            // level: a thermal slab 28.9 against 30.4 ms)
+            const int two = F.L.g == 1 && F.L.ngroups > 16LL * F.L.nlevels ? 1 : 2;
+            const int H = F.shares > 0 ? F.shares : env_int("XTFEM_ILU_SHARES", two);
             XT_TRY(get_stage<T>(F, Q, 4, s, st, H));
             if (st) return launch_reg_any<Q>(*st, dAinv, v, z, s, skip);
             fmt = 3;

@@ -1,17 +1,15 @@
-// dev_ilu_rows.cu -- the triangular sweeps in row records read straight into
-// registers: FP64 factors, and FP32 factors of one unknown per node.
+// dev_ilu_rows.cu -- the triangular sweeps of FP64 factors in row records.
 //
 // As the FP32 node-row sweep of dev_ilu.cu: one thread block per temporal
 // block, each on an SM of its own and each the whole level chain, with the
 // solution window in shared memory.
 //
-// What bounds it.  FP64: this part takes an FP64 instruction of one warp in
-// 64 cycles whatever its live lanes and however independent, and one of any
-// warp of the SM every 19 (measured), so a level costs the instructions of
-// one warp times the larger of 64 and 19 times the warps.  The
-// sweep it replaced ran all temporal blocks in one thread block (12,400
-// multiply-adds a level on the 80,703-row rod, on one SM).  FP32, one unknown
-// per node: the level chain's latency (window reads, multiply-adds, barrier).
+// What bounds it.  This part takes an FP64 instruction of one warp in 64 cycles
+// whatever its live lanes and however independent, and one of any warp of the
+// SM every 19 (measured), so a level costs the instructions of one warp times
+// the larger of 64 and 19 times the warps.  The sweep it replaced ran all
+// temporal blocks in one thread block (12,400 multiply-adds a level on the
+// 80,703-row rod, on one SM).
 //
 // Layout.  Lane = (group of the warp's chunk, row r of the group, share h of
 // the row's entries); G rows a group, H shares a row, 32 / (G H) groups a
@@ -44,7 +42,7 @@
 // warps of 23 FP64 instructions at the SM's rate of 19 to 21 cycles each;
 // 10 x 10 x 30 rod: 3,227 -> 787 us; 4 x 4 x 12 rod: 1,337 -> 320 us, 1,500
 // cycles a level, 700 of them the 11 FP64 instructions of its one chunk.
-// A thermal slab of the 20 x 20 x 60 mesh (q = 3, FP32): 114 -> 34 ms.
+// (With the copying warp off the level barrier, as in ilu_ring.cuh: 2,557 us.)
 #include <algorithm>
 #include <atomic>
 #include <cstdint>
@@ -63,15 +61,15 @@ constexpr unsigned kNone = 0xffffu;
 // Steps a lane's registers hold: rows of up to H * steps entries.
 __host__ __device__ constexpr int row_steps(int H) { return H == 1 ? 20 : (H == 2 ? 12 : 8); }
 // Bytes of a lane's record: G values, two words, to 16 bytes.
-template <class T, int G>
+template <int G>
 __host__ __device__ constexpr int rec_bytes()
 {
-    return (G * (int)sizeof(T) + 8 + 15) / 16 * 16;
+    return (G * 8 + 8 + 15) / 16 * 16;
 }
-template <class T, int G, int H>
+template <int G, int H>
 __host__ __device__ constexpr int row_slot_bytes()
 {
-    return 32 * (rec_bytes<T, G>() + row_steps(H) * (2 + (int)sizeof(T)));
+    return 32 * (rec_bytes<G>() + row_steps(H) * (2 + 8));
 }
 
 }  // namespace
@@ -94,14 +92,12 @@ struct RowSweep {
 namespace {
 
 // The cycles of a triangle's levels with H shares a row and at most kRowWarps
-// warps.  FP64: 64 cycles an instruction of one warp, 19 an instruction of
-// any; about 350 a level for the rest (window reads, shuffles, barrier).
-// FP32: instructions are 5 cycles of the chain; about 300 a level.
-template <class T>
+// warps: 64 cycles an instruction of one warp, 19 an instruction of any; about
+// 350 a level for the rest (window reads, shuffles, barrier).
 long long rows_cost(const TriHost& h, const std::vector<int>& longest, int H, bool& fits)
 {
     const int g = h.g, per = 32 / (g * H);
-    const int one = sizeof(T) == 8 ? 64 : 5, any = sizeof(T) == 8 ? 19 : 2, fixed = sizeof(T) == 8 ? 350 : 300;
+    constexpr int one = 64, any = 19, fixed = 350;
     long long cost = 0;
     fits = true;
     for (int l = 0; l < h.nlevels && fits; ++l) {
@@ -194,14 +190,14 @@ struct RowFill {
 };
 
 // One warp per slot.
-template <class T, int G, int H>
+template <int G, int H>
 __global__ void k_fill_rows(RowFill f)
 {
-    constexpr int S = row_steps(H), RB = rec_bytes<T, G>(), GS = G * H;
+    constexpr int S = row_steps(H), RB = rec_bytes<G>(), GS = G * H;
     const int lane = threadIdx.x & 31;
     const int sl = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (sl >= f.nslots) return;
-    unsigned char* b = f.slots + (size_t)sl * row_slot_bytes<T, G, H>();
+    unsigned char* b = f.slots + (size_t)sl * row_slot_bytes<G, H>();
     const int gw = lane / GS, r = (lane % GS) / H, hh = lane % H;
     const bool on = gw < f.count[sl];
     int k0 = 0, n = 0, row = -1, i = 0;
@@ -213,9 +209,9 @@ __global__ void k_fill_rows(RowFill f)
     }
     int steps = (n + H - 1) / H;
     for (int off = 16; off > 0; off >>= 1) steps = max(steps, __shfl_xor_sync(0xffffffffu, steps, off));
-    T* m = reinterpret_cast<T*>(b + lane * RB);
-    for (int k = 0; k < G; ++k) m[k] = on ? (T)f.minv[((size_t)i * G + r) * G + k] : T(0);
-    unsigned* w = reinterpret_cast<unsigned*>(b + lane * RB + G * sizeof(T));
+    double* m = reinterpret_cast<double*>(b + lane * RB);
+    for (int k = 0; k < G; ++k) m[k] = on ? (double)f.minv[((size_t)i * G + r) * G + k] : 0.0;
+    unsigned* w = reinterpret_cast<unsigned*>(b + lane * RB + G * 8);
     const bool own = on && hh == 0;
     w[0] = (own ? (unsigned)(f.wslot[f.row0[i] / G] * G + r) : kNone) | ((unsigned)steps << 16) |
            (f.count[sl] > 0 ? 1u << 24 : 0u);
@@ -226,18 +222,15 @@ __global__ void k_fill_rows(RowFill f)
     for (int st = 0; st < S; ++st) {
         const int e = st * H + hh;
         unsigned short o = (unsigned short)f.zero;
-        T v = T(0);
+        double v = 0.0;
         if (e < n) {
             const int c = f.ext_col[k0 + e];
             o = (unsigned short)(f.wslot[c / G] * G + c % G);
-            v = (T)-f.ext_v[k0 + e];
+            v = (double)-f.ext_v[k0 + e];
         }
         off16[((st >> 2) * 32 + lane) * 4 + (st & 3)] = o;
-        // FP32: four values of a lane together; FP64: two and two, so that
-        // a warp's 16-byte loads are consecutive
-        const size_t at = sizeof(T) == 4 ? ((size_t)(st >> 2) * 32 + lane) * 4 + (st & 3)
-                                         : ((size_t)(st >> 1) * 32 + lane) * 2 + (st & 1);
-        reinterpret_cast<T*>(vals)[at] = v;
+        // two values of a lane together: a warp's 16-byte loads are consecutive
+        reinterpret_cast<double*>(vals)[((size_t)(st >> 1) * 32 + lane) * 2 + (st & 1)] = v;
     }
 }
 
@@ -259,13 +252,7 @@ __device__ __forceinline__ uint2 lds2(unsigned a)
     asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(r.x), "=r"(r.y) : "r"(a));
     return r;
 }
-__device__ __forceinline__ float lds1(unsigned a, float)
-{
-    float r;
-    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(r) : "r"(a));
-    return r;
-}
-__device__ __forceinline__ double lds1(unsigned a, double)
+__device__ __forceinline__ double lds1(unsigned a)
 {
     double r;
     asm volatile("ld.shared.f64 %0, [%1];" : "=d"(r) : "r"(a));
@@ -305,19 +292,19 @@ __device__ __forceinline__ void bulk_copy(unsigned dst, const void* src, unsigne
 
 // A slot in registers; loaded in steps between the multiply-adds of the
 // level before it.
-template <class T, int G, int H>
+template <int G, int H>
 struct RowRegs {
-    static constexpr int S = row_steps(H), RB = rec_bytes<T, G>(), VQ = 4 * (int)sizeof(T) / 16;
+    static constexpr int S = row_steps(H), RB = rec_bytes<G>(), VQ = 4 * 8 / 16;
     uint4 rec[RB / 16];
     uint2 off[S / 4];
     uint4 val[S / 4 * VQ];
-    T b;
+    double b;
 
     __device__ __forceinline__ void load_rec(unsigned p, unsigned rhs, int lane)
     {
 #pragma unroll
         for (int k = 0; k < RB / 16; ++k) rec[k] = lds4(p + lane * RB + 16 * k);
-        b = lds1(rhs, T(0));
+        b = lds1(rhs);
     }
     __device__ __forceinline__ void load_quad(unsigned p, int k, int lane)
     {
@@ -331,50 +318,40 @@ struct RowRegs {
         const uint4 r = rec[i >> 2];
         return (i & 3) == 0 ? r.x : ((i & 3) == 1 ? r.y : ((i & 3) == 2 ? r.z : r.w));
     }
-    __device__ __forceinline__ T m(int k) const
+    __device__ __forceinline__ double m(int k) const
     {
-        if constexpr (sizeof(T) == 4) return __uint_as_float(word(k));
-        else return __hiloint2double((int)word(2 * k + 1), (int)word(2 * k));
+        return __hiloint2double((int)word(2 * k + 1), (int)word(2 * k));
     }
-    __device__ __forceinline__ unsigned wo() const { return word(G * (int)sizeof(T) / 4); }
-    __device__ __forceinline__ int dst() const { return (int)word(G * (int)sizeof(T) / 4 + 1); }
+    __device__ __forceinline__ unsigned wo() const { return word(G * 8 / 4); }
+    __device__ __forceinline__ int dst() const { return (int)word(G * 8 / 4 + 1); }
     __device__ __forceinline__ unsigned o(int st) const
     {
         const unsigned w = (st & 2) ? off[st >> 2].y : off[st >> 2].x;
         return (st & 1) ? (w >> 16) : (w & 0xffffu);
     }
-    __device__ __forceinline__ T v(int st) const
+    __device__ __forceinline__ double v(int st) const
     {
-        if constexpr (sizeof(T) == 4) {
-            const uint4 r = val[st >> 2];
-            return __uint_as_float((st & 3) == 0 ? r.x : ((st & 3) == 1 ? r.y : ((st & 3) == 2 ? r.z : r.w)));
-        } else {
-            const uint4 r = val[st >> 1];
-            return (st & 1) ? __hiloint2double((int)r.w, (int)r.z) : __hiloint2double((int)r.y, (int)r.x);
-        }
+        const uint4 r = val[st >> 1];
+        return (st & 1) ? __hiloint2double((int)r.w, (int)r.z) : __hiloint2double((int)r.y, (int)r.x);
     }
 };
 
-template <class T>
 struct RowArgs {
     const unsigned char* slots;
-    const T* rhs;
-    T* out;
+    const double* rhs;
+    double* out;
     long long rstride, ostride;  // between temporal blocks
     int nl, ncw, zero, win;
-    const int* skip;
     int* err;
 };
 
-// Levels in flight: FP64 levels are long (1,200 cycles and more), an FP32
-// level is about 400 cycles; four and eight levels cover a read from DRAM.
-template <class T>
-__host__ __device__ constexpr int ring_levels() { return sizeof(T) == 8 ? 4 : 8; }
+// Levels in flight: a level takes 1,200 cycles and more, four cover a read
+// from DRAM.
+constexpr int kRingLevels = 4;
 // Ring bytes a warp takes of one level: its slot and its 32 right-hand sides.
-template <class T, int G, int H>
-__host__ __device__ constexpr int ring_bytes() { return row_slot_bytes<T, G, H>() + 32 * (int)sizeof(T); }
-template <class T>
-__host__ __device__ constexpr unsigned window_bytes(int win) { return ((unsigned)win * (unsigned)sizeof(T) + 127u) / 128u * 128u; }
+template <int G, int H>
+__host__ __device__ constexpr int ring_bytes() { return row_slot_bytes<G, H>() + 32 * 8; }
+__host__ __device__ constexpr unsigned window_bytes(int win) { return ((unsigned)win * 8u + 127u) / 128u * 128u; }
 
 constexpr int kRowSpin = 1 << 20;
 
@@ -382,28 +359,27 @@ constexpr int kRowSpin = 1 << 20;
 // waits for them, one level barrier ahead of the warps that read them: a wait
 // on an mbarrier takes 180 cycles even when its copy has long landed, and
 // starting a copy 200, which the level chain does not see this way.
-template <class T, int G, int H, bool UPPER>
-__global__ void __launch_bounds__((kRowWarps + 1) * 32, 1) k_tri_rows(RowArgs<T> a)
+template <int G, int H, bool UPPER>
+__global__ void __launch_bounds__((kRowWarps + 1) * 32, 1) k_tri_rows(RowArgs a)
 {
     extern __shared__ __align__(128) unsigned char row_smem[];
-    constexpr int S = row_steps(H), GS = G * H, SB = row_slot_bytes<T, G, H>();
-    constexpr int NR = ring_levels<T>();
+    constexpr int S = row_steps(H), GS = G * H, SB = row_slot_bytes<G, H>();
+    constexpr int NR = kRingLevels;
     __shared__ unsigned long long bars[NR];
-    if (a.skip && a.skip[0] != 0) return;  // uniform: before any barrier
-    T* win = reinterpret_cast<T*>(row_smem);
+    double* win = reinterpret_cast<double*>(row_smem);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tb = blockIdx.x;
     const unsigned wbase = smem_at(win);
-    const unsigned ring = wbase + window_bytes<T>(a.win);
-    const unsigned lev_slots = (unsigned)a.ncw * SB, lev_rhs = (unsigned)a.ncw * 32 * sizeof(T);
+    const unsigned ring = wbase + window_bytes(a.win);
+    const unsigned lev_slots = (unsigned)a.ncw * SB, lev_rhs = (unsigned)a.ncw * 32 * 8;
     const unsigned lev = lev_slots + lev_rhs;
-    if (threadIdx.x < G) win[a.zero + threadIdx.x] = T(0);
+    if (threadIdx.x < G) win[a.zero + threadIdx.x] = 0.0;
     if (threadIdx.x == 0) {
         for (int k = 0; k < NR; ++k) bar_init(smem_at(bars + k));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
     if (warp == a.ncw) {  // copies
-        const T* gb = a.rhs + (size_t)tb * a.rstride;
+        const double* gb = a.rhs + (size_t)tb * a.rstride;
         auto copy = [&](int l) {
             const unsigned to = ring + (unsigned)(l % NR) * lev, bar = smem_at(bars + l % NR);
             bar_expect(bar, lev);
@@ -440,10 +416,10 @@ __global__ void __launch_bounds__((kRowWarps + 1) * 32, 1) k_tri_rows(RowArgs<T>
         return;
     }
     const int lane0 = (lane / GS) * GS;
-    T* out = UPPER ? a.out + tb : a.out + (size_t)tb * a.ostride;
+    double* out = UPPER ? a.out + tb : a.out + (size_t)tb * a.ostride;
     const unsigned myslot = ring + (unsigned)warp * SB;
-    const unsigned myrhs = ring + lev_slots + (unsigned)(warp * 32 + lane) * (unsigned)sizeof(T);
-    RowRegs<T, G, H> R[2];
+    const unsigned myrhs = ring + lev_slots + (unsigned)(warp * 32 + lane) * 8u;
+    RowRegs<G, H> R[2];
     asm volatile("bar.sync 0;" ::: "memory");  // levels 0 and 1 are there
     R[0].load_rec(myslot, myrhs, lane);
 #pragma unroll
@@ -451,46 +427,43 @@ __global__ void __launch_bounds__((kRowWarps + 1) * 32, 1) k_tri_rows(RowArgs<T>
     unsigned at = NR > 1 ? lev : 0;  // the next level's place
     // one level: its sums with r, while the next level's entry goes into nx
     // (a place beyond the last level holds old data: read, not used)
-    auto level = [&](RowRegs<T, G, H>& r, RowRegs<T, G, H>& nx) {
+    auto level = [&](RowRegs<G, H>& r, RowRegs<G, H>& nx) {
         const unsigned wo = r.wo();
         const int steps = (wo >> 24) ? (int)(wo >> 16) & 0xff : -1;  // -1: no chunk; the same for the whole warp
-        T x[S];
+        double x[S];
 #pragma unroll
         for (int st = 0; st < (S < 8 ? S : 8); ++st)
-            if ((st & ~3) < steps) x[st] = lds1(wbase + r.o(st) * (unsigned)sizeof(T), T(0));
-        T acc = r.b, acc1 = T(0);
+            if ((st & ~3) < steps) x[st] = lds1(wbase + r.o(st) * 8u);
+        double acc = r.b;
 #pragma unroll
         for (int k = 0; k < S / 4; ++k) {
             if (4 * k < steps) {
                 acc = fma(r.v(4 * k), x[4 * k], acc);
-                if constexpr (sizeof(T) == 4) acc1 = fma(r.v(4 * k + 1), x[4 * k + 1], acc1);
-                else acc = fma(r.v(4 * k + 1), x[4 * k + 1], acc);
+                acc = fma(r.v(4 * k + 1), x[4 * k + 1], acc);
             }
             if (k + 2 < S / 4 && 4 * k + 8 < steps)
 #pragma unroll
                 for (int u = 0; u < 4; ++u)
                     if (4 * k + 8 + u < S)
-                        x[4 * k + 8 + u] = lds1(wbase + r.o(4 * k + 8 + u) * (unsigned)sizeof(T), T(0));
+                        x[4 * k + 8 + u] = lds1(wbase + r.o(4 * k + 8 + u) * 8u);
             nx.load_quad(myslot + at, k, lane);
             if (4 * k + 2 < steps) {
                 acc = fma(r.v(4 * k + 2), x[4 * k + 2], acc);
-                if constexpr (sizeof(T) == 4) acc1 = fma(r.v(4 * k + 3), x[4 * k + 3], acc1);
-                else acc = fma(r.v(4 * k + 3), x[4 * k + 3], acc);
+                acc = fma(r.v(4 * k + 3), x[4 * k + 3], acc);
             }
         }
         nx.load_rec(myslot + at, myrhs + at, lane);
         if (steps >= 0) {
-            T d = acc;
-            if constexpr (sizeof(T) == 4) d += acc1;
+            double d = acc;
 #pragma unroll
             for (int m = 1; m < H; m <<= 1) d += __shfl_xor_sync(0xffffffffu, d, m);
-            T sol;
+            double sol;
             if constexpr (G == 1) {
                 sol = r.m(0) * d;
             } else {
-                const T d0 = __shfl_sync(0xffffffffu, d, lane0);
-                const T d1 = __shfl_sync(0xffffffffu, d, lane0 + H);
-                const T d2 = __shfl_sync(0xffffffffu, d, lane0 + 2 * H);
+                const double d0 = __shfl_sync(0xffffffffu, d, lane0);
+                const double d1 = __shfl_sync(0xffffffffu, d, lane0 + H);
+                const double d2 = __shfl_sync(0xffffffffu, d, lane0 + 2 * H);
                 sol = fma(r.m(2), d2, fma(r.m(1), d1, r.m(0) * d0));
             }
             if ((wo & 0xffffu) != kNone) {
@@ -509,25 +482,24 @@ __global__ void __launch_bounds__((kRowWarps + 1) * 32, 1) k_tri_rows(RowArgs<T>
 
 // Forward right-hand sides in lane order: rhs[q][lane] = sum_j Ainv(q, j)
 // v(row(lane), j).  Lanes without a row keep the zero they were built with.
-template <class T, int Q>
+template <int Q>
 __global__ void k_rows_rhs(const int* __restrict__ src, long long lanes,
-                           const double* __restrict__ dAinv, const T* __restrict__ v,
-                           T* __restrict__ rhs, const int* __restrict__ skip)
+                           const double* __restrict__ dAinv, const double* __restrict__ v,
+                           double* __restrict__ rhs)
 {
-    __shared__ T sA[Q * Q];
-    if (skip && skip[0] != 0) return;
-    for (int i = threadIdx.x; i < Q * Q; i += blockDim.x) sA[i] = (T)dAinv[i];
+    __shared__ double sA[Q * Q];
+    for (int i = threadIdx.x; i < Q * Q; i += blockDim.x) sA[i] = (double)dAinv[i];
     __syncthreads();
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < lanes;
          t += (long long)gridDim.x * blockDim.x) {
         const int row = src[t];
         if (row < 0) continue;
-        T vr[Q];
+        double vr[Q];
 #pragma unroll
         for (int j = 0; j < Q; ++j) vr[j] = v[(size_t)row * Q + j];
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
-            T b = T(0);
+            double b = 0.0;
 #pragma unroll
             for (int j = 0; j < Q; ++j) b = fma(sA[j * Q + q], vr[j], b);
             rhs[(size_t)q * lanes + t] = b;
@@ -535,7 +507,7 @@ __global__ void k_rows_rhs(const int* __restrict__ src, long long lanes,
     }
 }
 
-template <class T, int G, int H>
+template <int G, int H>
 int fill_tri(const DevTri& d, const TriHost& h, const std::vector<int>& ord, RowTri& t, int q,
              const int* dst, int* src, cudaStream_t s)
 {
@@ -547,33 +519,33 @@ int fill_tri(const DevTri& d, const TriHost& h, const std::vector<int>& ord, Row
     XT_TRY(dord.upload(ord.data(), ord.size(), s));
     XT_TRY(wslot.upload(h.slot.data(), h.slot.size(), s));
     XT_TRY(minv.upload(h.minv.data(), h.minv.size(), s));
-    XT_TRY(t.slots.alloc(nslot * (size_t)row_slot_bytes<T, G, H>()));
+    XT_TRY(t.slots.alloc(nslot * (size_t)row_slot_bytes<G, H>()));
     RowFill f{first.p, count.p, dord.p, d.group_row0.p, d.ext_ptr.p, d.ext_col.p, d.ext_v64.p,
               minv.p, wslot.p, dst, src, t.slots.p, (int)nslot, t.zero, q};
-    k_fill_rows<T, G, H><<<(unsigned)((nslot + 7) / 8), 256, 0, s>>>(f);
+    k_fill_rows<G, H><<<(unsigned)((nslot + 7) / 8), 256, 0, s>>>(f);
     note_launches(1);
     XT_CUDA(cudaGetLastError());
     XT_CUDA(cudaStreamSynchronize(s));  // the staging buffers go out of scope
     return XT_OK;
 }
 
-template <class T, int G>
+template <int G>
 int fill_any(const DevTri& d, const TriHost& h, const std::vector<int>& ord, RowTri& t, int q,
              const int* dst, int* src, cudaStream_t s)
 {
-    if (t.H == 1) return fill_tri<T, G, 1>(d, h, ord, t, q, dst, src, s);
-    if (t.H == 2) return fill_tri<T, G, 2>(d, h, ord, t, q, dst, src, s);
-    return fill_tri<T, G, 4>(d, h, ord, t, q, dst, src, s);
+    if (t.H == 1) return fill_tri<G, 1>(d, h, ord, t, q, dst, src, s);
+    if (t.H == 2) return fill_tri<G, 2>(d, h, ord, t, q, dst, src, s);
+    return fill_tri<G, 4>(d, h, ord, t, q, dst, src, s);
 }
 
-template <class T, int G>
+template <int G>
 size_t row_smem_bytes(const RowTri& t)
 {
-    const size_t e = t.H == 1 ? ring_bytes<T, G, 1>() : (t.H == 2 ? ring_bytes<T, G, 2>() : ring_bytes<T, G, 4>());
-    return window_bytes<T>(t.win) + (size_t)t.ncw * ring_levels<T>() * e;
+    const size_t e = t.H == 1 ? ring_bytes<G, 1>() : (t.H == 2 ? ring_bytes<G, 2>() : ring_bytes<G, 4>());
+    return window_bytes(t.win) + (size_t)t.ncw * kRingLevels * e;
 }
 
-template <class T, int G>
+template <int G>
 int build(const DevIlu& F, int q, RowSweep& R, bool& ok, cudaStream_t s)
 {
     ok = false;
@@ -589,7 +561,7 @@ int build(const DevIlu& F, int q, RowSweep& R, bool& ok, cudaStream_t s)
         long long bc = 0;
         for (int H : {1, 2, 4}) {
             bool f = false;
-            const long long c = rows_cost<T>(*h[k], longest[k], H, f);
+            const long long c = rows_cost(*h[k], longest[k], H, f);
             if (f && (force == 0 || force == H) && (best == 0 || c < bc)) {
                 best = H;
                 bc = c;
@@ -598,7 +570,7 @@ int build(const DevIlu& F, int q, RowSweep& R, bool& ok, cudaStream_t s)
         if (!best) return XT_OK;
         // fewer warps where window and ring would not fit in shared memory
         fit[k] = rows_plan(*h[k], ord[k], best, warps, *t[k]);
-        while (fit[k] && row_smem_bytes<T, G>(*t[k]) + 4096 > (size_t)max_dyn_smem()) {
+        while (fit[k] && row_smem_bytes<G>(*t[k]) + 4096 > (size_t)max_dyn_smem()) {
             if (t[k]->ncw == 1) fit[k] = false;
             else fit[k] = rows_plan(*h[k], ord[k], best, t[k]->ncw - 1, *t[k]);
         }
@@ -609,9 +581,9 @@ int build(const DevIlu& F, int q, RowSweep& R, bool& ok, cudaStream_t s)
     DBuf<int> dst;
     XT_TRY(dst.upload(R.U.row_slot.data(), R.U.row_slot.size(), s));
     XT_TRY(R.src.alloc((size_t)R.L.lanes));
-    XT_TRY((fill_any<T, G>(F.L, *h[0], ord[0], R.L, q, dst.p, R.src.p, s)));
-    XT_TRY((fill_any<T, G>(F.U, *h[1], ord[1], R.U, q, nullptr, nullptr, s)));
-    const size_t bl = (size_t)q * R.L.lanes * sizeof(T), bu = (size_t)q * R.U.lanes * sizeof(T);
+    XT_TRY((fill_any<G>(F.L, *h[0], ord[0], R.L, q, dst.p, R.src.p, s)));
+    XT_TRY((fill_any<G>(F.U, *h[1], ord[1], R.U, q, nullptr, nullptr, s)));
+    const size_t bl = (size_t)q * R.L.lanes * 8, bu = (size_t)q * R.U.lanes * 8;
     XT_TRY(R.rhsL.alloc(bl));
     XT_TRY(R.rhsU.alloc(bu));
     // lanes that own no row start their sums at zero
@@ -619,8 +591,8 @@ int build(const DevIlu& F, int q, RowSweep& R, bool& ok, cudaStream_t s)
     XT_CUDA(cudaMemsetAsync(R.rhsU.p, 0, bu, s));
     XT_CUDA(cudaStreamSynchronize(s));
     if (trace_on())
-        std::fprintf(stderr, "[xtfem] row sweep: %zu-byte values, shares %d/%d, warps %d/%d, levels %d/%d\n",
-                     sizeof(T), R.L.H, R.U.H, R.L.ncw, R.U.ncw, R.L.nl, R.U.nl);
+        std::fprintf(stderr, "[xtfem] row sweep: shares %d/%d, warps %d/%d, levels %d/%d\n",
+                     R.L.H, R.U.H, R.L.ncw, R.U.ncw, R.L.nl, R.U.nl);
     for (RowTri* x : t) {
         x->first = std::vector<int>();
         x->count = std::vector<int>();
@@ -630,99 +602,85 @@ int build(const DevIlu& F, int q, RowSweep& R, bool& ok, cudaStream_t s)
     return XT_OK;
 }
 
-template <class T, int G, int H, bool UPPER>
-int launch_tri_rows(const RowTri& t, const RowArgs<T>& a, int q, cudaStream_t s)
+template <int G, int H, bool UPPER>
+int launch_tri_rows(const RowTri& t, const RowArgs& a, int q, cudaStream_t s)
 {
     static std::atomic<bool> attr{false};
     if (!attr.load(std::memory_order_acquire)) {  // idempotent: concurrent first calls are harmless
-        XT_CUDA(cudaFuncSetAttribute(k_tri_rows<T, G, H, UPPER>,
+        XT_CUDA(cudaFuncSetAttribute(k_tri_rows<G, H, UPPER>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem() - 4096));
         attr.store(true, std::memory_order_release);
     }
-    k_tri_rows<T, G, H, UPPER><<<q, (t.ncw + 1) * 32, row_smem_bytes<T, G>(t), s>>>(a);
+    k_tri_rows<G, H, UPPER><<<q, (t.ncw + 1) * 32, row_smem_bytes<G>(t), s>>>(a);
     note_launches(1);
     XT_CUDA(cudaGetLastError());
     return XT_OK;
 }
 
-template <class T, int G, bool UPPER>
-int launch_shares(const RowTri& t, const RowArgs<T>& a, int q, cudaStream_t s)
+template <int G, bool UPPER>
+int launch_shares(const RowTri& t, const RowArgs& a, int q, cudaStream_t s)
 {
-    if (t.H == 1) return launch_tri_rows<T, G, 1, UPPER>(t, a, q, s);
-    if (t.H == 2) return launch_tri_rows<T, G, 2, UPPER>(t, a, q, s);
-    return launch_tri_rows<T, G, 4, UPPER>(t, a, q, s);
+    if (t.H == 1) return launch_tri_rows<G, 1, UPPER>(t, a, q, s);
+    if (t.H == 2) return launch_tri_rows<G, 2, UPPER>(t, a, q, s);
+    return launch_tri_rows<G, 4, UPPER>(t, a, q, s);
 }
 
-template <class T, int G>
-int launch_both(const RowSweep& R, int q, T* z, cudaStream_t s, const int* skip)
+template <int G>
+int launch_both(const RowSweep& R, int q, double* z, cudaStream_t s)
 {
     int* err = nullptr;
     XT_TRY(ilu_error_word(&err));
-    T *rl = reinterpret_cast<T*>(R.rhsL.p), *ru = reinterpret_cast<T*>(R.rhsU.p);
-    XT_TRY((launch_shares<T, G, false>(
-        R.L, RowArgs<T>{R.L.slots.p, rl, ru, R.L.lanes, R.U.lanes, R.L.nl, R.L.ncw, R.L.zero, R.L.win, skip, err}, q, s)));
-    return launch_shares<T, G, true>(
-        R.U, RowArgs<T>{R.U.slots.p, ru, z, R.U.lanes, 0, R.U.nl, R.U.ncw, R.U.zero, R.U.win, skip, err}, q, s);
+    double *rl = reinterpret_cast<double*>(R.rhsL.p), *ru = reinterpret_cast<double*>(R.rhsU.p);
+    XT_TRY((launch_shares<G, false>(
+        R.L, RowArgs{R.L.slots.p, rl, ru, R.L.lanes, R.U.lanes, R.L.nl, R.L.ncw, R.L.zero, R.L.win, err}, q, s)));
+    return launch_shares<G, true>(
+        R.U, RowArgs{R.U.slots.p, ru, z, R.U.lanes, 0, R.U.nl, R.U.ncw, R.U.zero, R.U.win, err}, q, s);
 }
 
-template <class T, int Q>
-void launch_rhs(const RowSweep& R, const double* dAinv, const T* v, cudaStream_t s, const int* skip)
+template <int Q>
+void launch_rhs(const RowSweep& R, const double* dAinv, const double* v, cudaStream_t s)
 {
     const int nb = (int)std::max(1LL, std::min<long long>((R.L.lanes + 255) / 256, 152LL * 8));
-    k_rows_rhs<T, Q><<<nb, 256, 0, s>>>(R.src.p, R.L.lanes, dAinv, v, reinterpret_cast<T*>(R.rhsL.p), skip);
+    k_rows_rhs<Q><<<nb, 256, 0, s>>>(R.src.p, R.L.lanes, dAinv, v, reinterpret_cast<double*>(R.rhsL.p));
     note_launches(1);
 }
 
 }  // namespace
 
-template <class T>
 int get_rows(const DevIlu& F, int q, cudaStream_t s, RowSweep*& out)
 {
     out = nullptr;
     if (!F.sched || q < 1 || q > 8) return XT_OK;
     const int g = F.L.g;
-    if (sizeof(T) == 8 ? (g != 1 && g != 3) : g != 1) return XT_OK;
-    const int key = ((q * 2 + (sizeof(T) == 4 ? 1 : 0)) * 8 +
-                     std::max(0, std::min(7, env_int("XTFEM_ILU_ROW_H", 0)))) * 32 +
+    if (g != 1 && g != 3) return XT_OK;
+    const int key = (q * 8 + std::max(0, std::min(7, env_int("XTFEM_ILU_ROW_H", 0)))) * 32 +
                     std::max(0, std::min(31, env_int("XTFEM_ILU_WARPS", 0)));
     auto it = F.rows.find(key);
     if (it == F.rows.end()) {
         auto R = std::make_shared<RowSweep>();
         R->g = g;
         bool ok = false;
-        if constexpr (sizeof(T) == 8) {
-            if (g == 3) XT_TRY((build<T, 3>(F, q, *R, ok, s)));
-        }
-        if (g == 1) XT_TRY((build<T, 1>(F, q, *R, ok, s)));
+        if (g == 3) XT_TRY((build<3>(F, q, *R, ok, s)));
+        else XT_TRY((build<1>(F, q, *R, ok, s)));
         it = F.rows.emplace(key, ok ? R : nullptr).first;
     }
     out = it->second.get();
     return XT_OK;
 }
 
-template <class T>
-int run_rows(const RowSweep& R, int q, const double* dAinv, const T* v, T* z, cudaStream_t s,
-             const int* skip)
+int run_rows(const RowSweep& R, int q, const double* dAinv, const double* v, double* z, cudaStream_t s)
 {
     switch (q) {
-    case 1: launch_rhs<T, 1>(R, dAinv, v, s, skip); break;
-    case 2: launch_rhs<T, 2>(R, dAinv, v, s, skip); break;
-    case 3: launch_rhs<T, 3>(R, dAinv, v, s, skip); break;
-    case 4: launch_rhs<T, 4>(R, dAinv, v, s, skip); break;
-    case 5: launch_rhs<T, 5>(R, dAinv, v, s, skip); break;
-    case 6: launch_rhs<T, 6>(R, dAinv, v, s, skip); break;
-    case 7: launch_rhs<T, 7>(R, dAinv, v, s, skip); break;
-    default: launch_rhs<T, 8>(R, dAinv, v, s, skip); break;
+    case 1: launch_rhs<1>(R, dAinv, v, s); break;
+    case 2: launch_rhs<2>(R, dAinv, v, s); break;
+    case 3: launch_rhs<3>(R, dAinv, v, s); break;
+    case 4: launch_rhs<4>(R, dAinv, v, s); break;
+    case 5: launch_rhs<5>(R, dAinv, v, s); break;
+    case 6: launch_rhs<6>(R, dAinv, v, s); break;
+    case 7: launch_rhs<7>(R, dAinv, v, s); break;
+    default: launch_rhs<8>(R, dAinv, v, s); break;
     }
-    if constexpr (sizeof(T) == 8) {
-        if (R.g == 3) return launch_both<T, 3>(R, q, z, s, skip);
-    }
-    return launch_both<T, 1>(R, q, z, s, skip);
+    return R.g == 3 ? launch_both<3>(R, q, z, s) : launch_both<1>(R, q, z, s);
 }
-
-template int get_rows<double>(const DevIlu&, int, cudaStream_t, RowSweep*&);
-template int get_rows<float>(const DevIlu&, int, cudaStream_t, RowSweep*&);
-template int run_rows<double>(const RowSweep&, int, const double*, const double*, double*, cudaStream_t, const int*);
-template int run_rows<float>(const RowSweep&, int, const double*, const float*, float*, cudaStream_t, const int*);
 
 }  // namespace xt

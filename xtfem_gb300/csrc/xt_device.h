@@ -208,7 +208,7 @@ struct DevIlu {
     std::shared_ptr<IluSched> sched;
     // built on first use for a (q, precision) pair; key 2*q + (FP32 ? 1 : 0)
     mutable std::map<int, std::shared_ptr<IluStage>> stages;
-    // row-record sweeps, built on first use for a (q, precision); null: unfit
+    // FP64 row-record sweeps, built on first use for a q; null: unfit
     mutable std::map<int, std::shared_ptr<RowSweep>> rows;
     // lanes per row of the FP32 register sweep (its rows per warp: 10 node
     // rows at 1, 5 at 2, 2 at 4); 0 = XTFEM_ILU_SHARES or 2.  Set by the
@@ -240,14 +240,11 @@ template <class T>
 int ilu_apply(const DevIlu& F, int q, const double* dAinv, const T* v, T* z, T* work,
               cudaStream_t s, const int* skip = nullptr);
 
-// The row-record sweep of F for FP64 (groups of 1 or 3 rows) or FP32 (one-row
-// groups), built on first use; out is null when its rows or window do not
-// fit.  run_rows: ilu_apply through it.
-template <class T>
+// The FP64 row-record sweep of F (groups of 1 or 3 rows), built on first use;
+// out is null when its rows or window do not fit.  run_rows: ilu_apply<double>
+// through it.
 int get_rows(const DevIlu& F, int q, cudaStream_t s, RowSweep*& out);
-template <class T>
-int run_rows(const RowSweep& R, int q, const double* dAinv, const T* v, T* z, cudaStream_t s,
-             const int* skip);
+int run_rows(const RowSweep& R, int q, const double* dAinv, const double* v, double* z, cudaStream_t s);
 
 // Reads and clears the device-side error word of the staged sweeps (a
 // bounded wait that gave up); XT_OK when clear.
