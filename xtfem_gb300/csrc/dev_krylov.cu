@@ -37,12 +37,49 @@ __device__ __forceinline__ double block_sum(double v, double* sh)
     return r;  // valid in thread 0
 }
 
+// Sums of kChunk values over the lanes of a warp in nine additions: at each of
+// the first three exchanges a lane keeps half of its values and gives the
+// others away, then the lane's one value is summed over four lanes.  (A
+// butterfly per value takes five additions each, every one 64 cycles of its SM
+// quarter.)  Every lane returns the sum of value lane_value(lane).
+__device__ __forceinline__ int lane_value(int lane)
+{
+    return ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
+}
+__device__ __forceinline__ double warp_sums(double (&v)[kChunk], int lane)
+{
+    static_assert(kChunk == 8, "three exchanges");
+#pragma unroll
+    for (int half = 4; half > 0; half >>= 1) {
+        const int off = half * 4;
+        const bool up = (lane & off) != 0;
+#pragma unroll
+        for (int c = 0; c < half; ++c)
+            v[c] = (up ? v[c + half] : v[c]) + __shfl_xor_sync(0xffffffffu, up ? v[c] : v[c + half], off);
+    }
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+    return v[0];
+}
+
+// Row blocks of an FP64 dot pass: 1024 rows a block or more (four a thread),
+// at most kRowBlocks.  With kRowBlocks blocks for a 67,518-entry vector (228
+// rows each) and a block sum per basis vector the pass over 45 vectors took 52
+// us, nearly all of it the sums (FP64 GMRES on that 10 x 10 x 30 rod 81.5 ms
+// with 228, 75.7 ms with 1,024).
+inline int dot_rows(size_t n, int nblocks)
+{
+    const size_t b = (n + 1023) / 1024;
+    return (int)(b < 1 ? 1 : (b < (size_t)nblocks ? b : (size_t)nblocks));
+}
+
 // partial[j * nb + b] = sum over block b's rows of V_j[r] * w[r]
 template <class TV>
-__global__ void k_multi_dot(const TV* __restrict__ V, size_t ld, int k, const TV* __restrict__ w,
-                            size_t n, double* __restrict__ partial)
+__global__ void __launch_bounds__(kThreads)
+k_multi_dot(const TV* __restrict__ V, size_t ld, int k, const TV* __restrict__ w,
+            size_t n, double* __restrict__ partial)
 {
-    __shared__ double sh[32];
+    __shared__ double sh[kChunk][kThreads / 32];
     const int j0 = blockIdx.y * kChunk;
     const int nb = gridDim.x;
     const size_t per = (n + nb - 1) / nb;
@@ -52,13 +89,23 @@ __global__ void k_multi_dot(const TV* __restrict__ V, size_t ld, int k, const TV
     for (int c = 0; c < kChunk; ++c) acc[c] = 0.0;
     for (size_t r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
         const double wr = (double)w[r];
+        double v[kChunk];
+#pragma unroll
+        for (int c = 0; c < kChunk; ++c) v[c] = j0 + c < k ? (double)V[(size_t)(j0 + c) * ld + r] : 0.0;
 #pragma unroll
         for (int c = 0; c < kChunk; ++c)
-            if (j0 + c < k) acc[c] = fma((double)V[(size_t)(j0 + c) * ld + r], wr, acc[c]);
+            if (j0 + c < k) acc[c] = fma(v[c], wr, acc[c]);
     }
-    for (int c = 0; c < kChunk && j0 + c < k; ++c) {
-        const double s = block_sum(acc[c], sh);
-        if (threadIdx.x == 0) partial[(size_t)(j0 + c) * nb + blockIdx.x] = s;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const double s = warp_sums(acc, lane);
+    if ((lane & 3) == 0) sh[lane_value(lane)][warp] = s;
+    __syncthreads();
+    if (threadIdx.x < 4 * kChunk) {  // four lanes a value, two warps' sums each
+        const int c = threadIdx.x >> 2, q = threadIdx.x & 3;
+        double t = sh[c][2 * q] + sh[c][2 * q + 1];
+        t += __shfl_xor_sync(0xffffffffu, t, 2);
+        t += __shfl_xor_sync(0xffffffffu, t, 1);
+        if (q == 0 && j0 + c < k) partial[(size_t)(j0 + c) * nb + blockIdx.x] = t;
     }
 }
 
@@ -648,9 +695,14 @@ __global__ void k_update(const TV* __restrict__ V, size_t ld, int k, const doubl
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t r = (size_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += stride) {
         double acc = (double)w[r];
-        for (int j = 0; j < k; ++j) {
-            const double hj = j < 512 ? hs[j] : h[j];
-            acc = fma(-hj, (double)V[(size_t)j * ld + r], acc);
+        for (int jb = 0; jb < k; jb += 8) {
+            double v[8];  // eight independent loads in flight per thread
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (jb + u < k) v[u] = (double)V[(size_t)(jb + u) * ld + r];
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (jb + u < k) acc = fma(-(jb + u < 512 ? hs[jb + u] : h[jb + u]), v[u], acc);
         }
         const TV out = (TV)acc;
         w[r] = out;
@@ -672,7 +724,15 @@ __global__ void k_lincomb(const TV* __restrict__ V, size_t ld, int k, const doub
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t r = (size_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += stride) {
         double acc = 0.0;
-        for (int j = 0; j < k; ++j) acc = fma(j < 512 ? cs[j] : c[j], (double)V[(size_t)j * ld + r], acc);
+        for (int jb = 0; jb < k; jb += 8) {
+            double v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (jb + u < k) v[u] = (double)V[(size_t)(jb + u) * ld + r];
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (jb + u < k) acc = fma(jb + u < 512 ? cs[jb + u] : c[jb + u], v[u], acc);
+        }
         y[r] = (TY)acc;
     }
 }
@@ -805,15 +865,17 @@ int multi_dot(const TV* V, size_t ld, int k, const TV* w, size_t n, Reduce& r, c
 {
     if (k > r.kmax) { set_error("multi_dot: k exceeds reduction capacity"); return XT_ERR_ARG; }
     if (k <= 0) return XT_OK;
-    dim3 grid(r.nblocks, (k + kChunk - 1) / kChunk);
     if (pairs_ok<TV>(V, ld, w, n)) {
+        const dim3 grid(r.nblocks, (k + kChunk - 1) / kChunk);
         k_multi_dot_f32<<<grid, kThreads, 0, s>>>(reinterpret_cast<const float2*>(V), ld / 2, k,
                                                   reinterpret_cast<const float2*>(w), n / 2,
                                                   r.partial.p);
         k_finish_df<<<k, kThreads, 0, s>>>(r.partial.p, r.nblocks, r.out.p);
     } else {
-        k_multi_dot<TV><<<grid, kThreads, 0, s>>>(V, ld, k, w, n, r.partial.p);
-        k_finish<<<k, kThreads, 0, s>>>(r.partial.p, r.nblocks, r.out.p, 0);
+        const int nb = dot_rows(n, r.nblocks);
+        k_multi_dot<TV><<<dim3(nb, (k + kChunk - 1) / kChunk), kThreads, 0, s>>>(V, ld, k, w, n,
+                                                                                r.partial.p);
+        k_finish<<<k, kThreads, 0, s>>>(r.partial.p, nb, r.out.p, 0);
     }
     note_launches(2);
     XT_CUDA(cudaGetLastError());
