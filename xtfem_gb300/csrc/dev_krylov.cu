@@ -162,12 +162,14 @@ __global__ void k_multi_dot_f32(const float2* __restrict__ V, size_t ld2, int k,
 // every operation runs on the FP32 pipe.
 
 // Row blocks per chunk of kChunk basis vectors in a double-float dot pass:
-// one wave of the six blocks per SM that the pass's registers allow, over
-// all chunks (row blocks shrink as k grows, so each block's rows outweigh
-// its block reduction).  Eight per SM made 1.34 waves (ncu).  The wave is
-// sized for 148 of the 152 SMs: a few SMs may hold a long-running block of
-// the damage update on the side stream, and a pass sized for every SM
-// would leave its last blocks a second wave.
+// six blocks per SM, two rounds of the three that the pass's registers
+// allow, over all chunks (row blocks shrink as k grows, so each block's rows
+// outweigh its block reduction).  Eight per SM left the last round nearly empty
+// (ncu).  Sized for 148 of the 152 SMs: a few SMs may hold a
+// long-running block of the damage update on the side stream, and a pass
+// sized for every SM would leave its last blocks a round of their own.
+// The count fixes the rounding of the sums: a batch, a system alone and both
+// drivers use the same.
 __host__ __device__ __forceinline__ int df_dot_blocks(int k, int nblocks)
 {
     const int nchunk = (k + kChunk - 1) / kChunk;
@@ -255,7 +257,12 @@ __device__ __forceinline__ void multi_dot_df_body(const float4* __restrict__ V, 
     }
 }
 
-__global__ void __launch_bounds__(256, 6) k_multi_dot_df(const float4* __restrict__ V, size_t ld2, int k,
+// Three blocks an SM: with the six that 40 registers allow, the eight loads of
+// a chunk were made one after the other.  A one-pass step of the 20 x 20 x 60
+// rod (up to 60 vectors) 125 us before, 113 us now, of the 25 x 9 x 7 rod 56.7
+// and 48.6 us, a 64-rod batch 183 and 175 ms; two blocks measure the same,
+// four 116 us.
+__global__ void __launch_bounds__(256, 3) k_multi_dot_df(const float4* __restrict__ V, size_t ld2, int k,
                                const float4* __restrict__ w, size_t n2,
                                double* __restrict__ partial)
 {
@@ -266,7 +273,7 @@ __global__ void __launch_bounds__(256, 6) k_multi_dot_df(const float4* __restric
 // device-driven GMRES; nothing to do once ctl[1] is set): block b takes row
 // block b mod nb of chunk b / nb, nb as the host launch would choose it,
 // so the partial sums are those of k_multi_dot_df bit for bit.
-__global__ void __launch_bounds__(256, 6) k_multi_dot_df_ctl(const float4* __restrict__ V, size_t ld2,
+__global__ void __launch_bounds__(256, 3) k_multi_dot_df_ctl(const float4* __restrict__ V, size_t ld2,
                                const float4* __restrict__ w, size_t n2,
                                double* __restrict__ partial, int nblocks,
                                const int* __restrict__ ctl)
@@ -1226,7 +1233,7 @@ __global__ void kb_flex_zcopy(const FlexStepItem* __restrict__ t)
 // (row block, chunk) items dealt to its e.dotblocks blocks in turn (a
 // system's share of one wave, by its size), so small and large systems
 // finish together and no block of the grid is there for the largest alone.
-__global__ void __launch_bounds__(256, 6) kb_dot(const FlexStepItem* __restrict__ t)
+__global__ void __launch_bounds__(256, 3) kb_dot(const FlexStepItem* __restrict__ t)
 {
     const FlexStepItem& e = t[blockIdx.y];
     const int* ctl = e.ctl;
