@@ -292,6 +292,38 @@ k_kron_df(int p, const int* __restrict__ kptr, const int* __restrict__ kcol,
 // 32 / (3 Q/2) node rows per warp.
 // This thread block is block bx of a gx-block pass (a batched launch runs
 // one such pass per system).
+//
+// What bounds it is how many bytes of K a warp has in flight: with the blocks
+// read where they are used, one block a lane ahead at best, 66 % of the issue
+// slots waited for them (1.15 TB/s).  A warp therefore copies its node rows'
+// blocks, masses and columns -- one contiguous range -- to shared memory at
+// once (cp.async, its own part, no block barrier) and keeps kNbAhead X
+// slices in flight.  For q of 2 and 4 a warp's 10 or 5 rows would take too
+// much shared memory to keep the warps that hide X's latency: those read
+// directly, as before.
+// Now FP32 and shared-memory issue are each busy half the time: the packed
+// operations take two cycles of the FP32 pipe, 21 us of it on the 20 x 20 x 60
+// rod.  Measured (q 6): 20 x 20 x 60 rod 55 us before, 45 us now; 25 x 9 x 7
+// rod 18.7 and 13.3 us; a 64-rod batch 175 and 168 ms.  One or three slices
+// ahead, 64 or 256 threads a block: 47 us.
+constexpr int kNbAhead = 2;
+
+template <int Q>
+constexpr int nb_threads()
+{
+    return Q >= 6 ? 128 : 256;
+}
+
+template <class V>
+__device__ __forceinline__ void copy_async(V* dst, const V* src)
+{
+    static_assert(sizeof(V) == 4 || sizeof(V) == 8, "cp.async of 4 or 8 bytes");
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(
+                     (unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(src), "n"(sizeof(V))
+                 : "memory");
+}
+
 template <int Q>
 __device__ __forceinline__ void kron_nb_body(int nodes, const int* __restrict__ bptr,
                                              const int* __restrict__ bcol,
@@ -304,6 +336,7 @@ __device__ __forceinline__ void kron_nb_body(int nodes, const int* __restrict__ 
 {
     static_assert(Q % 2 == 0 && Q <= 8, "pairs of temporal blocks");
     constexpr int NP = Q / 2, LPR = 3 * NP, RPW = 32 / LPR;
+    [[maybe_unused]] constexpr int WARPS = nb_threads<Q>() / 32;
     __shared__ float2 sA[Q * Q], sB[Q * Q];
     for (int i = threadIdx.x; i < Q * Q; i += blockDim.x) {
         const float ah = __double2float_rn(dA[i]), bh = __double2float_rn(dB[i]);
@@ -323,18 +356,68 @@ __device__ __forceinline__ void kron_nb_body(int nodes, const int* __restrict__ 
         // .y entry 2qp+1
         float2 kh = make_float2(0.f, 0.f), kl = kh, mh = kh, ml = kh;
         const int b0 = act ? bptr[a] : 0, b1 = act ? bptr[a + 1] : 0;
+        if constexpr (Q >= 6) {
+            constexpr int CAP = 27 * RPW, D = kNbAhead, N = D + 1;
+            __shared__ float2 stK[WARPS][CAP * 9], stM[WARPS][CAP];
+            __shared__ int stC[WARPS][CAP];
+            float2* const sK = stK[threadIdx.x >> 5];
+            float2* const sM = stM[threadIdx.x >> 5];
+            int* const sC = stC[threadIdx.x >> 5];
+            const int r1 = bptr[min(a0 + RPW, nodes)];
+            // CAP blocks at a time: all of the warp's rows on a hexahedral mesh
+            for (int base = bptr[a0]; base < r1; base += CAP) {
+                const int cnt = min(CAP, r1 - base);
+                for (int i = lane; i < 9 * cnt; i += 32) copy_async(sK + i, kv + (size_t)base * 9 + i);
+                for (int i = lane; i < cnt; i += 32) {
+                    copy_async(sM + i, mv + base + i);
+                    copy_async(sC + i, bcol + base + i);
+                }
+                asm volatile("cp.async.wait_all;" ::: "memory");
+                __syncwarp();
+                const int e1 = min(b1 - base, cnt);
+                int e = max(b0 - base, 0);
+                const float* xq = x + 2 * qp;
+                float2 xs[N][3];
+                auto fetch = [&](int at, int u) {
+                    const float* xb = xq + (size_t)sC[at] * (3 * Q);
+                    xs[u][0] = *reinterpret_cast<const float2*>(xb);
+                    xs[u][1] = *reinterpret_cast<const float2*>(xb + Q);
+                    xs[u][2] = *reinterpret_cast<const float2*>(xb + 2 * Q);
+                };
+#pragma unroll
+                for (int u = 0; u < D; ++u)
+                    if (e + u < e1) fetch(e + u, u);
+                for (; e < e1; e += N) {
+#pragma unroll
+                    for (int u = 0; u < N; ++u) {
+                        if (e + u + D < e1) fetch(e + u + D, (u + D) % N);
+                        if (e + u < e1) {
+                            const float2* kr = sK + (e + u) * 9 + c * 3;
+                            const float2 k0 = kr[0], k1 = kr[1], k2 = kr[2], m = sM[e + u];
+                            const float2 x0 = xs[u][0], x1 = xs[u][1], x2 = xs[u][2];
+                            df2_axpy(kh, kl, k0.x, k0.y, x0);
+                            df2_axpy(kh, kl, k1.x, k1.y, x1);
+                            df2_axpy(kh, kl, k2.x, k2.y, x2);
+                            df2_axpy(mh, ml, m.x, m.y, c == 0 ? x0 : (c == 1 ? x1 : x2));
+                        }
+                    }
+                }
+                __syncwarp();  // read before the next copy
+            }
+        } else {
 #pragma unroll 4
-        for (int b = b0; b < b1; ++b) {
-            const float* xb = x + (size_t)bcol[b] * (3 * Q) + 2 * qp;
-            const float2* kr = kv + (size_t)b * 9 + c * 3;
-            const float2 k0 = kr[0], k1 = kr[1], k2 = kr[2], m = mv[b];
-            const float2 x0 = *reinterpret_cast<const float2*>(xb);
-            const float2 x1 = *reinterpret_cast<const float2*>(xb + Q);
-            const float2 x2 = *reinterpret_cast<const float2*>(xb + 2 * Q);
-            df2_axpy(kh, kl, k0.x, k0.y, x0);
-            df2_axpy(kh, kl, k1.x, k1.y, x1);
-            df2_axpy(kh, kl, k2.x, k2.y, x2);
-            df2_axpy(mh, ml, m.x, m.y, c == 0 ? x0 : (c == 1 ? x1 : x2));
+            for (int b = b0; b < b1; ++b) {
+                const float* xb = x + (size_t)bcol[b] * (3 * Q) + 2 * qp;
+                const float2* kr = kv + (size_t)b * 9 + c * 3;
+                const float2 k0 = kr[0], k1 = kr[1], k2 = kr[2], m = mv[b];
+                const float2 x0 = *reinterpret_cast<const float2*>(xb);
+                const float2 x1 = *reinterpret_cast<const float2*>(xb + Q);
+                const float2 x2 = *reinterpret_cast<const float2*>(xb + 2 * Q);
+                df2_axpy(kh, kl, k0.x, k0.y, x0);
+                df2_axpy(kh, kl, k1.x, k1.y, x1);
+                df2_axpy(kh, kl, k2.x, k2.y, x2);
+                df2_axpy(mh, ml, m.x, m.y, c == 0 ? x0 : (c == 1 ? x1 : x2));
+            }
         }
         const float kh0 = kh.x, kl0 = kl.x, kh1 = kh.y, kl1 = kl.y;
         const float mh0 = mh.x, ml0 = ml.x, mh1 = mh.y, ml1 = ml.y;
@@ -373,7 +456,7 @@ __device__ __forceinline__ void kron_nb_body(int nodes, const int* __restrict__ 
 }
 
 template <int Q>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(nb_threads<Q>(), Q >= 6 ? 8 : 1)
 k_kron_nb(int nodes, const int* __restrict__ bptr, const int* __restrict__ bcol,
           const float2* __restrict__ kv, const float2* __restrict__ mv,
           const double* __restrict__ dA, const double* __restrict__ dB,
@@ -386,7 +469,7 @@ k_kron_nb(int nodes, const int* __restrict__ bptr, const int* __restrict__ bcol,
 // The node-block operator of table entry blockIdx.y: wfix = op(zfix), nothing
 // once the entry's cycle has ended.
 template <int Q>
-__global__ void __launch_bounds__(256) kb_kron_nb(const FlexStepItem* __restrict__ t)
+__global__ void __launch_bounds__(nb_threads<Q>(), Q >= 6 ? 8 : 1) kb_kron_nb(const FlexStepItem* __restrict__ t)
 {
     const FlexStepItem& e = t[blockIdx.y];
     if (e.ctl[1] != 0) return;
@@ -480,7 +563,7 @@ int launch_nb(const DevNodeBlocks& nb, const double* dA, const double* dB, const
               float2* y, cudaStream_t s, const int* skip)
 {
     constexpr int RPW = 32 / (3 * (Q / 2));
-    const int threads = 256, rows_per_block = (threads / 32) * RPW;
+    const int threads = nb_threads<Q>(), rows_per_block = (threads / 32) * RPW;
     const int blocks = std::max(1, (nb.nodes + rows_per_block - 1) / rows_per_block);
     k_kron_nb<Q><<<blocks, threads, 0, s>>>(nb.nodes, nb.ptr.p, nb.col.p, nb.kdf.p, nb.mdf.p, dA,
                                             dB, x, y, skip);
@@ -795,14 +878,15 @@ int kron_nb_batch(const FlexStepItem* t, int count, int q, const FlexStepDims& d
     // a quarter of the largest system's node rows per block pass: each warp
     // loops over about four row groups (any split gives the same rows)
     const int RPW = q == 2 ? 10 : (q == 4 ? 5 : (q == 6 ? 3 : 2));
-    const int rows_per_block = 8 * RPW;
+    const int threads = q >= 6 ? nb_threads<6>() : nb_threads<2>();
+    const int rows_per_block = threads / 32 * RPW;
     const int gx = std::max(1, (d.nodes_max + 4 * rows_per_block - 1) / (4 * rows_per_block));
     const dim3 grid(gx, count);
     switch (q) {
-    case 2: kb_kron_nb<2><<<grid, 256, 0, s>>>(t); break;
-    case 4: kb_kron_nb<4><<<grid, 256, 0, s>>>(t); break;
-    case 6: kb_kron_nb<6><<<grid, 256, 0, s>>>(t); break;
-    case 8: kb_kron_nb<8><<<grid, 256, 0, s>>>(t); break;
+    case 2: kb_kron_nb<2><<<grid, threads, 0, s>>>(t); break;
+    case 4: kb_kron_nb<4><<<grid, threads, 0, s>>>(t); break;
+    case 6: kb_kron_nb<6><<<grid, threads, 0, s>>>(t); break;
+    case 8: kb_kron_nb<8><<<grid, threads, 0, s>>>(t); break;
     default: set_error("kron_nb_batch: q must be 2, 4, 6 or 8"); return XT_ERR_ARG;
     }
     note_launches(1);
