@@ -722,7 +722,7 @@ int fused_build(FusedStep& f, const std::vector<int>& idx,
     f.lanes_max = 0;
     double ntot = 0.0;
     for (const FlexStepItem& e : all) ntot += (double)e.n;
-    // the dot pass's wave dealt to the systems by size, each at most the
+    // the dot pass's blocks dealt to the systems by size, each at most the
     // items its longest pass has
     for (FlexStepItem& e : all) {
         const int most = df_dot_blocks_max(im, e.dotrows);

@@ -1231,7 +1231,7 @@ __global__ void kb_flex_zcopy(const FlexStepItem* __restrict__ t)
 
 // The partial sums of k_multi_dot_df_ctl for entry blockIdx.y: the entry's
 // (row block, chunk) items dealt to its e.dotblocks blocks in turn (a
-// system's share of one wave, by its size), so small and large systems
+// system's share of them all, by its size), so small and large systems
 // finish together and no block of the grid is there for the largest alone.
 __global__ void __launch_bounds__(256, 3) kb_dot(const FlexStepItem* __restrict__ t)
 {
@@ -1309,7 +1309,10 @@ __global__ void kb_ctl_gather(const FlexStepItem* __restrict__ t, int count, int
 int df_row_blocks_for(long long nl, const Reduce& r) { return df_row_blocks(nl / 2, r.nblocks); }
 int df_dot_rows_for(long long nl, const Reduce& r) { return df_dot_rows(nl / 2, r.nblocks); }
 int df_dot_blocks_max(int im, int dotrows) { return df_dot_grid(im, dotrows); }
-int df_dot_wave() { return 6 * 148; }
+// Twelve blocks an SM in all: four rounds while every system runs, and still
+// all SMs when only a few large ones are left.  64 rods: 171 ms with 3 an SM,
+// 169 with 6, 167 with 12, 166 with 18.
+int df_dot_wave() { return 12 * 148; }
 
 int flexb_zcopy(const FlexStepItem* t, int count, const FlexStepDims& d, cudaStream_t s)
 {

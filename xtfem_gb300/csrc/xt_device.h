@@ -377,8 +377,7 @@ struct FlexStepDims {
 int df_row_blocks_for(long long nl, const Reduce& r);
 int df_dot_rows_for(long long nl, const Reduce& r);
 int df_dot_blocks_max(int im, int dotrows);
-// The thread blocks of one wave of a dot pass (a batch deals them to its
-// systems by size).
+// The thread blocks of a batch's dot pass, dealt to its systems by size.
 int df_dot_wave();
 // The ILU pre-pass of every entry from the hi part of its basis column j;
 // the ILU output into Z column j.
