@@ -295,23 +295,27 @@ k_kron_df(int p, const int* __restrict__ kptr, const int* __restrict__ kcol,
 //
 // What bounds it is how many bytes of K a warp has in flight: with the blocks
 // read where they are used, one block a lane ahead at best, 66 % of the issue
-// slots waited for them (1.15 TB/s).  A warp therefore copies its node rows'
+// slots wait for them (1.15 TB/s).  STAGED: a warp copies its node rows'
 // blocks, masses and columns -- one contiguous range -- to shared memory at
 // once (cp.async, its own part, no block barrier) and keeps kNbAhead X
-// slices in flight.  For q of 2 and 4 a warp's 10 or 5 rows would take too
-// much shared memory to keep the warps that hide X's latency: those read
-// directly, as before.
-// Now FP32 and shared-memory issue are each busy half the time: the packed
-// operations take two cycles of the FP32 pipe, 21 us of it on the 20 x 20 x 60
-// rod.  Measured (q 6): 20 x 20 x 60 rod 55 us before, 45 us now; 25 x 9 x 7
-// rod 18.7 and 13.3 us; a 64-rod batch 175 and 168 ms.  One or three slices
-// ahead, 64 or 256 threads a block: 47 us.
+// slices in flight; then FP32 (packed operations take two cycles) and
+// shared-memory reads are each busy half the time.
+// Measured (q 6), direct and staged: 25 x 9 x 7 rod 18.7 and 13.3 us, a step of
+// 64 rods in 175 and 168 ms a batch.  A system of more than one round of
+// thread blocks (kNbStagedNodes) reads directly all the same: a queue of
+// blocks that hold shared memory keeps another system's triangular sweep,
+// which wants most of an SM's, from starting (20 x 20 x 60 rod alone 54 and
+// 45 us, but eight of them at once 22.3-24.0 and 20.6 slabs/s).  One or three
+// slices ahead, 64 or 256 threads a block are slower.  q 2 and 4, whose 10 or
+// 5 rows a warp would take too much shared memory, and 8 read directly.
 constexpr int kNbAhead = 2;
 
-template <int Q>
+constexpr int kNbStagedNodes = 152 * 8 * 12;  // eight blocks an SM of four warps, three node rows each
+
+template <bool STAGED>
 constexpr int nb_threads()
 {
-    return Q >= 6 ? 128 : 256;
+    return STAGED ? 128 : 256;
 }
 
 template <class V>
@@ -324,7 +328,7 @@ __device__ __forceinline__ void copy_async(V* dst, const V* src)
                  : "memory");
 }
 
-template <int Q>
+template <int Q, bool STAGED>
 __device__ __forceinline__ void kron_nb_body(int nodes, const int* __restrict__ bptr,
                                              const int* __restrict__ bcol,
                                              const float2* __restrict__ kv,
@@ -336,7 +340,7 @@ __device__ __forceinline__ void kron_nb_body(int nodes, const int* __restrict__ 
 {
     static_assert(Q % 2 == 0 && Q <= 8, "pairs of temporal blocks");
     constexpr int NP = Q / 2, LPR = 3 * NP, RPW = 32 / LPR;
-    [[maybe_unused]] constexpr int WARPS = nb_threads<Q>() / 32;
+    [[maybe_unused]] constexpr int WARPS = nb_threads<STAGED>() / 32;
     __shared__ float2 sA[Q * Q], sB[Q * Q];
     for (int i = threadIdx.x; i < Q * Q; i += blockDim.x) {
         const float ah = __double2float_rn(dA[i]), bh = __double2float_rn(dB[i]);
@@ -356,7 +360,7 @@ __device__ __forceinline__ void kron_nb_body(int nodes, const int* __restrict__ 
         // .y entry 2qp+1
         float2 kh = make_float2(0.f, 0.f), kl = kh, mh = kh, ml = kh;
         const int b0 = act ? bptr[a] : 0, b1 = act ? bptr[a + 1] : 0;
-        if constexpr (Q >= 6) {
+        if constexpr (STAGED) {
             constexpr int CAP = 27 * RPW, D = kNbAhead, N = D + 1;
             __shared__ float2 stK[WARPS][CAP * 9], stM[WARPS][CAP];
             __shared__ int stC[WARPS][CAP];
@@ -455,25 +459,25 @@ __device__ __forceinline__ void kron_nb_body(int nodes, const int* __restrict__ 
     }
 }
 
-template <int Q>
-__global__ void __launch_bounds__(nb_threads<Q>(), Q >= 6 ? 8 : 1)
+template <int Q, bool STAGED>
+__global__ void __launch_bounds__(nb_threads<STAGED>(), STAGED ? 8 : 1)
 k_kron_nb(int nodes, const int* __restrict__ bptr, const int* __restrict__ bcol,
           const float2* __restrict__ kv, const float2* __restrict__ mv,
           const double* __restrict__ dA, const double* __restrict__ dB,
           const float* __restrict__ x, float2* __restrict__ y, const int* __restrict__ skip)
 {
     if (skip && skip[0] != 0) return;
-    kron_nb_body<Q>(nodes, bptr, bcol, kv, mv, dA, dB, x, y, blockIdx.x, gridDim.x);
+    kron_nb_body<Q, STAGED>(nodes, bptr, bcol, kv, mv, dA, dB, x, y, blockIdx.x, gridDim.x);
 }
 
 // The node-block operator of table entry blockIdx.y: wfix = op(zfix), nothing
 // once the entry's cycle has ended.
-template <int Q>
-__global__ void __launch_bounds__(nb_threads<Q>(), Q >= 6 ? 8 : 1) kb_kron_nb(const FlexStepItem* __restrict__ t)
+template <int Q, bool STAGED>
+__global__ void __launch_bounds__(nb_threads<STAGED>(), STAGED ? 8 : 1) kb_kron_nb(const FlexStepItem* __restrict__ t)
 {
     const FlexStepItem& e = t[blockIdx.y];
     if (e.ctl[1] != 0) return;
-    kron_nb_body<Q>(e.nodes, e.bptr, e.bcol, e.kv, e.mv, e.A, e.B, e.zfix, e.wfix, blockIdx.x,
+    kron_nb_body<Q, STAGED>(e.nodes, e.bptr, e.bcol, e.kv, e.mv, e.A, e.B, e.zfix, e.wfix, blockIdx.x,
                     gridDim.x);
 }
 
@@ -563,10 +567,18 @@ int launch_nb(const DevNodeBlocks& nb, const double* dA, const double* dB, const
               float2* y, cudaStream_t s, const int* skip)
 {
     constexpr int RPW = 32 / (3 * (Q / 2));
-    const int threads = nb_threads<Q>(), rows_per_block = (threads / 32) * RPW;
-    const int blocks = std::max(1, (nb.nodes + rows_per_block - 1) / rows_per_block);
-    k_kron_nb<Q><<<blocks, threads, 0, s>>>(nb.nodes, nb.ptr.p, nb.col.p, nb.kdf.p, nb.mdf.p, dA,
-                                            dB, x, y, skip);
+    auto launch = [&](auto kernel, int threads) {
+        const int rows_per_block = (threads / 32) * RPW;
+        const int blocks = std::max(1, (nb.nodes + rows_per_block - 1) / rows_per_block);
+        kernel<<<blocks, threads, 0, s>>>(nb.nodes, nb.ptr.p, nb.col.p, nb.kdf.p, nb.mdf.p, dA,
+                                          dB, x, y, skip);
+    };
+    if constexpr (Q == 6) {
+        if (nb.nodes <= kNbStagedNodes) launch(k_kron_nb<Q, true>, nb_threads<true>());
+        else launch(k_kron_nb<Q, false>, nb_threads<false>());
+    } else {
+        launch(k_kron_nb<Q, false>, nb_threads<false>());
+    }
     note_launches(1);
     XT_CUDA(cudaGetLastError());
     return XT_OK;
@@ -878,15 +890,19 @@ int kron_nb_batch(const FlexStepItem* t, int count, int q, const FlexStepDims& d
     // a quarter of the largest system's node rows per block pass: each warp
     // loops over about four row groups (any split gives the same rows)
     const int RPW = q == 2 ? 10 : (q == 4 ? 5 : (q == 6 ? 3 : 2));
-    const int threads = q >= 6 ? nb_threads<6>() : nb_threads<2>();
+    const bool staged = q == 6 && d.nodes_max <= kNbStagedNodes;
+    const int threads = staged ? nb_threads<true>() : nb_threads<false>();
     const int rows_per_block = threads / 32 * RPW;
     const int gx = std::max(1, (d.nodes_max + 4 * rows_per_block - 1) / (4 * rows_per_block));
     const dim3 grid(gx, count);
     switch (q) {
-    case 2: kb_kron_nb<2><<<grid, threads, 0, s>>>(t); break;
-    case 4: kb_kron_nb<4><<<grid, threads, 0, s>>>(t); break;
-    case 6: kb_kron_nb<6><<<grid, threads, 0, s>>>(t); break;
-    case 8: kb_kron_nb<8><<<grid, threads, 0, s>>>(t); break;
+    case 2: kb_kron_nb<2, false><<<grid, threads, 0, s>>>(t); break;
+    case 4: kb_kron_nb<4, false><<<grid, threads, 0, s>>>(t); break;
+    case 6:
+        if (staged) kb_kron_nb<6, true><<<grid, threads, 0, s>>>(t);
+        else kb_kron_nb<6, false><<<grid, threads, 0, s>>>(t);
+        break;
+    case 8: kb_kron_nb<8, false><<<grid, threads, 0, s>>>(t); break;
     default: set_error("kron_nb_batch: q must be 2, 4, 6 or 8"); return XT_ERR_ARG;
     }
     note_launches(1);
