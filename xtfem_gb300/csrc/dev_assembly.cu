@@ -141,9 +141,9 @@ k_element_k(int ne, const int* __restrict__ conn, const double* __restrict__ xyz
         for (int b = 0; b < 3; ++b) o[a * 3 + b] = s1[a][b] + s2[b][a] + (a == b ? tr : 0.0);
 }
 
-// K's entries from the element matrices, in every form the operators read:
-// FP64 and FP32 CSR values and, where K has them, its node blocks (FP64 and
-// double-float) at at[k].
+// K's entries from the element matrices: FP64 and FP32 CSR values and, where K
+// has them, its node blocks (FP64 and double-float) at at[k].  The CSR copies
+// in double-float and BF16 are dropped by the caller.
 __global__ void k_gather_k(int nnz, const int* __restrict__ cptr, const int* __restrict__ cidx,
                            const double* __restrict__ ke, const unsigned char* __restrict__ bcdiag,
                            double* __restrict__ kv, float* __restrict__ kv32,
@@ -423,7 +423,8 @@ int system_assemble_k_device(System& S, const double* ym, const double* nu, bool
                                      nb ? K.nb.from_csr.p : nullptr, K.nb.k64.p, K.nb.kdf.p);
     note_launches(2);
     XT_CUDA(cudaGetLastError());
-    K.vdf.release();  // remade from the new values on first use
+    K.vdf.release();  // these two are remade from the new values on first use
+    K.v16.release();
     return XT_OK;
 }
 

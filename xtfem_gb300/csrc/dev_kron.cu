@@ -708,7 +708,8 @@ int upload_csr(DevCsr& d, int n, const int* ia, const int* ja, const double* a,
     d.n = n;
     d.nnz = nnz;
     d.same_pattern = false;
-    d.vdf.release();  // remade from the new values on first use
+    d.vdf.release();  // these two are remade from the new values on first use
+    d.v16.release();
     d.nb.ok = false;  // rebuilt by csr_build_node_blocks
     XT_TRY(d.rowptr.upload(ia, (size_t)n + 1, s));
     XT_TRY(d.col.upload(ja, (size_t)(nnz > 0 ? nnz : 0), s));
