@@ -1559,7 +1559,7 @@ size_t reg_smem(const RegTri& t)
 }
 int reg_ring(const RegTri& t, int smax, bool w16, long long room)
 {
-    return ring_levels(reg_level_bytes(t, smax, w16), room - (long long)reg_pad((unsigned)t.win_elems * 4u));
+    return ring_levels(reg_level_bytes(t, smax, w16), t.ncw, room - (long long)reg_pad((unsigned)t.win_elems * 4u));
 }
 constexpr long long kRegStatic = 2048;  // static shared memory of a sweep, at most
 

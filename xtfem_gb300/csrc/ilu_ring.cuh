@@ -167,15 +167,20 @@ struct RingReader {
     }
 };
 
-// Levels of a part: starting a part's copies and waiting for it takes the
-// copying warp about 600 cycles, so two levels (of 300 cycles and more), four
-// where a level is one small warp's (the ring then stays under 40 KB, and a
-// batch's blocks share their SMs); one where two do not fit in `room` bytes,
-// 0 where one does not.
-inline int ring_levels(long long level_bytes, long long room)
+// Levels of a part, for levels of `warps` warps: handing a part over (its wait,
+// two barriers, the next copies) takes the copying warp 700 cycles or more, a
+// level about 350 with one or two warps, 400 with three and 500 and more with
+// wider ones: four, three and two levels.  Fewer where they do not fit in `room`
+// bytes, 0 where one does not.  With three warps a fourth level would leave a
+// batch one block an SM.  Measured, two levels (four up to 3 KB a level) before,
+// both sweeps of one apply with its copies: plate of 32 x 64 x 2 elements 419
+// and 374 us, panel of 96 x 24 x 1 450 and 398, 6 x 6 x 200 rod 792 and 691, 10
+// x 10 x 30 rod 246 and 232; with three levels the 16 x 16 x 48 rod, six warps,
+// takes 613 in place of 598.
+inline int ring_levels(long long level_bytes, int warps, long long room)
 {
     const long long n = room / (level_bytes * kRingParts);
-    const long long want = level_bytes <= 3072 ? 4 : 2;
+    const long long want = warps <= 2 ? 4 : (warps == 3 ? 3 : 2);
     return (int)(n < want ? (n < 0 ? 0 : n) : want);
 }
 
