@@ -1819,7 +1819,7 @@ __device__ __forceinline__ void reg_load(RegSet<SMAX, W16>& S, unsigned p, unsig
 
 // One temporal block tb of one sweep (one thread block of ncw + 1 warps).
 template <int G, int H, int SMAX, bool UPPER, bool W16>
-__device__ __forceinline__ void tri_reg_body(const RegArgs& a, int tb)
+__device__ __forceinline__ void tri_reg_body(const RegArgs& a, int tb, int polls)
 {
     extern __shared__ __align__(128) unsigned char reg_mem[];
     __shared__ unsigned long long bars[kRingParts];
@@ -1834,7 +1834,8 @@ __device__ __forceinline__ void tri_reg_body(const RegArgs& a, int tb)
     if (threadIdx.x == 0) ring.init();
     __syncthreads();
     if (warp == a.ncw) {
-        if (!ring.copies(a.slots, reinterpret_cast<const unsigned char*>(a.rhs + (size_t)tb * a.rstride), lane))
+        if (!ring.copies(a.slots, reinterpret_cast<const unsigned char*>(a.rhs + (size_t)tb * a.rstride), lane,
+                         polls))
             g_ilu_error = 1;
         return;
     }
@@ -1890,9 +1891,9 @@ __device__ __forceinline__ void tri_reg_body(const RegArgs& a, int tb)
 }
 
 template <int G, int H, int SMAX, bool UPPER, bool W16>
-__global__ void __launch_bounds__((kRegMaxWarps + 1) * 32, 1) k_tri_reg(RegArgs a)
+__global__ void __launch_bounds__((kRegMaxWarps + 1) * 32, 1) k_tri_reg(RegArgs a, int polls)
 {
-    tri_reg_body<G, H, SMAX, UPPER, W16>(a, blockIdx.x);
+    tri_reg_body<G, H, SMAX, UPPER, W16>(a, blockIdx.x, polls);
 }
 
 // One thread block per (entry, temporal block): entry blockIdx.x / q of the
@@ -1901,12 +1902,12 @@ __global__ void __launch_bounds__((kRegMaxWarps + 1) * 32, 1) k_tri_reg(RegArgs 
 // the sweeps of a batch of systems (each entry's own).
 template <int H, int SMAX, bool UPPER, bool W16>
 __global__ void __launch_bounds__((kRegMaxWarps + 1) * 32, 1)
-    k_tri_reg_parts(const RegArgs* __restrict__ args, int q, const int* skip, float* out)
+    k_tri_reg_parts(const RegArgs* __restrict__ args, int q, const int* skip, float* out, int polls)
 {
     RegArgs a = args[blockIdx.x / q];
     if (skip) a.skip = skip;
     if (out) a.out = out;
-    tri_reg_body<3, H, SMAX, UPPER, W16>(a, blockIdx.x % q);
+    tri_reg_body<3, H, SMAX, UPPER, W16>(a, blockIdx.x % q, polls);
 }
 
 // Forward-sweep right-hand sides in row order, one array per temporal
@@ -2048,8 +2049,9 @@ int launch_reg_blocks(const IluStage& st, const double* dAinv, const float* v, f
     const RegArgs* aL = reinterpret_cast<const RegArgs*>(st.argsL.p);
     const RegArgs* aU = reinterpret_cast<const RegArgs*>(st.argsU.p);
     const int threads = (st.ncw + 1) * 32;
-    k_tri_reg_parts<H, SMAX, false, W16><<<Q * st.parts, threads, st.smem, s>>>(aL, Q, skip, st.rrhsU.p);
-    k_tri_reg_parts<H, SMAX, true, W16><<<Q * st.parts, threads, st.smem, s>>>(aU, Q, skip, z);
+    k_tri_reg_parts<H, SMAX, false, W16><<<Q * st.parts, threads, st.smem, s>>>(aL, Q, skip, st.rrhsU.p,
+                                                                                    ring_polls());
+    k_tri_reg_parts<H, SMAX, true, W16><<<Q * st.parts, threads, st.smem, s>>>(aU, Q, skip, z, ring_polls());
     note_launches(3);
     XT_CUDA(cudaGetLastError());
     return XT_OK;
@@ -2082,8 +2084,8 @@ int launch_reg(const IluStage& st, const double* dAinv, const float* v, float* z
                      L.nr, L.zero_off, skip};
     const RegArgs aU{U.slots.p, st.rrhsU.p, z, U.lanes, 0, U.nl, U.ncw, U.win_elems, U.nr,
                      U.zero_off, skip};
-    k_tri_reg<G, H, SMAX, false, W16><<<Q, (L.ncw + 1) * 32, reg_smem(L), s>>>(aL);
-    k_tri_reg<G, H, SMAX, true, W16><<<Q, (U.ncw + 1) * 32, reg_smem(U), s>>>(aU);
+    k_tri_reg<G, H, SMAX, false, W16><<<Q, (L.ncw + 1) * 32, reg_smem(L), s>>>(aL, ring_polls());
+    k_tri_reg<G, H, SMAX, true, W16><<<Q, (U.ncw + 1) * 32, reg_smem(U), s>>>(aU, ring_polls());
     note_launches(3);
     XT_CUDA(cudaGetLastError());
     return XT_OK;
@@ -2477,7 +2479,7 @@ int reg_group_hs(const RegGroup& g, int q, cudaStream_t s, bool prepare)
                                      max_dyn_smem() - (int)kRegStatic));
         return XT_OK;
     }
-    kernel<<<q * g.count, (g.ncw + 1) * 32, g.smem, s>>>(a, q, nullptr, nullptr);
+    kernel<<<q * g.count, (g.ncw + 1) * 32, g.smem, s>>>(a, q, nullptr, nullptr, ring_polls());
     note_launches(1);
     XT_CUDA(cudaGetLastError());
     return XT_OK;

@@ -32,9 +32,7 @@
 // Flow.  One warp copies whole levels ahead into a ring in shared memory
 // (cp.async.bulk, an mbarrier per level) and the others read the next level's
 // entry into registers between the multiply-adds of the current one.  Waits
-// are bounded: one that gives up raises the error word that ilu_check reads,
-// starts no further copy, lets the remaining levels run on what is there and
-// leaves once the copies have landed.
+// are bounded; what follows one that gives up is as in ilu_ring.cuh.
 //
 // Measured (one apply through the C ABI with host vectors, GB300), before
 // with the row records through the ring in one thread block: 20 x 20 x 60 rod
@@ -343,6 +341,7 @@ struct RowArgs {
     long long rstride, ostride;  // between temporal blocks
     int nl, ncw, zero, win;
     int* err;
+    int polls;  // of a wait
 };
 
 // Levels in flight: a level takes 1,200 cycles and more, four cover a read
@@ -353,7 +352,7 @@ template <int G, int H>
 __host__ __device__ constexpr int ring_bytes() { return row_slot_bytes<G, H>() + 32 * 8; }
 __host__ __device__ constexpr unsigned window_bytes(int win) { return ((unsigned)win * 8u + 127u) / 128u * 128u; }
 
-constexpr int kRowSpin = 1 << 20;
+constexpr int kRowSpin = 1 << 20;  // polls of a wait for the copies in flight after one gave up
 
 // Warps 0 .. ncw - 1 compute; the last warp copies levels into the ring and
 // waits for them, one level barrier ahead of the warps that read them: a wait
@@ -386,12 +385,25 @@ __global__ void __launch_bounds__((kRowWarps + 1) * 32, 1) k_tri_rows(RowArgs a)
             bulk_copy(to, a.slots + (size_t)l * lev_slots, lev_slots, bar);
             bulk_copy(to + lev_slots, gb + (size_t)l * a.ncw * 32, lev_rhs, bar);
         };
-        auto wait = [&](int l) { return bar_wait(smem_at(bars + l % NR), (unsigned)(l / NR) & 1u, kRowSpin); };
+        auto landed = [&](int l, int polls) {
+            return bar_wait(smem_at(bars + l % NR), (unsigned)(l / NR) & 1u, polls);
+        };
         bool ok = true;
         int issued = min(NR, a.nl);
+        // level l is there, or, once a wait has given up, every level in
+        // flight has landed or its place is zeroed (no chunk)
+        auto wait = [&](int l) {
+            ok = landed(l, a.polls);
+            if (ok) return;
+            for (int m = l; m < issued; ++m)
+                if (!landed(m, kRowSpin))
+                    for (unsigned o = 0; o < lev; o += 16u)
+                        asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(ring + (unsigned)(m % NR) * lev + o), "r"(0) : "memory");
+        };
         if (lane == 0) {
             for (int l = 0; l < issued; ++l) copy(l);
-            ok = wait(0) && (a.nl < 2 || wait(1));
+            wait(0);
+            if (ok && a.nl > 1) wait(1);
         }
         __syncwarp();
         asm volatile("bar.sync 0;" ::: "memory");  // levels 0 and 1 are there
@@ -404,15 +416,12 @@ __global__ void __launch_bounds__((kRowWarps + 1) * 32, 1) k_tri_rows(RowArgs a)
                     copy(m);
                     issued = m + 1;
                 }
-                if (l + 2 < a.nl) ok = wait(l + 2);
+                if (l + 2 < a.nl) wait(l + 2);
             }
             __syncwarp();
             asm volatile("bar.sync 0;" ::: "memory");
         }
-        if (lane == 0 && !ok) {  // leave with no copy in flight
-            for (int l = max(0, issued - NR); l < issued; ++l) (void)wait(l);
-            *a.err = 1;
-        }
+        if (lane == 0 && !ok) *a.err = 1;
         return;
     }
     const int lane0 = (lane / GS) * GS;
@@ -632,9 +641,11 @@ int launch_both(const RowSweep& R, int q, double* z, cudaStream_t s)
     XT_TRY(ilu_error_word(&err));
     double *rl = reinterpret_cast<double*>(R.rhsL.p), *ru = reinterpret_cast<double*>(R.rhsU.p);
     XT_TRY((launch_shares<G, false>(
-        R.L, RowArgs{R.L.slots.p, rl, ru, R.L.lanes, R.U.lanes, R.L.nl, R.L.ncw, R.L.zero, R.L.win, err}, q, s)));
+        R.L, RowArgs{R.L.slots.p, rl, ru, R.L.lanes, R.U.lanes, R.L.nl, R.L.ncw, R.L.zero, R.L.win, err,
+                   ring_polls()}, q, s)));
     return launch_shares<G, true>(
-        R.U, RowArgs{R.U.slots.p, ru, z, R.U.lanes, 0, R.U.nl, R.U.ncw, R.U.zero, R.U.win, err}, q, s);
+        R.U, RowArgs{R.U.slots.p, ru, z, R.U.lanes, 0, R.U.nl, R.U.ncw, R.U.zero, R.U.win, err, ring_polls()},
+        q, s);
 }
 
 template <int Q>

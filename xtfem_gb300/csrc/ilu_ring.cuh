@@ -8,9 +8,11 @@
 // from it.  The copying warp takes no part in the levels: starting a copy
 // takes it about 200 cycles and an mbarrier wait 180 however long ago the copy
 // landed (joined to every level barrier it made a level of one warp 730 cycles
-// long).  Its waits are bounded: one that gives up raises the error word that
-// ilu_check reads, starts no further copy, lets the remaining levels run on
-// what is there and leaves once the copies have landed.
+// long).  Its waits are bounded.  Once one has given up it starts no further
+// copy, waits for those in flight with the full limit (settle), then hands over
+// the remaining parts as they are, by the same barriers, and the error word
+// that ilu_check reads is raised.  The computing warps run on, over records
+// that have landed or were zeroed: old data, but addresses within the buffers.
 //
 // Named barriers: 1 levels (the computing warps); 2, 3 a part has landed
 // (even, odd parts); 4, 5 a part has been read.  Both sides take part in every
@@ -20,7 +22,7 @@
 namespace xt {
 
 constexpr int kRingParts = 4;
-constexpr int kRingSpin = 1 << 20;  // polls of a wait before it gives up
+constexpr int kRingSpin = 1 << 20;  // polls of a wait in settle
 
 __device__ __forceinline__ void ring_sync(int id, int threads)
 {
@@ -34,6 +36,37 @@ __device__ __forceinline__ void ring_arrive(int id, int threads)
 __device__ __forceinline__ void ring_level(int threads)
 {
     asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
+}
+
+// Part m has landed, within `polls` polls of its mbarrier.
+__device__ __forceinline__ bool ring_wait(unsigned bars, int m, int polls)
+{
+    const unsigned bar = bars + 8u * (unsigned)(m % kRingParts), parity = (unsigned)(m / kRingParts) & 1u;
+    for (int i = 0; i < polls; ++i) {
+        unsigned ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+// One thread, after a wait has given up: parts m .. issued - 1 have landed, or,
+// should one not within the full limit, its place is zeroed, for the computing
+// warps take addresses from what they read.  A record of zeros reads and writes
+// element 0 of its buffers.  (Not inlined: the copying warp's loop stays short.)
+__device__ __noinline__ void ring_settle(unsigned at, unsigned bars, unsigned part, int m, int issued)
+{
+    for (; m < issued; ++m) {
+        if (ring_wait(bars, m, kRingSpin)) continue;
+        const unsigned to = at + (unsigned)(m % kRingParts) * part;
+        for (unsigned o = 0; o < part; o += 16u)
+            asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(to + o), "r"(0) : "memory");
+    }
 }
 
 struct SweepRing {
@@ -79,31 +112,20 @@ struct SweepRing {
             "l"(rhs + (size_t)m * B * lev_rhs), "r"(n * lev_rhs), "r"(bar)
             : "memory");
     }
-    __device__ __forceinline__ bool wait(int m) const
-    {
-        const unsigned bar = bars + 8u * (unsigned)(m % kRingParts), parity = (unsigned)(m / kRingParts) & 1u;
-        for (int i = 0; i < kRingSpin; ++i) {
-            unsigned ok;
-            asm volatile(
-                "{\n\t.reg .pred p;\n\t"
-                "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                "selp.u32 %0, 1, 0, p;\n\t}"
-                : "=r"(ok)
-                : "r"(bar), "r"(parity)
-                : "memory");
-            if (ok) return true;
-        }
-        return false;
-    }
-    // the copying warp's whole work; false when a wait gave up
-    __device__ __forceinline__ bool copies(const unsigned char* slots, const unsigned char* rhs, int lane) const
+    // the copying warp's whole work, its waits of at most `polls` polls; false
+    // in lane 0, which alone copies and waits, when one gave up
+    __device__ __forceinline__ bool copies(const unsigned char* slots, const unsigned char* rhs, int lane,
+                                           int polls) const
     {
         int issued = min(kRingParts, nparts);
         bool ok = true;
         if (lane == 0)
             for (int m = 0; m < issued; ++m) copy(m, slots, rhs);
         for (int m = 0; m < nparts; ++m) {
-            if (lane == 0 && ok) ok = wait(m);
+            if (lane == 0 && ok) {
+                ok = ring_wait(bars, m, polls);
+                if (!ok) ring_settle(at, bars, part, m, issued);
+            }
             __syncwarp();
             ring_arrive(2 + (m & 1), all());
             // the part before has been read: its place takes the next copy
@@ -115,8 +137,6 @@ struct SweepRing {
                 }
             }
         }
-        if (lane == 0 && !ok)  // leave with no copy in flight
-            for (int m = max(0, issued - kRingParts); m < issued; ++m) (void)wait(m);
         return ok;
     }
 };

@@ -93,4 +93,13 @@ inline int env_int(const char* name, int dflt)
     return e ? std::atoi(e) : dflt;
 }
 
+// Polls of a ring wait for a level's data.  XTFEM_ILU_SPIN_LIMIT=N makes it
+// N - 1, so that 1 gives up at once whatever has landed (tests make a wait run
+// out with the GPU still answering).
+inline int ring_polls()
+{
+    const int n = env_int("XTFEM_ILU_SPIN_LIMIT", 0);
+    return n > 0 ? n - 1 : 1 << 20;
+}
+
 }  // namespace xt
