@@ -1557,6 +1557,13 @@ size_t reg_smem(const RegTri& t)
     return reg_pad((unsigned)t.win_elems * 4u) +
            (size_t)kRingParts * t.nr * reg_level_bytes(t, t.smax, t.w16);
 }
+// Warps with which four parts of one level each fit in `room` bytes beside
+// the window.
+int reg_fit_warps(const RegTri& t, int smax, bool w16, long long room)
+{
+    const long long per = reg_slot_bytes(t.H, smax, w16) + 128u / (unsigned)t.H;
+    return (int)std::max(0LL, (room - (long long)reg_pad((unsigned)t.win_elems * 4u)) / (kRingParts * per));
+}
 int reg_ring(const RegTri& t, int smax, bool w16, long long room)
 {
     return ring_levels(reg_level_bytes(t, smax, w16), t.ncw, room - (long long)reg_pad((unsigned)t.win_elems * 4u));
@@ -1698,8 +1705,9 @@ int build_reg(const IluSched& S, int Q, int H, IluStage& st, cudaStream_t s)
     // fewer warps (more sub-levels) where the ring does not fit
     const long long room = (long long)max_dyn_smem() - kRegStatic;
     auto fit = [&](const TriHost& h, RegTri& t) {
-        while ((t.nr = reg_ring(t, smax, w16, room)) == 0 && t.ncw > 1)
-            if (!reg_plan(h, H, t, t.ncw - 1)) return false;
+        const int most = reg_fit_warps(t, smax, w16, room);
+        if (most < 1 || (most < t.ncw && !reg_plan(h, H, t, most))) return false;
+        t.nr = reg_ring(t, smax, w16, room);
         t.w16 = w16;
         return t.nr > 0;
     };
@@ -1967,11 +1975,20 @@ int build_reg_parts(const DevIlu& F, int Q, int H, IluStage& st, cudaStream_t s)
     const int smax = reg_smax(H, need);
     if (smax == 0) return XT_OK;
     const bool w16 = (long long)win * 4 <= 65536 && env_int("XTFEM_ILU_W16", 1) != 0;
+    // fewer warps (more sub-levels) where a block's ring does not fit
+    const long long room = (long long)max_dyn_smem() - kRegStatic;
+    int most = ncw;
     for (auto* v : {&Ls, &Us})
-        for (auto& t : *v) {
-            t->nr = reg_ring(*t, smax, w16, (long long)max_dyn_smem() - kRegStatic);
-            if (t->nr == 0) return XT_OK;
-        }
+        for (auto& t : *v) most = std::min(most, reg_fit_warps(*t, smax, w16, room));
+    if (most < 1) return XT_OK;
+    if (most < ncw) {
+        ncw = most;
+        for (int b = 0; b < P; ++b)
+            if (!reg_plan(F.part_sched[b]->L, H, *Ls[b], ncw) || !reg_plan(F.part_sched[b]->U, H, *Us[b], ncw))
+                return XT_OK;
+    }
+    for (auto* v : {&Ls, &Us})
+        for (auto& t : *v) t->nr = reg_ring(*t, smax, w16, room);
     std::vector<long long> offL(P + 1, 0), offU(P + 1, 0);
     for (int b = 0; b < P; ++b) {
         offL[b + 1] = offL[b] + Ls[b]->lanes;
