@@ -490,7 +490,13 @@ __global__ void __launch_bounds__(nb_threads<STAGED>(), STAGED ? 8 : 1) kb_kron_
 // instruction every 19 cycles of an SM) is what bounds the operator, 1.72 M
 // warp instructions and 105 us on the 20 x 20 x 60 rod (q = 6).  The CSR
 // kernel spends half as much again on row tails and the lanes' tree sums.
-// Measured there: 119 us; figures against the CSR kernel at kron_spmm.
+//
+// A thread keeps nine sums of KX (DOF of the block, block mod 3) and three of
+// MX, of nine terms each on a hexahedral mesh, and mixes in four: one sum of 81
+// terms in sequence had 1.5 times the rounding of the CSR kernel's eight lanes
+// (2.75e-16 of the result in the 2-norm against 1.78e-16; this 1.70e-16).
+// Measured on that rod: 132 us (119 with the one sum); figures against the CSR
+// kernel at kron_spmm.
 template <int Q>
 __global__ void __launch_bounds__(256)
 k_kron_nb64(int nodes, const int* __restrict__ bptr, const int* __restrict__ bcol,
@@ -511,9 +517,8 @@ k_kron_nb64(int nodes, const int* __restrict__ bptr, const int* __restrict__ bco
     const bool act = nl < NPB && a < nodes;
     double ak = 0.0, am = 0.0;
     if (act) {
-        const int b1 = bptr[a + 1];
-#pragma unroll 3
-        for (int k = bptr[a]; k < b1; ++k) {
+        double s0[3] = {}, s1[3] = {}, s2[3] = {}, sm[3] = {};
+        auto block = [&](int k, int u) {
             const double* xb = x + (size_t)bcol[k] * TPN + b;
             const double* kr = kv + (size_t)k * 9 + c * 3;
             const double x0 = xb[0], x1 = xb[Q], x2 = xb[2 * Q];
@@ -521,30 +526,43 @@ k_kron_nb64(int nodes, const int* __restrict__ bptr, const int* __restrict__ bco
             const double k0 = kr[0], k1 = kr[1], k2 = kr[2], m = mv[k];
             const int mk = mask[k];
             if (mk == 0xfff) {
-                ak = fma(k0, x0, ak);
-                ak = fma(k1, x1, ak);
-                ak = fma(k2, x2, ak);
-                am = fma(m, xc, am);
+                s0[u] = fma(k0, x0, s0[u]);
+                s1[u] = fma(k1, x1, s1[u]);
+                s2[u] = fma(k2, x2, s2[u]);
+                sm[u] = fma(m, xc, sm[u]);
             } else {  // only the entries that K and M have: 0 times an infinite x is no zero
                 const int r = mk >> (3 * c);
-                if (r & 1) ak = fma(k0, x0, ak);
-                if (r & 2) ak = fma(k1, x1, ak);
-                if (r & 4) ak = fma(k2, x2, ak);
-                if (mk >> 9) am = fma(m, xc, am);
+                if (r & 1) s0[u] = fma(k0, x0, s0[u]);
+                if (r & 2) s1[u] = fma(k1, x1, s1[u]);
+                if (r & 4) s2[u] = fma(k2, x2, s2[u]);
+                if (mk >> 9) sm[u] = fma(m, xc, sm[u]);
             }
+        };
+        const int b1 = bptr[a + 1];
+        int k = bptr[a];
+        for (; k + 3 <= b1; k += 3) {
+            block(k, 0);
+            block(k + 1, 1);
+            block(k + 2, 2);
         }
+        if (k < b1) block(k, 0);
+        if (k + 1 < b1) block(k + 1, 1);
+        auto sum = [](const double (&s)[3]) { return (s[0] + s[1]) + s[2]; };
+        ak = (sum(s0) + sum(s1)) + sum(s2);
+        am = sum(sm);
     }
     sK[t] = ak;
     sM[t] = am;
     __syncthreads();
     if (act) {
         const int base = t - b;
-        double acc = 0.0;
+        double pk[2] = {}, pm[2] = {};
 #pragma unroll
         for (int j = 0; j < Q; ++j) {
-            acc = fma(sA[j * Q + b], sK[base + j], acc);
-            acc = fma(sB[j * Q + b], sM[base + j], acc);
+            pk[j & 1] = fma(sA[j * Q + b], sK[base + j], pk[j & 1]);
+            pm[j & 1] = fma(sB[j * Q + b], sM[base + j], pm[j & 1]);
         }
+        const double acc = (pk[0] + pk[1]) + (pm[0] + pm[1]);
         double* yp = y + (size_t)(3 * a + c) * Q + b;
         *yp = beta == 0.0 ? alpha * acc : fma(beta, *yp, alpha * acc);
     }
@@ -853,8 +871,8 @@ int kron_spmm(const DevCsr& K, const DevCsr& M, int q, const double* dA,
         // FP64 in node blocks where these hold little but K's own entries (a
         // place without an entry costs its issue all the same: with blocks
         // less than 5/8 full the CSR kernel does less work).  20 x 20 x 60
-        // rod, q = 6: 179 us in CSR form, 119 us in blocks (255 us in CSR form
-        // with a mixing branch per output); 10 x 10 x 30 rod 38 and 25 us.
+        // rod, q = 6: 180 us in CSR form, 132 us in blocks (251 us in CSR form
+        // with a mixing branch per output); 10 x 10 x 30 rod 38 and 27.5 us.
         if (K.nb.ok && 5LL * 9 * K.nb.nblocks <= 8LL * K.nnz && nb_enabled()) {
             switch (q) {
             case 1: return launch_nb64<1>(K.nb, dA, dB, alpha, beta, x, y, s);
