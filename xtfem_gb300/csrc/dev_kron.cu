@@ -161,7 +161,8 @@ k_kron_spmm(int p, const int* __restrict__ kptr, const int* __restrict__ kcol,
     }
 }
 
-// XTFEM_KRON_NB=0 keeps the CSR kernel (tests compare the two).
+// XTFEM_KRON_NB=0 keeps the CSR kernels, 2 takes the FP64 node blocks at any
+// size (tests compare the two).
 bool nb_enabled()
 {
     const char* e = std::getenv("XTFEM_KRON_NB");
@@ -868,12 +869,19 @@ int kron_spmm(const DevCsr& K, const DevCsr& M, int q, const double* dA,
     }
     if (K.n == 0) return XT_OK;
     if constexpr (sizeof(T) == 8) {
-        // FP64 in node blocks where these hold little but K's own entries (a
+        // FP64 in node blocks where the rows fill the GPU (a thread follows a
+        // node row's blocks alone, 20 us for 27 of them however few the rows:
+        // us in CSR form and in blocks, q = 6, at 325 nodes 17.2 and 20.8, 1,539
+        // 18.4 and 20.0, 2,080 27.5 and 20.7; q = 3, 3,025 17.3 and 21.1, 3,751
+        // 23.1 and 21.0; q = 1, 14,801 27.5 and 29.4, 22,491 36.4 and 29.4) and
+        // the blocks hold little but K's own entries (a
         // place without an entry costs its issue all the same: with blocks
         // less than 5/8 full the CSR kernel does less work).  20 x 20 x 60
         // rod, q = 6: 180 us in CSR form, 132 us in blocks (251 us in CSR form
         // with a mixing branch per output); 10 x 10 x 30 rod 38 and 27.5 us.
-        if (K.nb.ok && 5LL * 9 * K.nb.nblocks <= 8LL * K.nnz && nb_enabled()) {
+        const char* e = std::getenv("XTFEM_KRON_NB");
+        const bool large = (long long)q * K.nb.nodes >= (q < 3 ? 16000 : 10500) || (e && std::atoi(e) == 2);
+        if (K.nb.ok && large && 5LL * 9 * K.nb.nblocks <= 8LL * K.nnz && nb_enabled()) {
             switch (q) {
             case 1: return launch_nb64<1>(K.nb, dA, dB, alpha, beta, x, y, s);
             case 2: return launch_nb64<2>(K.nb, dA, dB, alpha, beta, x, y, s);
