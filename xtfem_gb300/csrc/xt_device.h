@@ -107,7 +107,7 @@ struct DevNodeBlocks {
     DBuf<float2> mdf;      // 1 per block, double-float
     DBuf<double> k64, m64; // the same in FP64
     DBuf<int> mask;        // entries of the block that K (bits 0..8) and M (9..11) have
-    DBuf<int> from_csr;    // K's nnz entries: position of each in kdf
+    DBuf<int> from_csr;    // K's nnz entries: position of each in kdf and k64
 };
 
 
@@ -142,8 +142,11 @@ struct DevCsr {
 int node_blocks_refresh(DevCsr& K, cudaStream_t s);
 
 // Builds K.nb from the 1-based host CSR pairs after both were uploaded;
-// leaves K.nb.ok false when the pair has no exact node-block form (order
-// not a multiple of 3, M not m_ab I3 blockwise, or M outside K's blocks).
+// leaves K.nb.ok false when the pair has no exact node-block form: order
+// not a multiple of 3, M not m_ab I3 blockwise, M outside K's blocks, or a
+// column listed twice.  One node with some but not all of its components
+// constrained (a roller) is enough, for M lacks those components' entries:
+// the whole system then runs through the CSR kernels.
 int csr_build_node_blocks(DevCsr& K, int n, const int* ki, const int* kj, const double* kv,
                           const int* mi, const int* mj, const double* mv, cudaStream_t s);
 
