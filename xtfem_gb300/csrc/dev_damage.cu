@@ -37,14 +37,13 @@ namespace xt {
 namespace {
 
 // src/damage.h:9-17
-constexpr double CY = 1740.0, HH = 0.2, SD = 0.5, SEXP = 0.5, SIGF = 180.0, SIGU = 577.0,
-                 EPSD = 0.08;
+constexpr double CY = 1740.0, HH = 0.2, SD = 0.5, SIGF = 180.0, SIGU = 577.0, EPSD = 0.08;
 constexpr double WD = (SIGU - SIGF) * EPSD;
 constexpr int kNtChunk = 1024;  // temporal points per shared-memory chunk
 constexpr int kRun = 32;        // steps proven elastic by one bound
 
 struct Mat {
-    double nu, E, ca, cb, G, Kb, coef;
+    double nu, E, ca, cb, coef;
 };
 
 __device__ __forceinline__ double vm_equiv(const double s[6])
@@ -226,8 +225,10 @@ __device__ __noinline__ void slow_materialize(Slow* s, const double* __restrict_
 // points, 2,560 steps, host arrays, 31.0 -> 5.1 ms; no plastic point (192,000
 // points, 25,600 steps) 2.1 -> 0.45 ms, from the chunk bound and fused sums.
 //
-// L = 32 (one point a warp) when few of the warp's points need exact steps,
-// else L = 8 (four points a warp, each FP64 instruction serving four).  The
+// L = 32 for a warp's only point that needs exact steps (32 steps a screening
+// pass), else L = 8 (four points a warp, each FP64 instruction serving four; two
+// points one after the other with L = 32 took 569 points of a 10 x 10 x 30 rod
+// 8.3 ms in place of 4.9, 726 of a 14 x 14 x 40 one 11.9 in place of 6.7).  The
 // teams of a warp run in step: every branch below is taken by the whole warp
 // (a vote), and a team that does not take part keeps its values.
 template <int L>
@@ -453,7 +454,7 @@ struct Team {
             const double r = sqrt(fma(ky, sp, -yn) * (1.0 / SD));
             if (ws < WD) rate = r;
         }
-        // SEXP = 1/2
+        // (the exponent of the damage law, src/damage.h:15, is 1/2)
         const double nd = grow ? fma(rate, dp, d) : 0.0;
         const bool changed = take && nd != d;
         if (take) {
@@ -618,70 +619,70 @@ __device__ __noinline__ void exact_points(const DamageArgs& A, const float* __re
     }
 }
 
-// The slab's update of point gidx (a copy of the last point, storing
-// nothing, when gidx is past it: every thread of the block must reach the
-// barriers of the chunk loop).
+// The slab's update of point gidx.  A thread without a point (gidx past the
+// last one) loads and screens nothing: it is there for the barriers of the chunk
+// loop and the warp's votes.
 __device__ __forceinline__ void damage_point(const DamageArgs& a, const float* __restrict__ ntmax,
                                              int run_bound, long long gidx)
 {
     const bool live = gidx < a.ngp;
-    const int gp = live ? (int)gidx : a.ngp - 1;
+    const int gp = live ? (int)gidx : 0;
     Slow s;
-    Mat& m = s.m;
-    m.nu = a.nu[gp];
-    m.E = a.ym[gp];
-    m.ca = (1.0 + m.nu) / (3.0 * (1.0 - m.nu));
-    m.cb = 2.0 * (4.0 - 5.0 * m.nu) / (15.0 * (1.0 - m.nu));
-    m.G = m.E / (2.0 * (1.0 + m.nu));
-    m.Kb = m.E / (3.0 * (1.0 - 2.0 * m.nu));
-    m.coef = m.E / ((1.0 + m.nu) * (1.0 - 2.0 * m.nu));
-
-    // strain basis E_k = B u_k (6 temporal blocks, checked on the host)
-    for (int k = 0; k < 6; ++k)
-        for (int c = 0; c < 6; ++c) s.E[k][c] = 0.0;
-    for (int i = 0; i < a.nnse; ++i) {
-        const int nd = a.nodes[(size_t)gp * a.nnse + i] - 1;
-        const double nx = a.Nx[(size_t)gp * a.nnse + i];
-        const double ny = a.Ny[(size_t)gp * a.nnse + i];
-        const double nz = a.Nz[(size_t)gp * a.nnse + i];
-        for (int k = 0; k < 6; ++k) {
-            const double* u = a.sol + (size_t)k * a.nn * a.ndofn + (size_t)nd * a.ndofn;
-            const double u0 = u[0], u1 = u[1], u2 = u[2];
-            s.E[k][0] = fma(nx, u0, s.E[k][0]);
-            s.E[k][1] = fma(ny, u1, s.E[k][1]);
-            s.E[k][2] = fma(nz, u2, s.E[k][2]);
-            s.E[k][3] = fma(ny, u0, fma(nx, u1, s.E[k][3]));
-            s.E[k][4] = fma(nz, u1, fma(ny, u2, s.E[k][4]));
-            s.E[k][5] = fma(nz, u0, fma(nx, u2, s.E[k][5]));
-        }
-    }
     State& st = s.st;
     const size_t b6 = (size_t)gp * a.ncmp;
-    for (int i = 0; i < 6; ++i) {
-        st.epo[i] = a.eps_old[b6 + i];
-        st.epl[i] = a.eps_pl[b6 + i];
-        st.sef[i] = a.sig_eff[b6 + i];
-        st.sbk[i] = a.sig_back[b6 + i];
-    }
-    st.p = a.p[gp];
-    st.d = a.D[gp];
-    st.ws = a.ws[gp];
-    st.dpo = a.del_po[gp];
-    st.sigd = a.sig_d[gp];
+    float G[6][6] = {}, C0[6] = {}, ecomp[6] = {}, err2 = 0.0f;
+    if (live) {
+        Mat& m = s.m;
+        m.nu = a.nu[gp];
+        m.E = a.ym[gp];
+        m.ca = (1.0 + m.nu) / (3.0 * (1.0 - m.nu));
+        m.cb = 2.0 * (4.0 - 5.0 * m.nu) / (15.0 * (1.0 - m.nu));
+        m.coef = m.E / ((1.0 + m.nu) * (1.0 - 2.0 * m.nu));
 
-    Screen sc;
-    slow_screen(&s, ntmax, &sc);
-    float G[6][6], C0[6], ecomp[6], err2;
+        // strain basis E_k = B u_k (6 temporal blocks, checked on the host)
+        for (int k = 0; k < 6; ++k)
+            for (int c = 0; c < 6; ++c) s.E[k][c] = 0.0;
+        for (int i = 0; i < a.nnse; ++i) {
+            const int nd = a.nodes[(size_t)gp * a.nnse + i] - 1;
+            const double nx = a.Nx[(size_t)gp * a.nnse + i];
+            const double ny = a.Ny[(size_t)gp * a.nnse + i];
+            const double nz = a.Nz[(size_t)gp * a.nnse + i];
+            for (int k = 0; k < 6; ++k) {
+                const double* u = a.sol + (size_t)k * a.nn * a.ndofn + (size_t)nd * a.ndofn;
+                const double u0 = u[0], u1 = u[1], u2 = u[2];
+                s.E[k][0] = fma(nx, u0, s.E[k][0]);
+                s.E[k][1] = fma(ny, u1, s.E[k][1]);
+                s.E[k][2] = fma(nz, u2, s.E[k][2]);
+                s.E[k][3] = fma(ny, u0, fma(nx, u1, s.E[k][3]));
+                s.E[k][4] = fma(nz, u1, fma(ny, u2, s.E[k][4]));
+                s.E[k][5] = fma(nz, u0, fma(nx, u2, s.E[k][5]));
+            }
+        }
+        for (int i = 0; i < 6; ++i) {
+            st.epo[i] = a.eps_old[b6 + i];
+            st.epl[i] = a.eps_pl[b6 + i];
+            st.sef[i] = a.sig_eff[b6 + i];
+            st.sbk[i] = a.sig_back[b6 + i];
+        }
+        st.p = a.p[gp];
+        st.d = a.D[gp];
+        st.ws = a.ws[gp];
+        st.dpo = a.del_po[gp];
+        st.sigd = a.sig_d[gp];
+
+        Screen sc;
+        slow_screen(&s, ntmax, &sc);
 #pragma unroll
-    for (int k = 0; k < 6; ++k)
+        for (int k = 0; k < 6; ++k)
 #pragma unroll
-        for (int i = 0; i < 6; ++i) G[k][i] = sc.G[k][i];
+            for (int i = 0; i < 6; ++i) G[k][i] = sc.G[k][i];
 #pragma unroll
-    for (int i = 0; i < 6; ++i) {
-        C0[i] = sc.C0[i];
-        ecomp[i] = sc.e[i];
+        for (int i = 0; i < 6; ++i) {
+            C0[i] = sc.C0[i];
+            ecomp[i] = sc.e[i];
+        }
+        err2 = sc.err2;
     }
-    err2 = sc.err2;
     // proven elastic when q + err2 < sig_f^2 (margin covers the float add)
     const float thr = (float)(SIGF * SIGF) * 0.99999976f;
     int last_el = -1;  // last step known elastic whose outputs are pending
@@ -698,7 +699,7 @@ __device__ __forceinline__ void damage_point(const DamageArgs& a, const float* _
     // mx_k |g_ki| with mx_k the chunk's largest |Nt_k|, inflated as the run
     // bound below.  Most points (stress well under yield) need nothing else,
     // and a block of such points does not load the chunk's table.
-    bool open = first < 0;
+    bool open = live && first < 0;
     if (run_bound && open && err2 < thr) {
         const float* mx = ntmax + 8 * (1 + j0 / kNtChunk);
         float qb = 0.0f;
@@ -788,12 +789,10 @@ __device__ __forceinline__ void damage_point(const DamageArgs& a, const float* _
     }
     }
     // Points with an unproven step go to the whole warp, which takes the rest
-    // of their slab; nothing of their state has changed yet.  Two points or
-    // fewer one after another (their plastic chains at full speed, 32 steps a
-    // screening pass), more four at a time.
+    // of their slab; nothing of their state has changed yet.
     const unsigned todo = __ballot_sync(0xffffffffu, live && first >= 0);
     if (todo) {
-        if (__popc(todo) <= 2) exact_points<32>(a, ntmax, todo, gp, first, last_el);
+        if (__popc(todo) == 1) exact_points<32>(a, ntmax, todo, gp, first, last_el);
         else exact_points<8>(a, ntmax, todo, gp, first, last_el);
     }
     if (!live || first >= 0) return;
@@ -823,7 +822,7 @@ __device__ __forceinline__ void damage_point(const DamageArgs& a, const float* _
 // a few blocks on a few SMs while the rest of the GPU idles.  One pass per
 // slot is one slot per point; a small grid with several passes keeps the
 // update on a few SMs.  A warp has ppw slots (its first ppw lanes; the others
-// follow along on a copy of the last point): fewer than 32 where the points
+// only keep its barriers and votes): fewer than 32 where the points
 // do not fill the GPU, so that fewer plastic chains share a warp.
 __global__ void __launch_bounds__(256)
 k_damage(DamageArgs a, const float* __restrict__ ntmax, int run_bound, int passes, int ppw)
@@ -1038,11 +1037,15 @@ int damage_update(const DamageArgs& a, cudaStream_t s)
     // points in turn (0: one thread per point)
     const char* eb = std::getenv("XTFEM_DAMAGE_BLOCKS");
     const long long want = eb ? std::atoll(eb) : 0;
-    // slots per warp: as many as leave about twelve warps an SM.  A 1,536-point
-    // update (2,560 steps) takes 7.0 ms with 32 slots a warp, its plastic
-    // points three and more to a warp, and 5.1 ms with one.
+    // slots per warp: as few as make no more than six warps an SM.  A plastic
+    // chain that shares its warp with three others waits for each of theirs to
+    // end, but every warp issues the strains and the screen's coefficients, some
+    // 800 FP64 instructions.  1,536 points, 2,560 steps, without a plastic point,
+    // with 97 and with 278 of them: at most twelve warps an SM 162 us, 5.02 and
+    // 5.99 ms, six 122 us, 5.02 and 5.98, four 96 us, 5.02 and 6.19 (a thread a
+    // point 146 us, 30.8 and 38.4).
     int ppw = 32;
-    while (ppw > 1 && (long long)a.ngp <= (long long)(ppw / 2) * 152 * 12) ppw /= 2;
+    while (ppw > 1 && (long long)a.ngp <= (long long)(ppw / 2) * 152 * 6) ppw /= 2;
     const int slots = nt / 32 * ppw;
     const long long full = ((long long)a.ngp + slots - 1) / slots;
     const int grid = (int)((want > 0 && want < full) ? want : full);
