@@ -238,10 +238,11 @@ struct Team {
     double a, off, w, third;
     double cb, ca, cacb, kb3, g3;     // factors of the moduli (load)
     double cden;                      // the coefficient of d in the lane's quotient of factors()
-    double ky, kn;                    // (1 + nu) / 2E and nu / 2E
+    double ky, kn;                    // (1 + nu) / 2E and nu / 2E, divided by SD
     double E[6];                      // strain basis of the lane's component
     double epo, epl, sef, sbk;        // the lane's components
     double p, d, ws, dpo, sigd;       // the point's scalars
+    double sold;                      // |sigd - SIGF|
     double c1, c3m1, c2i, Ai, Bi, rgam, cyd, hx2;  // factors of d
     float g[6][6], c0[6], err2;       // FP32 screen of the whole point
     double sumg;                      // sum_k ntmax_k |g_k| of the lane's component
@@ -269,8 +270,8 @@ struct Team {
         cacb = ca - cb;
         g3 = 3.0 * (Ey / (2.0 * (1.0 + nu))) * (1.0 - cb);
         cden = i == 0 ? cb : (i == 1 ? ca : HH);
-        ky = (1.0 + nu) / (2.0 * Ey);
-        kn = nu / (2.0 * Ey);
+        ky = (1.0 + nu) / (2.0 * Ey) * (1.0 / SD);
+        kn = nu / (2.0 * Ey) * (1.0 / SD);
         const double coef = Ey / ((1.0 + nu) * (1.0 - 2.0 * nu)), mn = coef * (1.0 - 2.0 * nu);
         const bool norm = i < 3, shear = i >= 3 && i < 6, tr = i == 6;
         a = shear ? 0.5 * mn : (norm || tr ? mn : 0.0);
@@ -311,6 +312,7 @@ struct Team {
         ws = A.ws[gp];
         dpo = A.del_po[gp];
         sigd = A.sig_d[gp];
+        sold = fabs(sigd - SIGF);
     }
 
     // the factors of d: 1 / (1 - cb d), 1 / (1 - ca d), (1 - d) / (1 - H d) and
@@ -397,6 +399,7 @@ struct Team {
             sef = s;
             epo = eps;
             sigd = t;
+            sold = fabs(t - SIGF);
         }
     }
     // plastic corrector; returns whether d changed
@@ -440,18 +443,19 @@ struct Team {
             t += __shfl_xor_sync(mask, t, 2, L);
             t += __shfl_xor_sync(mask, t, 1, L);
             const double yn = kn * (tr2 >= 0.0 ? 1.0 : hx2) * tr2 * tr2;
-            const double root = sqrt(up ? fma(ky, t, -yn) * (1.0 / SD) : t);
+            const double root = sqrt(up ? fma(ky, t, -yn) : t);
             seq = get(root, 0);
             rate = get(root, 4);
         } else {
             seq = sqrt(sum8(v));
         }
-        const double nws = ws + fma(fabs(seq - SIGF), dp, fabs(sigd - SIGF) * dpo) * 0.5;
+        const double snew = fabs(seq - SIGF);
+        const double nws = ws + fma(snew, dp, sold * dpo) * 0.5;
         const bool grow = take && nws >= WD;
         if (any(grow && ws < WD)) {  // the step that crosses the threshold
             const double sp = sum8(lane < 3 ? (nsef < 0.0 ? hx2 : 1.0) * nsef * nsef : 0.0);
             const double yn = kn * (tr2 >= 0.0 ? 1.0 : hx2) * tr2 * tr2;
-            const double r = sqrt(fma(ky, sp, -yn) * (1.0 / SD));
+            const double r = sqrt(fma(ky, sp, -yn));
             if (ws < WD) rate = r;
         }
         // (the exponent of the damage law, src/damage.h:15, is 1/2)
@@ -466,6 +470,7 @@ struct Team {
             d = nd;
             epo = eps;
             sigd = seq;
+            sold = snew;
             dpo = dp;
         }
         return changed;
@@ -1037,7 +1042,7 @@ int damage_update(const DamageArgs& a, cudaStream_t s)
     // points in turn (0: one thread per point)
     const char* eb = std::getenv("XTFEM_DAMAGE_BLOCKS");
     const long long want = eb ? std::atoll(eb) : 0;
-    // slots per warp: as few as make no more than six warps an SM.  A plastic
+    // slots per warp: as few as make no more than four warps an SM.  A plastic
     // chain that shares its warp with three others waits for each of theirs to
     // end, but every warp issues the strains and the screen's coefficients, some
     // 800 FP64 instructions.  1,536 points, 2,560 steps, without a plastic point,
@@ -1045,7 +1050,7 @@ int damage_update(const DamageArgs& a, cudaStream_t s)
     // 5.99 ms, six 122 us, 5.02 and 5.98, four 96 us, 5.02 and 6.19 (a thread a
     // point 146 us, 30.8 and 38.4).
     int ppw = 32;
-    while (ppw > 1 && (long long)a.ngp <= (long long)(ppw / 2) * 152 * 6) ppw /= 2;
+    while (ppw > 1 && (long long)a.ngp <= (long long)(ppw / 2) * 152 * 4) ppw /= 2;
     const int slots = nt / 32 * ppw;
     const long long full = ((long long)a.ngp + slots - 1) / slots;
     const int grid = (int)((want > 0 && want < full) ? want : full);
