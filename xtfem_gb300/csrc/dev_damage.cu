@@ -624,6 +624,9 @@ __device__ __noinline__ void exact_points(const DamageArgs& A, const float* __re
     }
 }
 
+// The larger of two numbers; NaN when one of them is.
+__device__ __forceinline__ float nan_max(float m, float v) { return v > m || v != v ? v : m; }
+
 // The slab's update of point gidx.  A thread without a point (gidx past the
 // last one) loads and screens nothing: it is there for the barriers of the chunk
 // loop and the warp's votes.
@@ -735,7 +738,7 @@ __device__ __forceinline__ void damage_point(const DamageArgs& a, const float* _
             const float* f = reinterpret_cast<const float*>(sNt);
             const float base = f[r0 * 6 + k];
             float mx = 0.0f;
-            for (int j = r0 + 1; j < min(r0 + kRun, jn); ++j) mx = fmaxf(mx, fabsf(f[j * 6 + k] - base));
+            for (int j = r0 + 1; j < min(r0 + kRun, jn); ++j) mx = nan_max(mx, fabsf(f[j * 6 + k] - base));
             sDel[run][k] = mx * 1.000001f + __ldg(ntmax + k) * 2.4e-7f;
         }
     }
@@ -840,23 +843,25 @@ k_damage(DamageArgs a, const float* __restrict__ ntmax, int run_bound, int passe
 }
 
 // max_t |Nt_k(t)| per k of each chunk of kNtChunk steps (one block a chunk)
-// into out + 8 (1 + chunk), then of the whole slab into out
+// into out + 8 (1 + chunk), then of the whole slab into out.  A chunk that holds
+// a NaN has a NaN maximum, so that no bound passes over it; the slab's leaves
+// NaNs out.
 __global__ void __launch_bounds__(256) k_ntmax(const float* __restrict__ nt32, int nip, float* __restrict__ out)
 {
     __shared__ float sh[6][8];
     float m[6] = {0, 0, 0, 0, 0, 0};
     const int j1 = min(nip, ((int)blockIdx.x + 1) * kNtChunk);
     for (int j = blockIdx.x * kNtChunk + threadIdx.x; j < j1; j += blockDim.x)
-        for (int k = 0; k < 6; ++k) m[k] = fmaxf(m[k], fabsf(nt32[(size_t)j * 6 + k]));
+        for (int k = 0; k < 6; ++k) m[k] = nan_max(m[k], fabsf(nt32[(size_t)j * 6 + k]));
     for (int k = 0; k < 6; ++k) {
         float v = m[k];
-        for (int off = 16; off > 0; off >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, off));
+        for (int off = 16; off > 0; off >>= 1) v = nan_max(v, __shfl_xor_sync(0xffffffffu, v, off));
         if ((threadIdx.x & 31) == 0) sh[k][threadIdx.x >> 5] = v;
     }
     __syncthreads();
     if (threadIdx.x < 6) {
         float v = 0.0f;
-        for (int w = 0; w < 8; ++w) v = fmaxf(v, sh[threadIdx.x][w]);
+        for (int w = 0; w < 8; ++w) v = nan_max(v, sh[threadIdx.x][w]);
         out[8 * (1 + blockIdx.x) + threadIdx.x] = v * 1.000001f;
     }
 }
