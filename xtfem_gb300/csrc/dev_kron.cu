@@ -302,16 +302,20 @@ k_kron_df(int p, const int* __restrict__ kptr, const int* __restrict__ kcol,
 // slices in flight; then FP32 (packed operations take two cycles) and
 // shared-memory reads are each busy half the time.
 // Measured (q 6), direct and staged: 25 x 9 x 7 rod 18.7 and 13.3 us, a step of
-// 64 rods in 175 and 168 ms a batch.  A system of more than one round of
-// thread blocks (kNbStagedNodes) reads directly all the same: a queue of
-// blocks that hold shared memory keeps another system's triangular sweep,
-// which wants most of an SM's, from starting (20 x 20 x 60 rod alone 54 and
-// 45 us, but eight of them at once 22.3-24.0 and 20.6 slabs/s).  One or three
+// 64 rods in 175 and 168 ms a batch.  A system alone of more than kNbStagedNodes
+// nodes reads directly all the same: a queue of blocks that hold shared memory
+// keeps another system's triangular sweep, which wants most of an SM's, from
+// starting.  Eight slab loops at once, slabs/s: 3,751 nodes 295 and 303, 5,239
+// nodes 196 and 190, 14,161 nodes 62.3 and 58.2 (one alone the same either way),
+// 26,901 nodes 24 and 20.6.  The kernel of a batch, whose sweeps come between
+// its steps, is staged up to one round of thread blocks: sixteen rods of 5,239
+// nodes 131 and 127 ms, eight of 9,225 nodes 128 and 125.  One or three
 // slices ahead, 64 or 256 threads a block are slower.  q 2 and 4, whose 10 or
 // 5 rows a warp would take too much shared memory, and 8 read directly.
 constexpr int kNbAhead = 2;
 
-constexpr int kNbStagedNodes = 152 * 8 * 12;  // eight blocks an SM of four warps, three node rows each
+constexpr int kNbStagedNodes = 152 * 30;       // two and a half blocks an SM of four warps, three node rows each
+constexpr int kNbStagedBatch = 152 * 8 * 12;  // eight
 
 template <bool STAGED>
 constexpr int nb_threads()
@@ -917,7 +921,7 @@ int kron_nb_batch(const FlexStepItem* t, int count, int q, const FlexStepDims& d
     // a quarter of the largest system's node rows per block pass: each warp
     // loops over about four row groups (any split gives the same rows)
     const int RPW = q == 2 ? 10 : (q == 4 ? 5 : (q == 6 ? 3 : 2));
-    const bool staged = q == 6 && d.nodes_max <= kNbStagedNodes;
+    const bool staged = q == 6 && d.nodes_max <= kNbStagedBatch;
     const int threads = staged ? nb_threads<true>() : nb_threads<false>();
     const int rows_per_block = threads / 32 * RPW;
     const int gx = std::max(1, (d.nodes_max + 4 * rows_per_block - 1) / (4 * rows_per_block));
