@@ -9,10 +9,11 @@
 // takes it about 200 cycles and an mbarrier wait 180 however long ago the copy
 // landed (joined to every level barrier it made a level of one warp 730 cycles
 // long).  Its waits are bounded.  Once one has given up it starts no further
-// copy, waits for those in flight with the full limit (settle), then hands over
-// the remaining parts as they are, by the same barriers, and the error word
-// that ilu_check reads is raised.  The computing warps run on, over records
-// that have landed or were zeroed: old data, but addresses within the buffers.
+// copy, hands over the remaining parts as they are, by the same barriers, raises
+// the error word that ilu_check reads and leaves once the copies in flight have
+// landed.  The computing warps run on, over records of earlier parts or, for the
+// first parts, whose places hold none yet, after ring_settle: wrong sums, but
+// addresses within the buffers.
 //
 // Named barriers: 1 levels (the computing warps); 2, 3 a part has landed
 // (even, odd parts); 4, 5 a part has been read.  Both sides take part in every
@@ -22,7 +23,7 @@
 namespace xt {
 
 constexpr int kRingParts = 4;
-constexpr int kRingSpin = 1 << 20;  // polls of a wait in settle
+constexpr int kRingSpin = 1 << 20;  // polls of a wait before it gives up
 
 __device__ __forceinline__ void ring_sync(int id, int threads)
 {
@@ -55,10 +56,10 @@ __device__ __forceinline__ bool ring_wait(unsigned bars, int m, int polls)
     }
     return false;
 }
-// One thread, after a wait has given up: parts m .. issued - 1 have landed, or,
-// should one not within the full limit, its place is zeroed, for the computing
-// warps take addresses from what they read.  A record of zeros reads and writes
-// element 0 of its buffers.  (Not inlined: the copying warp's loop stays short.)
+// One thread, after the wait for one of the first kRingParts parts has given up:
+// parts m .. issued - 1 have landed, or, should one not within the full limit,
+// its place is zeroed, for the computing warps take addresses from what they
+// read.  A record of zeros reads and writes element 0 of its buffers.
 __device__ __noinline__ void ring_settle(unsigned at, unsigned bars, unsigned part, int m, int issued)
 {
     for (; m < issued; ++m) {
@@ -112,8 +113,11 @@ struct SweepRing {
             "l"(rhs + (size_t)m * B * lev_rhs), "r"(n * lev_rhs), "r"(bar)
             : "memory");
     }
-    // the copying warp's whole work, its waits of at most `polls` polls; false
-    // in lane 0, which alone copies and waits, when one gave up
+    // the copying warp's whole work; false in lane 0, which alone copies and
+    // waits, when a wait gave up.  The waits for the first parts take at most
+    // `polls` polls.  They have a loop of their own: one more test in the loop of
+    // the others costs a part 130 cycles, and with four warps a level the copying
+    // warp is what the others wait for (12 x 12 x 30 rod 177 -> 187 us an apply).
     __device__ __forceinline__ bool copies(const unsigned char* slots, const unsigned char* rhs, int lane,
                                            int polls) const
     {
@@ -121,11 +125,7 @@ struct SweepRing {
         bool ok = true;
         if (lane == 0)
             for (int m = 0; m < issued; ++m) copy(m, slots, rhs);
-        for (int m = 0; m < nparts; ++m) {
-            if (lane == 0 && ok) {
-                ok = ring_wait(bars, m, polls);
-                if (!ok) ring_settle(at, bars, part, m, issued);
-            }
+        auto hand_over = [&](int m) {
             __syncwarp();
             ring_arrive(2 + (m & 1), all());
             // the part before has been read: its place takes the next copy
@@ -136,7 +136,23 @@ struct SweepRing {
                     issued = m + kRingParts;
                 }
             }
+        };
+        const int first = issued;
+#pragma unroll 1
+        for (int m = 0; m < first; ++m) {
+            if (lane == 0 && ok) {
+                ok = ring_wait(bars, m, polls);
+                if (!ok) ring_settle(at, bars, part, m, issued);
+            }
+            hand_over(m);
         }
+#pragma unroll 1
+        for (int m = first; m < nparts; ++m) {
+            if (lane == 0 && ok) ok = ring_wait(bars, m, kRingSpin);
+            hand_over(m);
+        }
+        if (lane == 0 && !ok)  // leave with no copy in flight
+            for (int m = max(0, issued - kRingParts); m < issued; ++m) (void)ring_wait(bars, m, kRingSpin);
         return ok;
     }
 };
