@@ -48,6 +48,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <exception>
+#include <memory>
 #include <string>
 #include <thread>
 #include <vector>
@@ -1571,7 +1572,11 @@ int reg_ring(const RegTri& t, int smax, bool w16, long long room)
 constexpr long long kRegStatic = 2048;  // static shared memory of a sweep, at most
 
 // Slots of a planned triangle.  dst: forward, the other triangle's
-// row_slot; backward (dst empty): row * Q.
+// row_slot; backward (dst empty): row * Q.  The slots are independent and shared
+// out to host threads, for the first apply of a new factor waits for them: on
+// the 20 x 20 x 60 rod 41.6 ms on two threads, 8.9 now, in one-row groups 53.8 and
+// 10.9 (12.4 in the row format), on the 10 x 10 x 30 rod 6.8 and 2.5, 8.7 and 2.8
+// (2.8).
 int reg_fill(const TriHost& h, RegTri& t, int smax, int Q, const std::vector<int>* dst,
              cudaStream_t s, int row0 = 0)
 {
@@ -1580,93 +1585,104 @@ int reg_fill(const TriHost& h, RegTri& t, int smax, int Q, const std::vector<int
     const unsigned rb = reg_rows_bytes(H), ob = reg_offs_bytes(smax, t.w16);
     const int rw = 32 / H;  // row records of a slot
     t.slot_bytes = (int)reg_slot_bytes(H, smax, t.w16);
-    const size_t nslot = (size_t)t.nl * t.ncw;
-    std::vector<unsigned char> blob(nslot * t.slot_bytes, 0);
-    // every lane of every slot starts empty: no store, all steps on the zero slot
-    for (size_t sl = 0; sl < nslot; ++sl) {
-        unsigned char* b = blob.data() + sl * t.slot_bytes;
-        const int none = -1;
-        for (int r = 0; r < rw; ++r) std::memcpy(b + r * 16 + 12, &none, 4);
-        for (int e = 0; e < smax * 32; ++e) {
-            if (t.w16) reinterpret_cast<unsigned short*>(b + rb)[e] = (unsigned short)(t.zero_off * 4);
-            else reinterpret_cast<unsigned*>(b + rb)[e] = (unsigned)t.zero_off * 4u;
-        }
-    }
-    std::vector<int> seen(t.win_elems, 0);
-    int epoch = 0;
-    bool valid = true;
+    const size_t nslot = (size_t)t.nl * t.ncw, bytes = nslot * t.slot_bytes;
+    std::vector<int> chunk_of(nslot, -1);
+    for (size_t c = 0; c < t.chunks.size(); ++c) chunk_of[t.chunk_slot[c]] = (int)c;
+    std::unique_ptr<unsigned char[]> blob(new unsigned char[bytes]);
+    std::atomic<bool> valid{true};
     const bool banks = env_int("XTFEM_ILU_BANKS", 1) != 0;  // 0: entries in row order
-    std::vector<std::vector<std::pair<int, float>>> ent(32);
-    std::vector<int> lanes(32);
-    for (size_t c = 0; c < t.chunks.size(); ++c) {
-        const int slot = t.chunk_slot[c];
-        unsigned char* b = blob.data() + (size_t)slot * t.slot_bytes;
-        float* gm = reinterpret_cast<float*>(b);
-        int* go = reinterpret_cast<int*>(b + 16 * rw);
-        unsigned* off = reinterpret_cast<unsigned*>(b + rb);
-        unsigned short* off16 = reinterpret_cast<unsigned short*>(b + rb);
-        float* val = reinterpret_cast<float*>(b + rb + ob);
-        const auto& grp = t.chunks[c];
-        for (int lane = 0; lane < 32; ++lane) {
-            ent[lane].clear();
-            const int gw = lane / GS, r = (lane % GS) / H, hh = lane % H;
-            if (gw >= GPW || gw >= (int)grp.size()) continue;
-            const int i = grp[gw], G = h.order[i];
-            if (hh == 0) {
-                const int rec = gw * g + r, wo = h.slot[G] * g + r;
-                for (int k = 0; k < g; ++k) gm[rec * 4 + k] = (float)h.minv[((size_t)i * g + r) * g + k];
-                std::memcpy(&gm[rec * 4 + 3], &wo, 4);
-                const long long d = dst ? (long long)(*dst)[(size_t)G * g + r]
-                                        : ((long long)row0 + (long long)G * g + r) * Q;
-                valid = valid && wo >= 0 && wo < t.zero_off && d >= 0 && d < INT32_MAX;
-                go[rec] = (int)d;
-            }
-            const int kb = h.ext_ptr[(size_t)i * g + r], ke = h.ext_ptr[(size_t)i * g + r + 1];
-            for (int k = kb + hh; k < ke; k += H) {
-                const int col = h.ext_col[k], Gc = col / g;
-                ent[lane].push_back({h.slot[Gc] * g + (col - Gc * g), (float)h.ext_v[k]});
-            }
-        }
-        // Step order: at every step each lane takes, of its remaining
-        // entries, one whose shared-memory bank the warp's reads of that step
-        // use least (an address another lane already reads is a broadcast
-        // and costs nothing); lanes with more entries left choose first.
-        for (int st = 0; st < smax; ++st) {
-            int load[32] = {0};
-            ++epoch;
-            for (int l2 = 0; l2 < 32; ++l2) lanes[l2] = l2;
-            std::stable_sort(lanes.begin(), lanes.end(),
-                             [&](int a, int b2) { return ent[a].size() > ent[b2].size(); });
-            for (int lane : lanes) {
-                int o = t.zero_off;
-                float v = 0.0f;
-                if (!ent[lane].empty()) {
-                    size_t best = 0;
-                    int bcost = 1 << 30;
-                    for (size_t e = 0; banks && e < ent[lane].size(); ++e) {
-                        const int a = ent[lane][e].first;
-                        const int cost = seen[a] == epoch ? 0 : load[a & 31] + 1;
-                        if (cost < bcost) { bcost = cost; best = e; }
+    constexpr int kMost = 32;                               // entries of a lane, as reg_plan allows
+    shared_out(nslot, 96, [&](size_t s0, size_t s1) {
+        std::vector<int> seen(t.win_elems, 0);
+        int epoch = 0;
+        bool good = true;
+        int eo[32][kMost], en[32], order[32];
+        float ev[32][kMost];
+        for (size_t sl = s0; sl < s1; ++sl) {
+            unsigned char* b = blob.get() + sl * t.slot_bytes;
+            float* gm = reinterpret_cast<float*>(b);
+            int* go = reinterpret_cast<int*>(b + 16 * rw);
+            unsigned* off = reinterpret_cast<unsigned*>(b + rb);
+            unsigned short* off16 = reinterpret_cast<unsigned short*>(b + rb);
+            float* val = reinterpret_cast<float*>(b + rb + ob);
+            // empty: no store, all steps on the zero slot
+            std::memset(b, 0, rb);
+            const int none = -1;
+            for (int r = 0; r < rw; ++r) std::memcpy(b + r * 16 + 12, &none, 4);
+            std::memset(en, 0, sizeof en);
+            for (int lane = 0; lane < 32 && chunk_of[sl] >= 0; ++lane) {
+                const auto& grp = t.chunks[chunk_of[sl]];
+                const int gw = lane / GS, r = (lane % GS) / H, hh = lane % H;
+                if (gw >= GPW || gw >= (int)grp.size()) continue;
+                const int i = grp[gw], G = h.order[i];
+                if (hh == 0) {
+                    const int rec = gw * g + r, wo = h.slot[G] * g + r;
+                    for (int k = 0; k < g; ++k) gm[rec * 4 + k] = (float)h.minv[((size_t)i * g + r) * g + k];
+                    std::memcpy(&gm[rec * 4 + 3], &wo, 4);
+                    const long long d = dst ? (long long)(*dst)[(size_t)G * g + r]
+                                            : ((long long)row0 + (long long)G * g + r) * Q;
+                    good = good && wo >= 0 && wo < t.zero_off && d >= 0 && d < INT32_MAX;
+                    go[rec] = (int)d;
+                }
+                const int kb = h.ext_ptr[(size_t)i * g + r], ke = h.ext_ptr[(size_t)i * g + r + 1];
+                for (int k = kb + hh; k < ke; k += H) {
+                    if (en[lane] == kMost) {
+                        good = false;
+                        break;
                     }
-                    o = ent[lane][best].first;
-                    v = ent[lane][best].second;
-                    ent[lane].erase(ent[lane].begin() + best);
+                    const int col = h.ext_col[k], Gc = col / g;
+                    eo[lane][en[lane]] = h.slot[Gc] * g + (col - Gc * g);
+                    ev[lane][en[lane]++] = (float)h.ext_v[k];
                 }
-                valid = valid && o >= 0 && o < t.win_elems;
-                if (valid && seen[o] != epoch) {
-                    seen[o] = epoch;
-                    load[o & 31]++;
-                }
-                const size_t oi = reg_step_at(smax, st, lane);
-                if (t.w16) off16[oi] = (unsigned short)(o * 4);
-                else off[oi] = (unsigned)o * 4u;
-                val[oi] = v;
             }
+            // Step order: at every step each lane takes, of its remaining
+            // entries, one whose shared-memory bank the warp's reads of that step
+            // use least (an address another lane already reads is a broadcast
+            // and costs nothing); lanes with more entries left choose first.
+            for (int st = 0; st < smax; ++st) {
+                int load[32] = {0}, first[kMost + 2] = {0};
+                ++epoch;
+                for (int l = 0; l < 32; ++l) ++first[kMost - en[l] + 1];
+                for (int k = 0; k <= kMost; ++k) first[k + 1] += first[k];
+                for (int l = 0; l < 32; ++l) order[first[kMost - en[l]]++] = l;
+                for (int lane : order) {
+                    int o = t.zero_off;
+                    float v = 0.0f;
+                    if (en[lane] > 0) {
+                        int best = 0, bcost = 1 << 30;
+                        for (int e = 0; banks && e < en[lane]; ++e) {
+                            const int a = eo[lane][e];
+                            const int cost = seen[a] == epoch ? 0 : load[a & 31] + 1;
+                            if (cost < bcost) {
+                                bcost = cost;
+                                best = e;
+                            }
+                        }
+                        o = eo[lane][best];
+                        v = ev[lane][best];
+                        for (int e = best + 1; e < en[lane]; ++e) {  // the others keep their order
+                            eo[lane][e - 1] = eo[lane][e];
+                            ev[lane][e - 1] = ev[lane][e];
+                        }
+                        --en[lane];
+                    }
+                    good = good && o >= 0 && o < t.win_elems;
+                    if (good && seen[o] != epoch) {
+                        seen[o] = epoch;
+                        load[o & 31]++;
+                    }
+                    const size_t oi = reg_step_at(smax, st, lane);
+                    if (t.w16) off16[oi] = (unsigned short)(o * 4);
+                    else off[oi] = (unsigned)o * 4u;
+                    val[oi] = v;
+                }
+            }
+            for (int lane = 0; lane < 32; ++lane) good = good && en[lane] == 0;
         }
-        for (int lane = 0; lane < 32; ++lane) valid = valid && ent[lane].empty();
-    }
+        if (!good) valid = false;
+    });
     if (!valid) return XT_OK;
-    XT_TRY(t.slots.upload(blob.data(), blob.size(), s));
+    XT_TRY(t.slots.upload(blob.get(), bytes, s));
     XT_CUDA(cudaStreamSynchronize(s));  // host staging vectors go out of scope
     t.chunks.clear();
     t.chunks.shrink_to_fit();

@@ -2,6 +2,7 @@
 // host helpers shared by the sweep builders (dev_ilu.cu, dev_ilu_rows.cu).
 #pragma once
 
+#include <algorithm>
 #include <cstdlib>
 #include <exception>
 #include <string>
@@ -85,6 +86,35 @@ int side_by_side(A&& a, B&& b)
         return ra;
     }
     return rb;
+}
+
+// fn(begin, end) over [0, n), shared among as many host threads (eight at most)
+// as get `least` items each; an exception is rethrown once all have ended.
+template <class F>
+void shared_out(size_t n, size_t least, F&& fn)
+{
+    const size_t hw = std::max(1u, std::thread::hardware_concurrency());
+    const size_t T = std::max<size_t>(1, std::min({n / least, hw, (size_t)8}));
+    std::vector<std::exception_ptr> err(T);
+    auto part = [&](size_t k) {
+        try {
+            fn(n * k / T, n * (k + 1) / T);
+        } catch (...) {
+            err[k] = std::current_exception();
+        }
+    };
+    std::vector<std::thread> th;
+    th.reserve(T);
+    size_t k = 1;
+    try {
+        for (; k < T; ++k) th.emplace_back(part, k);
+    } catch (const std::exception&) {  // no more threads: the rest here
+    }
+    part(0);
+    for (; k < T; ++k) part(k);
+    for (std::thread& t : th) t.join();
+    for (const std::exception_ptr& e : err)
+        if (e) std::rethrow_exception(e);
 }
 
 inline int env_int(const char* name, int dflt)
