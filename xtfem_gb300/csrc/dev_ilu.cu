@@ -2350,12 +2350,15 @@ int launch_tri(const DevIlu& F, const double* dAinv, const T* v, T* z, T* work, 
     }
     if constexpr (sizeof(T) == 4) {
         if ((F.L.g == 3 || F.L.g == 1) && fmt == 4) {
-            // two lanes a row; one where a level of one-row groups is wider
-            // than the 16 rows of a warp at two (20 x 20 x 60 mesh, 35 rows a
-            // level: a thermal slab 28.9 against 30.4 ms)
-            const int two = F.L.g == 1 && F.L.ngroups > 16LL * F.L.nlevels ? 1 : 2;
-            const int H = F.shares > 0 ? F.shares : env_int("XTFEM_ILU_SHARES", two);
-            XT_TRY(get_stage<T>(F, Q, 4, s, st, H));
+            // two lanes a row with three rows a group; one in one-row groups,
+            // whose levels then need fewer warps (thermal sweeps, one lane and
+            // two, us an apply: 10 x 10 x 30 mesh 166.5 and 170.5, 16 x 16 x 48
+            // 265 and 277, 20 x 20 x 60 332 and 339, 30 x 30 x 30 250 and 298,
+            // plate of 48 x 96 x 2 533 and 542, 4 x 4 x 12 72.3 and 72.0), and
+            // two where a row is longer than one lane takes
+            const int asked = F.shares > 0 ? F.shares : env_int("XTFEM_ILU_SHARES", 0);
+            XT_TRY(get_stage<T>(F, Q, 4, s, st, asked > 0 ? asked : (F.L.g == 1 ? 1 : 2)));
+            if (!st && asked <= 0 && F.L.g == 1) XT_TRY(get_stage<T>(F, Q, 4, s, st, 2));
             if (st) return launch_reg_any<Q>(*st, dAinv, v, z, s, skip);
             fmt = 3;
         }
