@@ -368,7 +368,7 @@ int system_set_mesh(System& S, int nn, int ne, const double* xyz, const int* con
     for (int& v : mrp) ++v;
     for (int& v : mcol) ++v;
     XT_TRY(upload_csr(S.K, n, ia.data(), ja.data(), val.data(), s));
-    XT_TRY(csr_build_node_blocks(S.K, n, ia.data(), ja.data(), val.data(), mrp.data(), mcol.data(),
+    XT_TRY(csr_build_node_blocks(S.K, n, ia.data(), ja.data(), mrp.data(), mcol.data(),
                                  mval.data(), s));
     A.nn = nn;
     A.ne = ne;

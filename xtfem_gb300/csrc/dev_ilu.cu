@@ -746,10 +746,6 @@ k_tri_sweep(TriView<T> t, const double* __restrict__ dAinv, const T* __restrict_
 
 // ---------------------------------------------------------------------------
 // Staged sweep.
-__device__ __forceinline__ unsigned smem_addr(const void* p)
-{
-    return (unsigned)__cvta_generic_to_shared(p);
-}
 __device__ __forceinline__ void mbar_init(unsigned long long* b, unsigned count)
 {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(b)), "r"(count) : "memory");
@@ -1751,32 +1747,6 @@ int build_reg(const IluSched& S, int Q, int H, IluStage& st, cudaStream_t s)
     return XT_OK;
 }
 
-__device__ __forceinline__ float lds_f(unsigned addr)
-{
-    float r;
-    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(r) : "r"(addr));
-    return r;
-}
-__device__ __forceinline__ unsigned lds_u(unsigned addr)
-{
-    unsigned r;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(r) : "r"(addr));
-    return r;
-}
-__device__ __forceinline__ uint2 lds_v2(unsigned addr)
-{
-    uint2 r;
-    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(r.x), "=r"(r.y) : "r"(addr));
-    return r;
-}
-__device__ __forceinline__ uint4 lds_v4(unsigned addr)
-{
-    uint4 r;
-    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
-                 : "r"(addr));
-    return r;
-}
 // One level's data of a lane: window byte offsets (32-bit words, or W16 two
 // 16-bit ones to a word) and factor values of the steps, the row's record,
 // destination and right-hand side.

@@ -46,6 +46,7 @@
 #include <cstdint>
 #include <cstdio>
 
+#include "ilu_ring.cuh"
 #include "ilu_sched.h"
 #include "xt_device.h"
 
@@ -232,62 +233,6 @@ __global__ void k_fill_rows(RowFill f)
     }
 }
 
-__device__ __forceinline__ unsigned smem_at(const void* p)
-{
-    return (unsigned)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ uint4 lds4(unsigned a)
-{
-    uint4 r;
-    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
-                 : "r"(a));
-    return r;
-}
-__device__ __forceinline__ uint2 lds2(unsigned a)
-{
-    uint2 r;
-    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(r.x), "=r"(r.y) : "r"(a));
-    return r;
-}
-__device__ __forceinline__ double lds1(unsigned a)
-{
-    double r;
-    asm volatile("ld.shared.f64 %0, [%1];" : "=d"(r) : "r"(a));
-    return r;
-}
-__device__ __forceinline__ void bar_init(unsigned b)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(b) : "memory");
-}
-__device__ __forceinline__ void bar_expect(unsigned b, unsigned bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(bytes) : "memory");
-}
-// Bounded wait for the phase of the given parity.
-__device__ __forceinline__ bool bar_wait(unsigned b, unsigned parity, int limit)
-{
-    for (int i = 0; i < limit; ++i) {
-        unsigned ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(b), "r"(parity)
-            : "memory");
-        if (ok) return true;
-    }
-    return false;
-}
-__device__ __forceinline__ void bulk_copy(unsigned dst, const void* src, unsigned bytes, unsigned bar)
-{
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-        "l"(src), "r"(bytes), "r"(bar)
-        : "memory");
-}
-
 // A slot in registers; loaded in steps between the multiply-adds of the
 // level before it.
 template <int G, int H>
@@ -301,15 +246,15 @@ struct RowRegs {
     __device__ __forceinline__ void load_rec(unsigned p, unsigned rhs, int lane)
     {
 #pragma unroll
-        for (int k = 0; k < RB / 16; ++k) rec[k] = lds4(p + lane * RB + 16 * k);
-        b = lds1(rhs);
+        for (int k = 0; k < RB / 16; ++k) rec[k] = lds_v4(p + lane * RB + 16 * k);
+        b = lds_d(rhs);
     }
     __device__ __forceinline__ void load_quad(unsigned p, int k, int lane)
     {
-        off[k] = lds2(p + 32 * RB + k * 256 + lane * 8);
+        off[k] = lds_v2(p + 32 * RB + k * 256 + lane * 8);
 #pragma unroll
         for (int u = 0; u < VQ; ++u)
-            val[k * VQ + u] = lds4(p + 32 * RB + 32 * S * 2 + (k * VQ + u) * 512 + lane * 16);
+            val[k * VQ + u] = lds_v4(p + 32 * RB + 32 * S * 2 + (k * VQ + u) * 512 + lane * 16);
     }
     __device__ __forceinline__ unsigned word(int i) const  // word i of the record
     {
@@ -367,26 +312,26 @@ __global__ void __launch_bounds__((kRowWarps + 1) * 32, 1) k_tri_rows(RowArgs a)
     __shared__ unsigned long long bars[NR];
     double* win = reinterpret_cast<double*>(row_smem);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tb = blockIdx.x;
-    const unsigned wbase = smem_at(win);
+    const unsigned wbase = smem_addr(win);
     const unsigned ring = wbase + window_bytes(a.win);
     const unsigned lev_slots = (unsigned)a.ncw * SB, lev_rhs = (unsigned)a.ncw * 32 * 8;
     const unsigned lev = lev_slots + lev_rhs;
     if (threadIdx.x < G) win[a.zero + threadIdx.x] = 0.0;
     if (threadIdx.x == 0) {
-        for (int k = 0; k < NR; ++k) bar_init(smem_at(bars + k));
+        for (int k = 0; k < NR; ++k) bar_init(smem_addr(bars + k));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
     if (warp == a.ncw) {  // copies
         const double* gb = a.rhs + (size_t)tb * a.rstride;
         auto copy = [&](int l) {
-            const unsigned to = ring + (unsigned)(l % NR) * lev, bar = smem_at(bars + l % NR);
+            const unsigned to = ring + (unsigned)(l % NR) * lev, bar = smem_addr(bars + l % NR);
             bar_expect(bar, lev);
             bulk_copy(to, a.slots + (size_t)l * lev_slots, lev_slots, bar);
             bulk_copy(to + lev_slots, gb + (size_t)l * a.ncw * 32, lev_rhs, bar);
         };
         auto landed = [&](int l, int polls) {
-            return bar_wait(smem_at(bars + l % NR), (unsigned)(l / NR) & 1u, polls);
+            return bar_wait(smem_addr(bars + l % NR), (unsigned)(l / NR) & 1u, polls);
         };
         bool ok = true;
         int issued = min(NR, a.nl);
@@ -442,7 +387,7 @@ __global__ void __launch_bounds__((kRowWarps + 1) * 32, 1) k_tri_rows(RowArgs a)
         double x[S];
 #pragma unroll
         for (int st = 0; st < (S < 8 ? S : 8); ++st)
-            if ((st & ~3) < steps) x[st] = lds1(wbase + r.o(st) * 8u);
+            if ((st & ~3) < steps) x[st] = lds_d(wbase + r.o(st) * 8u);
         double acc = r.b;
 #pragma unroll
         for (int k = 0; k < S / 4; ++k) {
@@ -454,7 +399,7 @@ __global__ void __launch_bounds__((kRowWarps + 1) * 32, 1) k_tri_rows(RowArgs a)
 #pragma unroll
                 for (int u = 0; u < 4; ++u)
                     if (4 * k + 8 + u < S)
-                        x[4 * k + 8 + u] = lds1(wbase + r.o(4 * k + 8 + u) * 8u);
+                        x[4 * k + 8 + u] = lds_d(wbase + r.o(4 * k + 8 + u) * 8u);
             nx.load_quad(myslot + at, k, lane);
             if (4 * k + 2 < steps) {
                 acc = fma(r.v(4 * k + 2), x[4 * k + 2], acc);

@@ -758,8 +758,8 @@ void csr_mark_shared_pattern(const DevCsr& K, DevCsr& M, const int* ki, const in
     M.same_pattern = true;
 }
 
-int csr_build_node_blocks(DevCsr& K, int n, const int* ki, const int* kj, const double* kv,
-                          const int* mi, const int* mj, const double* mv, cudaStream_t s)
+int csr_build_node_blocks(DevCsr& K, int n, const int* ki, const int* kj, const int* mi,
+                          const int* mj, const double* mv, cudaStream_t s)
 {
     DevNodeBlocks& nb = K.nb;
     nb.ok = false;

@@ -25,6 +25,75 @@ namespace xt {
 constexpr int kRingParts = 4;
 constexpr int kRingSpin = 1 << 20;  // polls of a wait before it gives up
 
+// Shared memory, mbarriers and bulk copies by shared-memory address.
+__device__ __forceinline__ unsigned smem_addr(const void* p)
+{
+    return (unsigned)__cvta_generic_to_shared(p);
+}
+__device__ __forceinline__ float lds_f(unsigned addr)
+{
+    float r;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(r) : "r"(addr));
+    return r;
+}
+__device__ __forceinline__ double lds_d(unsigned addr)
+{
+    double r;
+    asm volatile("ld.shared.f64 %0, [%1];" : "=d"(r) : "r"(addr));
+    return r;
+}
+__device__ __forceinline__ unsigned lds_u(unsigned addr)
+{
+    unsigned r;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(r) : "r"(addr));
+    return r;
+}
+__device__ __forceinline__ uint2 lds_v2(unsigned addr)
+{
+    uint2 r;
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(r.x), "=r"(r.y) : "r"(addr));
+    return r;
+}
+__device__ __forceinline__ uint4 lds_v4(unsigned addr)
+{
+    uint4 r;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
+                 : "r"(addr));
+    return r;
+}
+__device__ __forceinline__ void bar_init(unsigned bar)
+{
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void bar_expect(unsigned bar, unsigned bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+// The phase of the given parity is complete, within `polls` polls.
+__device__ __forceinline__ bool bar_wait(unsigned bar, unsigned parity, int polls)
+{
+    for (int i = 0; i < polls; ++i) {
+        unsigned ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+__device__ __forceinline__ void bulk_copy(unsigned dst, const void* src, unsigned bytes, unsigned bar)
+{
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+        "l"(src), "r"(bytes), "r"(bar)
+        : "memory");
+}
+
 __device__ __forceinline__ void ring_sync(int id, int threads)
 {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
@@ -42,25 +111,13 @@ __device__ __forceinline__ void ring_level(int threads)
 // Part m has landed, within `polls` polls of its mbarrier.
 __device__ __forceinline__ bool ring_wait(unsigned bars, int m, int polls)
 {
-    const unsigned bar = bars + 8u * (unsigned)(m % kRingParts), parity = (unsigned)(m / kRingParts) & 1u;
-    for (int i = 0; i < polls; ++i) {
-        unsigned ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (ok) return true;
-    }
-    return false;
+    return bar_wait(bars + 8u * (unsigned)(m % kRingParts), (unsigned)(m / kRingParts) & 1u, polls);
 }
 // One thread, after the wait for one of the first kRingParts parts has given up:
 // parts m .. issued - 1 have landed, or, should one not within the full limit,
 // its place is zeroed, for the computing warps take addresses from what they
 // read.  A record of zeros reads and writes element 0 of its buffers.
-__device__ __noinline__ void ring_settle(unsigned at, unsigned bars, unsigned part, int m, int issued)
+inline __device__ __noinline__ void ring_settle(unsigned at, unsigned bars, unsigned part, int m, int issued)
 {
     for (; m < issued; ++m) {
         if (ring_wait(bars, m, kRingSpin)) continue;
@@ -91,8 +148,7 @@ struct SweepRing {
     // one thread, before the block's first barrier
     __device__ __forceinline__ void init() const
     {
-        for (int k = 0; k < kRingParts; ++k)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bars + 8 * k) : "memory");
+        for (int k = 0; k < kRingParts; ++k) bar_init(bars + 8u * (unsigned)k);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __device__ __forceinline__ void copy(int m, const unsigned char* slots, const unsigned char* rhs) const
@@ -100,18 +156,9 @@ struct SweepRing {
         const unsigned bar = bars + 8u * (unsigned)(m % kRingParts);
         const unsigned to = at + (unsigned)(m % kRingParts) * part;
         const unsigned n = (unsigned)min(B, nl - m * B);
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
-                     "r"(n * (lev_slots + lev_rhs))
-                     : "memory");
-        asm volatile(
-            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(to),
-            "l"(slots + (size_t)m * part_slots), "r"(n * lev_slots), "r"(bar)
-            : "memory");
-        asm volatile(
-            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                to + part_slots),
-            "l"(rhs + (size_t)m * B * lev_rhs), "r"(n * lev_rhs), "r"(bar)
-            : "memory");
+        bar_expect(bar, n * (lev_slots + lev_rhs));
+        bulk_copy(to, slots + (size_t)m * part_slots, n * lev_slots, bar);
+        bulk_copy(to + part_slots, rhs + (size_t)m * B * lev_rhs, n * lev_rhs, bar);
     }
     // the copying warp's whole work; false in lane 0, which alone copies and
     // waits, when a wait gave up.  The waits for the first parts take at most

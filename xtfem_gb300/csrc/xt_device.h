@@ -141,14 +141,15 @@ struct DevCsr {
 // the device); no-op when K has no node-block form.
 int node_blocks_refresh(DevCsr& K, cudaStream_t s);
 
-// Builds K.nb from the 1-based host CSR pairs after both were uploaded;
+// Builds K.nb from the 1-based host CSR pair after both were uploaded (K's
+// values come from its device copy);
 // leaves K.nb.ok false when the pair has no exact node-block form: order
 // not a multiple of 3, M not m_ab I3 blockwise, M outside K's blocks, or a
 // column listed twice.  One node with some but not all of its components
 // constrained (a roller) is enough, for M lacks those components' entries:
 // the whole system then runs through the CSR kernels.
-int csr_build_node_blocks(DevCsr& K, int n, const int* ki, const int* kj, const double* kv,
-                          const int* mi, const int* mj, const double* mv, cudaStream_t s);
+int csr_build_node_blocks(DevCsr& K, int n, const int* ki, const int* kj, const int* mi,
+                          const int* mj, const double* mv, cudaStream_t s);
 
 // Marks M as sharing K's sparsity pattern when the 1-based host arrays are
 // identical (both matrices of one mesh), after both were uploaded.
