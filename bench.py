@@ -158,14 +158,15 @@ def algorithmic_bytes(problem, ilu_nnz, p, q=6, merged=True):
 
 
 # DRAM bytes per launch of the kernel classes, from one ncu capture each on
-# this workload (profiles/): dram__bytes_read.sum + dram__bytes_write.sum.
+# the 20 x 20 x 60 rod (profiles/dram_c2.md): dram__bytes_read.sum +
+# dram__bytes_write.sum.
 # ilu_apply_fp32 = its forward and backward sweep kernels (the 6 us
 # right-hand-side pre-pass is not included; the six thread blocks of a sweep
 # read its blob, DRAM serves it once).  kron_spmm_df = the node-block
 # kernel, which reads K as 3 x 3 blocks and M as one scalar per block (its
 # algorithmic bytes are counted for the CSR operands, as for the others).
-NCU_TRAFFIC = {1: 65_922_560 + 519_168, 3: 18_887_680 + 19_129_856,
-               4: 99_808_256 + 41_192_960, 7: 57_748_992 + 28_160}
+NCU_TRAFFIC = {1: 65_922_560 + 519_168, 3: 18_896_640 + 19_138_304,
+               4: 99_917_824 + 35_362_304, 7: 57_742_592 + 114_944}
 
 ROOFLINE_NOTES = {
     3: "level-scheduled triangular sweeps: 764 + 743 dependent levels, each sweep on six SMs, one "

@@ -24,8 +24,9 @@ LIB_SAN = HERE / "libxtfem_gb300_san.so"
 SAN = ["-fsanitize=address", "-fsanitize=undefined", "-fno-omit-frame-pointer"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
-# per-file extra flags: the damage kernel keeps the reference's operation
-# order in its exact FP64 path, so multiply-adds are not contracted there
+# per-file extra flags: the damage kernel places its multiply-adds by hand (the
+# screen's bounds and the rounding of the plastic chains count on them), so the
+# compiler contracts none there
 EXTRA = {"dev_damage.cu": ["-fmad=false"]}
 
 

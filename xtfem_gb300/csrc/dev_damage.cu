@@ -4,8 +4,9 @@
 // src/damage.h:9-17): for every spatial Gauss point and every temporal
 // interpolation point of the slab, interpolate the strain, run the elastic
 // predictor and, when the trial von Mises stress exceeds sig_f, the plastic
-// corrector with stored energy ws and damage D.  One thread per Gauss point,
-// all state in FP64.
+// corrector with stored energy ws and damage D, all state in FP64.  A thread
+// screens the steps of one Gauss point; a point that yields goes to a team of 8
+// or 32 lanes of its warp, in the reference's formulas with regrouped sums.
 //
 // The reference spends 144 FMAs per step re-interpolating the displacement
 // of the 8 nodes (src/kokkos_kernel.h:55-71).  The strain is linear in the
@@ -25,8 +26,8 @@
 // proves elastic change nothing but the "last elastic" markers (sig_eff,
 // eps_old, sig_d are overwritten by every elastic step, so only the last one
 // before a plastic step, or before the slab ends, has to be evaluated).
-// A point's first step the screen cannot decide, and all that follow, go to a
-// team of lanes of the warp that takes the point's FP64 steps (Team).
+// A point's first step the screen cannot decide, and all that follow, are the
+// team's (Team).
 #include <cstdlib>
 #include <mutex>
 
@@ -210,7 +211,7 @@ __device__ __noinline__ void slow_materialize(Slow* s, const double* __restrict_
 // lane 6 the trace of every tensor as a component of its own (the predictor
 // and the corrector act on the trace as on a component, with coefficients of
 // its own, so no trace is ever summed), and the scalars are held by all: about
-// 85 instructions a plastic step without damage growth, 130 with it.  The
+// 90 instructions a plastic step without damage growth, 134 with it.  The
 // factors of the damage (four quotients) are formed by four lanes in one
 // division, and again only when the damage has changed.  A team's L lanes
 // screen L steps at once between plastic phases.
@@ -220,10 +221,11 @@ __device__ __noinline__ void slow_materialize(Slow* s, const double* __restrict_
 // a (tee - tr / 3)); everything in FP64.
 //
 // Measured (GB300, against one thread a point): a slab of 25,600 steps on
-// 192,000 points, 170 of them plastic, 122 -> 19.6 ms (3.05 us a plastic step
-// of the point with the most, 4,900 of its 6,300 cycles FP64 issue); 1,536
-// points, 2,560 steps, host arrays, 31.0 -> 5.1 ms; no plastic point (192,000
-// points, 25,600 steps) 2.1 -> 0.45 ms, from the chunk bound and fused sums.
+// 192,000 points, displacement amplitudes of 115 MPa at other seeds, 122 to 159
+// -> 21.5 to 26 ms; 1,536 points, 2,560 steps, host arrays, 31 to 33 -> 5.7 ms;
+// no plastic point (192,000 points, 25,600 steps) 2.1 -> 0.45 ms, from the chunk
+// bound and fused sums; every point of 24,000 yielding, 1,024 steps, 14.6 -> 11.9
+// ms, with their damage growing 16.5 -> 16.5.
 //
 // L = 32 for a warp's only point that needs exact steps (32 steps a screening
 // pass), else L = 8 (four points a warp, each FP64 instruction serving four; two
@@ -1037,10 +1039,10 @@ int damage_update(const DamageArgs& a, cudaStream_t s)
     const char* e = std::getenv("XTFEM_DAMAGE_RUN");
     const int run_bound = (!e || std::atoi(e) != 0) ? 1 : 0;
     // 128 threads per block (XTFEM_DAMAGE_THREADS=256: 256).  A block that
-    // holds a plastic point runs for the whole update; at 170 registers a
-    // thread, a 128-thread block leaves its SM room for the solve's blocks
-    // beside it, where a 256-thread block (43.5 K registers) left room for
-    // two dot-pass blocks of six.
+    // holds a plastic point runs for the whole update; at 202 registers a
+    // thread, a 128-thread block (26 K registers) leaves its SM room for the
+    // solve's blocks beside it, a 256-thread block (52 K) for none of the dot
+    // pass's.
     const char* et = std::getenv("XTFEM_DAMAGE_THREADS");
     const int nt = (et && std::atoi(et) == 256) ? 256 : 128;
     // XTFEM_DAMAGE_BLOCKS=B: a grid of B blocks, each thread taking several
