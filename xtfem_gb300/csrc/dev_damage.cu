@@ -208,24 +208,24 @@ __device__ __noinline__ void slow_materialize(Slow* s, const double* __restrict_
 // live lanes, so a point's chain of plastic steps costs its FP64 instruction
 // count: one thread doing the six components in turn took about 940 of them a
 // step (29 us).  Here lane i < 6 of a team holds component i of every tensor,
-// lane 6 the trace of every tensor as a component of its own (the predictor
-// and the corrector act on the trace as on a component, with coefficients of
-// its own, so no trace is ever summed), and the scalars are held by all: about
-// 90 instructions a plastic step without damage growth, 134 with it.  The
+// lane 6 the mean of every tensor as a component of its own (the predictor
+// and the corrector act on the mean as on a component, so no trace is ever
+// summed), and the scalars are held by all: about
+// 87 instructions a plastic step without damage growth, 131 with it.  The
 // factors of the damage (four quotients) are formed by four lanes in one
 // division, and again only when the damage has changed.  A team's L lanes
 // screen L steps at once between plastic phases.
 //
 // The formulas are those of src/kokkos_kernel.h:96-341 with the sums regrouped
 // (c5 = 1 + gam dp / SIGF is qeq / SIGF; the deviator of D tee is
-// a (tee - tr / 3)); everything in FP64.
+// a (tee - mean)); everything in FP64.
 //
 // Measured (GB300, against one thread a point): a slab of 25,600 steps on
 // 192,000 points, displacement amplitudes of 115 MPa at other seeds, 122 to 159
-// -> 21.5 to 26 ms; 1,536 points, 2,560 steps, host arrays, 31 to 33 -> 5.7 ms;
+// -> 21.2 to 26 ms; 1,536 points, 2,560 steps, host arrays, 31 to 33 -> 5.6 ms;
 // no plastic point (192,000 points, 25,600 steps) 2.1 -> 0.45 ms, from the chunk
-// bound and fused sums; every point of 24,000 yielding, 1,024 steps, 14.6 -> 11.9
-// ms, with their damage growing 16.5 -> 16.5.
+// bound and fused sums; every point of 24,000 yielding, 1,024 steps, 14.6 -> 11.4
+// ms, with their damage growing 16.5 -> 16.0.
 //
 // L = 32 for a warp's only point that needs exact steps (32 steps a screening
 // pass), else L = 8 (four points a warp, each FP64 instruction serving four; two
@@ -236,11 +236,11 @@ __device__ __noinline__ void slow_materialize(Slow* s, const double* __restrict_
 template <int L>
 struct Team {
     // lane constants: elastic coefficients, weight in the equivalent stress,
-    // share of the trace (normal 1/3, shear 0, trace 1)
-    double a, off, w, third;
+    // share of the mean (shear 0, else 1)
+    double a, off, w, nrm;
     double cb, ca, cacb, kb3, g3;     // factors of the moduli (load)
     double cden;                      // the coefficient of d in the lane's quotient of factors()
-    double ky, kn;                    // (1 + nu) / 2E and nu / 2E, divided by SD
+    double ky, kn;                    // (1 + nu) / 2E and 9 nu / 2E, divided by SD
     double E[6];                      // strain basis of the lane's component
     double epo, epl, sef, sbk;        // the lane's components
     double p, d, ws, dpo, sigd;       // the point's scalars
@@ -273,14 +273,14 @@ struct Team {
         g3 = 3.0 * (Ey / (2.0 * (1.0 + nu))) * (1.0 - cb);
         cden = i == 0 ? cb : (i == 1 ? ca : HH);
         ky = (1.0 + nu) / (2.0 * Ey) * (1.0 / SD);
-        kn = nu / (2.0 * Ey) * (1.0 / SD);
+        kn = 9.0 * (nu / (2.0 * Ey)) * (1.0 / SD);
         const double coef = Ey / ((1.0 + nu) * (1.0 - 2.0 * nu)), mn = coef * (1.0 - 2.0 * nu);
-        const bool norm = i < 3, shear = i >= 3 && i < 6, tr = i == 6;
-        a = shear ? 0.5 * mn : (norm || tr ? mn : 0.0);
-        off = norm ? coef * nu : (tr ? 3.0 * coef * nu : 0.0);
-        w = norm ? 1.5 : (shear ? 3.0 : 0.0);
-        third = norm ? 1.0 / 3.0 : (tr ? 1.0 : 0.0);
-        kb3 = Ey / (3.0 * (1.0 - 2.0 * nu)) * (norm ? 1.0 : (tr ? 3.0 : 0.0));
+        const bool shear = i >= 3 && i < 6, norm = i < 3 || i == 6;  // normal component or mean
+        a = shear ? 0.5 * mn : (norm ? mn : 0.0);
+        off = norm ? 3.0 * coef * nu : 0.0;
+        w = i < 3 ? 1.5 : (shear ? 3.0 : 0.0);
+        nrm = norm ? 1.0 : 0.0;
+        kb3 = norm ? Ey / (1.0 - 2.0 * nu) : 0.0;
         // component i of the strain rows: N_a u_x (+ N_b u_y for a shear)
         const double* Na = (i == 0 ? A.Nx : (i == 1 || i == 3 ? A.Ny : A.Nz)) + (size_t)gp * A.nnse;
         const double* Nb = (i == 4 ? A.Ny : A.Nx) + (size_t)gp * A.nnse;
@@ -300,15 +300,15 @@ struct Team {
         epl = i < 6 ? A.eps_pl[b6] : 0.0;
         sef = i < 6 ? A.sig_eff[b6] : 0.0;
         sbk = i < 6 ? A.sig_back[b6] : 0.0;
-        auto trace = [&](double& v) {
-            const double t = get(v, 0) + get(v, 1) + get(v, 2);
-            if (tr) v = t;
+        auto mean = [&](double& v) {
+            const double t = (get(v, 0) + get(v, 1) + get(v, 2)) / 3.0;
+            if (i == 6) v = t;
         };
-        for (int k = 0; k < 6; ++k) trace(E[k]);
-        trace(epo);
-        trace(epl);
-        trace(sef);
-        trace(sbk);
+        for (int k = 0; k < 6; ++k) mean(E[k]);
+        mean(epo);
+        mean(epl);
+        mean(sef);
+        mean(sbk);
         p = A.p[gp];
         d = A.D[gp];
         ws = A.ws[gp];
@@ -330,7 +330,7 @@ struct Team {
         c1 = r1;
         c3m1 = fma(cb * omd, r1, -1.0);
         const double c2 = cacb * d * r1 * ra;
-        c2i = c2 * third;
+        c2i = c2 * nrm;
         Ai = a * r1;
         Bi = fma(off, r1, kb3 * c2);
         cyd = (2.0 * CY / 3.0) * omd;
@@ -343,7 +343,7 @@ struct Team {
     {
         sumg = 0.0;
         for (int k = 0; k < 6; ++k) {
-            const double gk = c1 * a * fma(-third, get(E[k], 6), E[k]);
+            const double gk = c1 * a * fma(-nrm, get(E[k], 6), E[k]);
             sumg = fma((double)__ldg(ntmax + k), fabs(gk), sumg);
             const float f = (float)gk;
 #pragma unroll
@@ -352,7 +352,7 @@ struct Team {
     }
     __device__ __forceinline__ void screen_state()
     {
-        const double c = fma(c3m1 * a, fma(-third, get(epl, 6), epl), -sbk);
+        const double c = fma(c3m1 * a, fma(-nrm, get(epl, 6), epl), -sbk);
         const float f = (float)c;
 #pragma unroll
         for (int i = 0; i < 6; ++i) c0[i] = __shfl_sync(mask, f, i, L);
@@ -385,18 +385,18 @@ struct Team {
         for (int k = 1; k < 6; ++k) e = fma(nt[k], E[k], e);
         return e;
     }
-    // elastic predictor: the trial elastic strain, its trace and teq^2
-    __device__ __forceinline__ double predict(double eps, double& tee, double& ttr) const
+    // elastic predictor: the trial elastic strain, its mean and teq^2
+    __device__ __forceinline__ double predict(double eps, double& tee, double& tm) const
     {
         tee = fma(c2i, get(eps, 6), fma(c3m1, epl, c1 * eps));
-        ttr = get(tee, 6);
-        const double ts = fma(a, fma(-third, ttr, tee), -sbk);
+        tm = get(tee, 6);
+        const double ts = fma(a, fma(-nrm, tm, tee), -sbk);
         return sum8(w * ts * ts);
     }
     // outputs of an elastic step
-    __device__ __forceinline__ void elastic(double eps, double tee, double ttr, double q, bool take)
+    __device__ __forceinline__ void elastic(double eps, double tee, double tm, double q, bool take)
     {
-        const double s = fma(off, ttr, a * tee), t = sqrt(q);
+        const double s = fma(off, tm, a * tee), t = sqrt(q);
         if (L == 32 || take) {
             sef = s;
             epo = eps;
@@ -410,14 +410,12 @@ struct Team {
         const bool take = L == 32 || part;
         const double de = eps - epo;
         const double qs = sbk - sef - fma(Ai, de, Bi * get(de, 6));
-        // the mean of qs, its trace / 3 as a division rounds it (0 for a shear,
-        // the trace itself in the trace's lane).  It leaves qs here and returns
-        // to the stress below: a third by multiplication, always too small, and
-        // a common factor for dsg grew over a chain of steps to 1.9 times the
-        // error of p, 1.4 times that of the stresses.
-        const double qtr = get(qs, 6), t3 = qtr * third;
-        const double qm = fma(fma(lane < 3 ? -3.0 : -1.0, t3, qtr), third, t3);
-        const double dq = qs - qm;
+        // The mean of qs, the same number here and below: with a trace and a
+        // third by multiplication, always too small, and a common factor for dsg
+        // a chain of steps ended with 1.9 times the error of p and 1.4 times that
+        // of the stresses that the reference's sequence has; this has 0.85 to 1.
+        const double qm = get(qs, 6);
+        const double dq = fma(-nrm, qm, qs);
         const double q2 = sum8(w * dq * dq);
         // qeq = sqrt(q2), and its reciprocal: one Newton step on q2 rsqrt(q2)
         const double rq = rsqrt(q2);
@@ -430,12 +428,12 @@ struct Team {
         const double k1 = dp * (1.5 / SIGF);
         const double nepl = fma(dsg, k1, epl);
         const double nsbk = fma(dsg, k1 * cyd, sbk);
-        const double nsef = (dsg - qm) + nsbk;
+        const double nsef = fma(-nrm, qm, dsg) + nsbk;
         // the equivalent stress, and the damage rate's square where it may be
         // needed: both sums in one butterfly (lanes 0..3 the one, 4..7 the
         // other) and both roots in one
-        const double tr2 = get(nsef, 6);
-        const double sd = fma(-third, tr2, nsef);
+        const double m2 = get(nsef, 6);
+        const double sd = fma(-nrm, m2, nsef);
         const double v = w * sd * sd;
         double seq, rate = 0.0;
         if (any(take && ws >= WD)) {
@@ -444,7 +442,7 @@ struct Team {
             double t = (up ? y : v) + __shfl_xor_sync(mask, up ? v : y, 4, L);
             t += __shfl_xor_sync(mask, t, 2, L);
             t += __shfl_xor_sync(mask, t, 1, L);
-            const double yn = kn * (tr2 >= 0.0 ? 1.0 : hx2) * tr2 * tr2;
+            const double yn = kn * (m2 >= 0.0 ? 1.0 : hx2) * m2 * m2;
             const double root = sqrt(up ? fma(ky, t, -yn) : t);
             seq = get(root, 0);
             rate = get(root, 4);
@@ -452,11 +450,11 @@ struct Team {
             seq = sqrt(sum8(v));
         }
         const double snew = fabs(seq - SIGF);
-        const double nws = ws + fma(snew, dp, sold * dpo) * 0.5;
+        const double nws = fma(fma(snew, dp, sold * dpo), 0.5, ws);
         const bool grow = take && nws >= WD;
         if (any(grow && ws < WD)) {  // the step that crosses the threshold
             const double sp = sum8(lane < 3 ? (nsef < 0.0 ? hx2 : 1.0) * nsef * nsef : 0.0);
-            const double yn = kn * (tr2 >= 0.0 ? 1.0 : hx2) * tr2 * tr2;
+            const double yn = kn * (m2 >= 0.0 ? 1.0 : hx2) * m2 * m2;
             const double r = sqrt(fma(ky, sp, -yn));
             if (ws < WD) rate = r;
         }
@@ -553,20 +551,20 @@ __device__ __noinline__ void exact_points(const DamageArgs& A, const float* __re
             double nx[6];  // the next step's shape values, loaded meanwhile
             shape_row(A.Nt, min(jj + 1, A.nip - 1), nx);
             const double eps = T.strain(nt);
-            double tee, ttr;
-            const double q = T.predict(eps, tee, ttr);
+            double tee, tm;
+            const double q = T.predict(eps, tee, tm);
             const bool plastic = act && !(q <= SIGF * SIGF);
             if (act) ++n_exact;
             // a plastic step after proven ones: their last one's outputs first
             const bool pend = plastic && last >= 0;
             if (Team<L>::any(pend)) {
-                double lt[6], le_tee, le_ttr;
+                double lt[6], le_tee, le_tm;
                 shape_row(A.Nt, last >= 0 ? last : 0, lt);
                 const double le = T.strain(lt);
-                const double lq = T.predict(le, le_tee, le_ttr);
-                T.elastic(le, le_tee, le_ttr, lq, pend);
+                const double lq = T.predict(le, le_tee, le_tm);
+                T.elastic(le, le_tee, le_tm, lq, pend);
             }
-            if (Team<L>::any(act && !plastic)) T.elastic(eps, tee, ttr, q, act && !plastic);
+            if (Team<L>::any(act && !plastic)) T.elastic(eps, tee, tm, q, act && !plastic);
             bool dch = false;
             if (Team<L>::any(plastic)) {
                 dch = T.correct(eps, plastic);
@@ -594,11 +592,11 @@ __device__ __noinline__ void exact_points(const DamageArgs& A, const float* __re
         }
         // outputs of the last proven step
         if (Team<L>::any(last >= 0)) {
-            double lt[6], tee, ttr;
+            double lt[6], tee, tm;
             shape_row(A.Nt, last >= 0 ? last : 0, lt);
             const double le = T.strain(lt);
-            const double lq = T.predict(le, tee, ttr);
-            T.elastic(le, tee, ttr, lq, last >= 0);
+            const double lq = T.predict(le, tee, tm);
+            T.elastic(le, tee, tm, lq, last >= 0);
         }
         if (on) {
             const int i = T.lane;
